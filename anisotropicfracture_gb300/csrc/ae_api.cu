@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../../include/aefast.h"
+#include "ae_bottom_ell.h"
 #include "ae_csr_chunks.h"
 #include "ae_launch.h"
 #include "ae_split.h"
@@ -101,7 +102,7 @@ struct MGLevel {
     SplitList split;
     bool split_built = false;
     // coarsest MG level of AMR level 0: its operator as an FP64 CSR matrix, for the bottom solve
-    // of the FP32 cycle (assembled by prepare32)
+    // (assembled on the first solve after the model, the boundary types or the uniform flag changed)
     int* csr_rowptr = nullptr;
     int* csr_col = nullptr;
     double* csr_val = nullptr;
@@ -110,6 +111,13 @@ struct MGLevel {
     int* csr_rch = nullptr;
     int csr_nchunk = 0, csr_ccap = 0;
     bool csr_ok = false;
+    bool csr_built = false;
+    int csr_uniform = -1;
+    // the same matrix in the four-warp form, in one allocation (BottomEll points into it)
+    unsigned char* ell_buf = nullptr;
+    size_t ell_cap = 0;
+    BottomEll ell{};
+    bool ell_ok = false;
 };
 
 struct AmrLevel {
@@ -347,11 +355,56 @@ void alloc_level_fp32(ae_op* op) {
     op->have32 = true;
 }
 
+// The four-warp form of the assembled matrix, when the level is small enough for it.
+void upload_bottom_ell(ae_op* op, MGLevel& L, const std::vector<int>& rp, const std::vector<int>& cl,
+                       const std::vector<double>& vl) {
+    const BottomEllHost h = bottom_ell(rp, cl, vl, kBottomQuadLayers);
+    if (!h.ok) return;
+    BottomEll& m = L.ell;
+    m = BottomEll{};
+    m.nval = (int)h.val.size();
+    m.ngroups = (int)h.goff.size() - 1;
+    m.nchunk = h.nchunk;
+    m.layers = h.layers;
+    if (!bottom_quad_init(m)) return;
+    std::vector<unsigned char> host;
+    const auto put = [&](const void* p, size_t bytes) {
+        const size_t at = (host.size() + 15) / 16 * 16;
+        host.resize(at + bytes);
+        if (bytes) std::memcpy(host.data() + at, p, bytes);
+        return at;
+    };
+    const size_t o_val = put(h.val.data(), h.val.size() * sizeof(double));
+    const size_t o_col = put(h.col.data(), h.col.size() * sizeof(unsigned short));
+    const size_t o_goff = put(h.goff.data(), h.goff.size() * sizeof(int));
+    const size_t o_slot = put(h.slot.data(), h.slot.size() * sizeof(int));
+    const size_t o_wgrp = put(h.wgrp.data(), h.wgrp.size() * sizeof(int));
+    const size_t o_rows = put(h.rows.data(), h.rows.size() * sizeof(int));
+    const size_t o_perm = put(h.perm.data(), h.perm.size() * sizeof(int));
+    if (host.size() > L.ell_cap) {
+        L.ell_buf = op->alloc<unsigned char>((long long)host.size());
+        L.ell_cap = host.size();
+    }
+    AE_CHECK(cudaMemcpyAsync(L.ell_buf, host.data(), host.size(), cudaMemcpyHostToDevice, op->st));
+    AE_CHECK(cudaStreamSynchronize(op->st));
+    m.val = reinterpret_cast<const double*>(L.ell_buf + o_val);
+    m.col = reinterpret_cast<const unsigned short*>(L.ell_buf + o_col);
+    m.goff = reinterpret_cast<const int*>(L.ell_buf + o_goff);
+    m.slot = reinterpret_cast<const int*>(L.ell_buf + o_slot);
+    m.wgrp = reinterpret_cast<const int*>(L.ell_buf + o_wgrp);
+    m.rows = reinterpret_cast<const int*>(L.ell_buf + o_rows);
+    m.perm = reinterpret_cast<const int*>(L.ell_buf + o_perm);
+    L.ell_ok = true;
+}
+
 // The coarsest level of AMR level 0 as an FP64 CSR matrix (levels of up to kBottomCsrMaxN
 // unknowns): dense columns A e_j on the device, compressed here, uploaded once per preparation.
 void assemble_bottom(ae_op* op) {
     MGLevel& L = op->amr[0].mg.back();
-    L.csr_ok = false;
+    if (L.csr_built && L.csr_uniform == op->uniform) return;
+    L.csr_ok = L.ell_ok = false;
+    L.csr_built = true;
+    L.csr_uniform = op->uniform;
     const long long N = 3 * L.nn;
     if (N > kBottomCsrMaxN) return;
     cudaStream_t st = op->st;
@@ -367,8 +420,11 @@ void assemble_bottom(ae_op* op) {
             if (p) cudaFree(p);
         }
     } A, E;
-    AE_CHECK(cudaMalloc(&A.p, sizeof(double) * N * N));
-    AE_CHECK(cudaMalloc(&E.p, sizeof(double) * N * N));
+    // without room for the scratch the bottom solve runs on the stencil
+    if (cudaMalloc(&A.p, sizeof(double) * N * N) != cudaSuccess || cudaMalloc(&E.p, sizeof(double) * N * N) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
     std::vector<double> h((size_t)(N * N));
     launch_bottom_assemble(a, A.p, E.p, st);
     AE_CHECK(cudaMemcpyAsync(h.data(), A.p, sizeof(double) * N * N, cudaMemcpyDeviceToHost, st));
@@ -412,6 +468,7 @@ void assemble_bottom(ae_op* op) {
     L.csr_nnz = nnz;
     L.csr_nchunk = nchunk;
     L.csr_ok = true;
+    upload_bottom_ell(op, L, rp, cl, vl);
 }
 
 // FP32 copies of the stiffness and diagonal on every level (mixed-precision cycle)
@@ -426,7 +483,6 @@ void prepare32(ae_op* op) {
             launch_copy<float, double>(s, 3, level_view(L.g, L.invD32), cview(level_view(L.g, L.invD)), op->st);
         }
     AE_CHECK(cudaStreamSynchronize(op->st));
-    assemble_bottom(op);
     op->prepared32 = true;
 }
 
@@ -481,6 +537,7 @@ void prepare(ae_op* op) {
             launch_diagonal<double>(op->params(L.g), cview(level_view(L.g, L.C)), level_view(L.g, L.D),
                                     level_view(L.g, L.invD), op->dflag, st);
     op->prepared32 = false;
+    op->amr[0].mg.back().csr_built = false;
     for (auto& A : op->amr)
         for (auto& L : A.mg) {
             if (L.split.list) AE_CHECK(cudaFree(L.split.list));
@@ -620,8 +677,6 @@ struct Cycle {
         const int m = (int)lv.size() - 1;
         MGLevel& L = lv[m];
         const Box3 s = geo_store(L.g);
-        if (sizeof(R) == 4) launch_copy<double, R>(s, 3, level_view(L.g, L.res), cview(level_view(L.g, ptrs<R>(L).res)), st);
-        launch_fill<double>(s, 3, level_view(L.g, L.cor), 0.0, st);
         BottomArgs a;
         a.P = op->params(L.g);
         a.K = make_scoef<double>(L.g);
@@ -639,8 +694,15 @@ struct Cycle {
         a.sweeps = o.sweeps;
         a.omega = o.omega;
         a.fail_count = op->dflag + 1;
-        // the FP32 cycle's bottom: the same FP64 Krylov loop over the assembled level operator
-        if (sizeof(R) == 4 && L.csr_ok)
+        // the FP64 Krylov loop over the assembled level operator: four warps with the vectors in
+        // registers when the level is small (reading and writing the cycle's own precision), else one block
+        if (L.ell_ok) {
+            launch_bottom_quad<R>(a, L.ell, ptrs<R>(L).res, ptrs<R>(L).cor, st);
+            return;
+        }
+        if (sizeof(R) == 4) launch_copy<double, R>(s, 3, level_view(L.g, L.res), cview(level_view(L.g, ptrs<R>(L).res)), st);
+        launch_fill<double>(s, 3, level_view(L.g, L.cor), 0.0, st);
+        if (L.csr_ok)
             launch_bottom_csr(a, BottomCsr{L.csr_rowptr, L.csr_col, L.csr_val, L.csr_nnz, L.csr_cptr, L.csr_rch,
                                            L.csr_nchunk},
                               st);
@@ -1684,6 +1746,7 @@ static int solve_entry(ae_op* op, const ae_fab* sol, const ae_fab* rhs, double t
         require(o.bottom == 0 || o.bottom == 1, "bottom must be 0 (CG) or 1 (BiCGStab)");
         if (!op->prepared) prepare(op);
         if (o.precision) prepare32(op);
+        assemble_bottom(op);
         const int namr = (int)op->amr.size();
         // fields: level 0 over its domain, finer levels over the patch and its 2 ghost layers
         std::vector<Box3> region(namr);

@@ -2,6 +2,7 @@
 // values, post-processing fields and the single-CTA bottom solver.
 #include <type_traits>
 
+#include "ae_bottom_ell.h"
 #include "ae_kernels.cuh"
 #include "ae_krylov.cuh"
 
@@ -694,13 +695,11 @@ void launch_ring_interp_fix(const Geo& gf, View<double> x, View<const float> ecr
 }
 
 // ------------------------------------------------------------------ assembled bottom operator
-// The coarsest level's operator as an explicit FP64 matrix, for the bottom solve of the FP32
-// cycle.  GB300 issues FP64 at a small fraction of its FP32 rate, and the stencil form of the
-// level operator costs a few hundred FP64 instructions per node on one SM; the assembled rows
-// cost one FMA per nonzero.  Column j is the operator applied to the unit vector e_j (so every
-// entry is the stencil's own coefficient sum for that pair of unknowns); the host compresses
-// the columns to CSR.  The FP64 solve keeps the stencil form (its bottom follows the reference
-// operation for operation).
+// The coarsest level's operator as an explicit FP64 matrix, for the bottom solve.  GB300 issues
+// FP64 at a small fraction of its FP32 rate, and the stencil form of the level operator costs a few
+// hundred FP64 instructions per node on one SM; the assembled rows cost one FMA per nonzero.  Column
+// j is the operator applied to the unit vector e_j (so every entry is the stencil's own coefficient
+// sum for that pair of unknowns); the host compresses the columns to CSR.
 
 // block j: column j of the dense N x N matrix A (row-major); E holds one unit vector per block
 template <int M>
@@ -857,6 +856,336 @@ void launch_bottom_csr(const BottomArgs& a, const BottomCsr& m, cudaStream_t st)
     else k_bottom_csr<false><<<1, threads, 0, st>>>(a, m);
     launched();
 }
+
+// ------------------------------------------------------------------ four-warp bottom solve
+// The Krylov loop of krylov_bottom on up to 768 unknowns: four warps, vectors in registers, the
+// matrix in shared memory.
+//
+// What bounds it: FP64 issue.  A sub-partition of a GB300 SM takes a warp-wide DFMA every 64 cycles,
+// whatever lanes are active (a dependent one after 74, a division about 560), so the time of an
+// iteration is the number of warp-wide FP64 instructions on the busiest sub-partition.  A 256-thread
+// block puts two warps on each and makes every one of them join each reduction and repeat each
+// division.  Here there is one warp per sub-partition, and
+//   - the product's chunks are dealt to the warps by length; a long row's chunk sums are added by 8
+//     lanes;
+//   - sum of squares and max-norm of r share a reduction, the max on integer bit patterns (REDUX);
+//   - rho / p.Ap and 1 / rho (for the next beta) are one division instruction, on two lanes;
+//   - a reduction needs one barrier.
+// Measured on the 3^3-node coarsest level (81 unknowns), a call of 200 CG iterations: 256-thread
+// block on the assembled matrix 0.95 ms, on the stencil (the FP64 solve) 2.54 ms, one warp 0.80 ms,
+// this kernel 0.54 ms (loads unrolled four steps ahead: 0.60).  648 unknowns, BiCGStab: 4.2 ms in
+// the block, 2.7 ms here.
+struct QuadShared {
+    double part[2][kEllWarps];
+    unsigned long long top[2][kEllWarps];
+};
+// |v| as bits; NaN counts as 0, as fmax drops it
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    return b > 0x7ff0000000000000ull ? 0ull : b;
+}
+// a < b for non-negative doubles
+__device__ __forceinline__ bool lt_bits(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
+__device__ __forceinline__ bool is_zero(double a) { return (__double_as_longlong(a) << 1) == 0; }
+
+// E: unknowns per thread (slots t, t + 128, ...)
+template <int E>
+struct QuadEll {
+    const double* val;
+    const unsigned short* col;
+    const int* goff;
+    const int* slot;
+    double* part;  // chunk sums
+    double* xs;    // the vector multiplied
+    QuadShared* sh;
+    int g0, g1;    // this warp's groups
+    int lane, warp, buf;
+    int rows[E];
+    int most[E];   // most chunks of a row of this warp in each layer, long rows apart
+    bool wide[E];  // a long row among them
+
+    // out = A v
+    __device__ __forceinline__ void apply(const double (&v)[E], double (&out)[E]) const {
+#pragma unroll
+        for (int e = 0; e < E; ++e) xs[threadIdx.x + kEllThreads * e] = v[e];
+        __syncthreads();
+        for (int g = g0; g < g1; ++g) {
+            const int w = slot[32 * g + lane], len = (w >> 16) - 1;
+            const int base = goff[g] + lane;
+            double s = 0.0;
+            for (int q = 0; q < len; ++q) s = fma(val[base + 32 * q], xs[col[base + 32 * q]], s);
+            if (w) part[w & 0xffff] = s;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const int first = rows[e] & 0xffff, n = rows[e] >> 16;
+            const bool mine = n <= kEllLongRow;
+            const auto at = [&](int c) { return mine && c < n ? part[first + c] : 0.0; };
+            double s = at(0);
+            if (most[e] > 2) s = (s + at(1)) + (at(2) + at(3));
+            else if (most[e] > 1) s = s + at(1);
+            if (wide[e]) {
+                const int w = __shfl_sync(0xffffffffu, rows[e], lane & 24), n8 = w >> 16, f8 = w & 0xffff;
+                double t = 0.0;
+                if (n8 > kEllLongRow) {
+                    t = (lane & 7) < n8 ? part[f8 + (lane & 7)] : 0.0;
+                    for (int c = (lane & 7) + 8; c < n8; c += 8) t += part[f8 + c];
+                }
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (!mine) s = t;
+            }
+            out[e] = s;
+        }
+    }
+    // the sum of s over the block; with TOP also the max of the bit patterns m
+    template <bool TOP>
+    __device__ __forceinline__ double reduce(double s, unsigned long long m, double& top) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        unsigned long long t = 0;
+        if (TOP) {
+            const unsigned h = __reduce_max_sync(0xffffffffu, (unsigned)(m >> 32));
+            const unsigned l = __reduce_max_sync(0xffffffffu, (unsigned)(m >> 32) == h ? (unsigned)m : 0u);
+            t = ((unsigned long long)h << 32) | l;
+        }
+        // two buffers: a warp may be writing the next sum while another still reads this one
+        buf ^= 1;
+        if (lane == 0) {
+            sh->part[buf][warp] = s;
+            if (TOP) sh->top[buf][warp] = t;
+        }
+        __syncthreads();
+        if (TOP)
+            top = __longlong_as_double((long long)max(max(sh->top[buf][0], sh->top[buf][1]),
+                                                      max(sh->top[buf][2], sh->top[buf][3])));
+        return (sh->part[buf][0] + sh->part[buf][1]) + (sh->part[buf][2] + sh->part[buf][3]);
+    }
+    __device__ __forceinline__ double dot(const double (&x)[E], const double (&y)[E]) {
+        double s = x[0] * y[0], none;
+#pragma unroll
+        for (int e = 1; e < E; ++e) s = fma(x[e], y[e], s);
+        return reduce<false>(s, 0, none);
+    }
+    // the dot product x.y and the max-norm of r
+    __device__ __forceinline__ double dot_max(const double (&x)[E], const double (&y)[E], const double (&r)[E],
+                                              double& rmax) {
+        double s = x[0] * y[0];
+        unsigned long long m = abs_bits(r[0]);
+#pragma unroll
+        for (int e = 1; e < E; ++e) {
+            s = fma(x[e], y[e], s);
+            m = max(m, abs_bits(r[e]));
+        }
+        return reduce<true>(s, m, rmax);
+    }
+};
+
+// the quotients a / b and c / d as one division
+__device__ __forceinline__ void div2(double a, double b, double c, double d, int lane, double& q0, double& q1) {
+    const double q = (lane == 1 ? c : a) / (lane == 1 ? d : b);
+    q0 = __shfl_sync(0xffffffffu, q, 0);
+    q1 = __shfl_sync(0xffffffffu, q, 1);
+}
+// a / d from inv = 1 / d: the product and one correction by its remainder
+__device__ __forceinline__ double div_by(double a, double d, double inv) {
+    const double q = a * inv;
+    const double c = fma(fma(-d, q, a), inv, q);
+    // outside the range where the remainder is exact, or with infinities, divide
+    const unsigned e = ((unsigned)__double2hiint(c) >> 20) & 0x7ff, ed = ((unsigned)__double2hiint(d) >> 20) & 0x7ff,
+                   ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ff;
+    return e - 64u < 0x780u && ed - 64u < 0x780u && ea - 64u < 0x780u ? c : a / d;
+}
+
+template <class R, int E>
+__global__ void __launch_bounds__(kEllThreads) k_bottom_quad(BottomArgs a, BottomEll m, const R* __restrict__ bg,
+                                                             R* __restrict__ xg) {
+    extern __shared__ double smem[];
+    __shared__ QuadShared shared;
+    const int tid = threadIdx.x;
+    QuadEll<E> A;
+    double* sval = smem;
+    A.part = sval + m.nval;
+    A.xs = A.part + m.nchunk;
+    int* sgoff = reinterpret_cast<int*>(A.xs + kEllThreads * E);
+    int* sslot = sgoff + m.ngroups + 1;
+    unsigned short* scol = reinterpret_cast<unsigned short*>(sslot + 32 * m.ngroups);
+    for (int t = tid; t < m.nval; t += kEllThreads) {
+        sval[t] = __ldg(m.val + t);
+        scol[t] = __ldg(m.col + t);
+    }
+    for (int t = tid; t <= m.ngroups; t += kEllThreads) sgoff[t] = __ldg(m.goff + t);
+    for (int t = tid; t < 32 * m.ngroups; t += kEllThreads) sslot[t] = __ldg(m.slot + t);
+    A.val = sval;
+    A.col = scol;
+    A.goff = sgoff;
+    A.slot = sslot;
+    A.sh = &shared;
+    A.lane = tid & 31;
+    A.warp = tid >> 5;
+    A.buf = 0;
+    A.g0 = __ldg(m.wgrp + A.warp);
+    A.g1 = __ldg(m.wgrp + A.warp + 1);
+    int pm[E];
+    double b[E], x[E], r[E], p[E], q[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int t = tid + kEllThreads * e;
+        const bool in = t < kEllThreads * m.layers;
+        A.rows[e] = in ? __ldg(m.rows + t) : 0;
+        pm[e] = in ? __ldg(m.perm + t) : -1;
+        const unsigned n = (unsigned)A.rows[e] >> 16;
+        A.most[e] = (int)__reduce_max_sync(0xffffffffu, n <= (unsigned)kEllLongRow ? n : 0u);
+        A.wide[e] = __any_sync(0xffffffffu, n > (unsigned)kEllLongRow);
+        b[e] = pm[e] >= 0 ? (double)bg[pm[e]] : 0.0;
+        x[e] = 0.0;
+        r[e] = b[e];  // the correction starts at zero
+    }
+    double rnorm = 0.0;
+    double rho = A.dot_max(r, r, r, rnorm);
+    const double rnorm0 = rnorm, stop = a.reltol * rnorm0;
+    int ret = 0;
+    if (!is_zero(rnorm0)) {
+        if (a.bottom == 0) {
+            double rho_1 = 0.0, inv_1 = 0.0;
+            for (int iter = 1; iter <= a.maxiter; ++iter) {
+                if (is_zero(rho)) { ret = 1; break; }
+                if (iter == 1) {
+#pragma unroll
+                    for (int e = 0; e < E; ++e) p[e] = r[e];
+                } else {
+                    const double beta = div_by(rho, rho_1, inv_1);
+#pragma unroll
+                    for (int e = 0; e < E; ++e) p[e] = fma(beta, p[e], r[e]);
+                }
+                A.apply(p, q);
+                const double pw = A.dot(p, q);
+                if (is_zero(pw)) { ret = 1; break; }
+                double alpha;
+                div2(rho, pw, 1.0, rho, A.lane, alpha, inv_1);
+#pragma unroll
+                for (int e = 0; e < E; ++e) r[e] = fma(-alpha, q[e], r[e]);
+                rho_1 = rho;
+                rho = A.dot_max(r, r, r, rnorm);
+#pragma unroll
+                for (int e = 0; e < E; ++e) x[e] = fma(alpha, p[e], x[e]);
+                if (lt_bits(rnorm, stop)) break;
+            }
+        } else {
+            double rh[E], v[E], tt[E];
+            double rho_1 = 0.0, inv_1 = 0.0, alpha = 0.0, omega = 0.0, inv_omega = 0.0;
+#pragma unroll
+            for (int e = 0; e < E; ++e) { rh[e] = r[e]; p[e] = 0.0; v[e] = 0.0; }
+            for (int iter = 1; iter <= a.maxiter; ++iter) {
+                if (is_zero(rho)) { ret = 1; break; }
+                if (iter == 1) {
+#pragma unroll
+                    for (int e = 0; e < E; ++e) p[e] = r[e];
+                } else {
+                    const double beta = div_by(rho, rho_1, inv_1) * div_by(alpha, omega, inv_omega);
+#pragma unroll
+                    for (int e = 0; e < E; ++e) p[e] = fma(beta, fma(-omega, v[e], p[e]), r[e]);
+                }
+                A.apply(p, v);
+                const double rhTv = A.dot(rh, v);
+                if (is_zero(rhTv)) { ret = 2; break; }
+                div2(rho, rhTv, 1.0, rho, A.lane, alpha, inv_1);
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    r[e] = fma(-alpha, v[e], r[e]);
+                    x[e] = fma(alpha, p[e], x[e]);
+                }
+                // the max-norm of r ends the iteration when it is small; t = A r does no harm then
+                A.apply(r, tt);
+                const double t_t = A.dot_max(tt, tt, r, rnorm);
+                if (lt_bits(rnorm, stop)) break;
+                const double t_r = A.dot(tt, r);
+                if (is_zero(t_t)) { ret = 3; break; }
+                div2(t_r, t_t, t_t, t_r, A.lane, omega, inv_omega);
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    x[e] = fma(omega, r[e], x[e]);
+                    r[e] = fma(-omega, tt[e], r[e]);
+                }
+                rho_1 = rho;
+                rho = A.dot_max(rh, r, r, rnorm);
+                if (lt_bits(rnorm, stop)) break;
+                if (is_zero(omega)) { ret = 4; break; }
+            }
+        }
+        if (ret == 0 && lt_bits(stop, rnorm)) ret = 8;
+    }
+    // MLMG: the correction is kept when the residual fell, and on failure nuf smoother calls from
+    // zero take its place
+    const bool keep = ret == 0 && lt_bits(rnorm, rnorm0);
+    if (ret != 0) {
+        double D[E], I[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            x[e] = 0.0;
+            D[e] = pm[e] >= 0 ? __ldg(a.D + pm[e]) : 0.0;
+            I[e] = pm[e] >= 0 ? __ldg(a.invD + pm[e]) : 0.0;
+        }
+        for (int s = 0; s < a.nuf * a.sweeps; ++s) {
+            A.apply(x, q);
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const double rx = q[e] - x[e] * D[e];
+                x[e] = (1.0 - a.omega) * x[e] + a.omega * (b[e] - rx) * I[e];
+            }
+        }
+        if (tid == 0 && a.fail_count) atomicAdd(a.fail_count, 1);
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+        if (pm[e] >= 0) xg[pm[e]] = (R)(ret != 0 || keep ? x[e] : 0.0);
+}
+
+namespace {
+constexpr size_t kQuadSmemMax = 200 * 1024;
+// E: the instantiations (layers rounded up)
+template <class F>
+void quad_by_layers(int layers, F&& f) {
+    if (layers <= 1) f(std::integral_constant<int, 1>());
+    else if (layers <= 2) f(std::integral_constant<int, 2>());
+    else if (layers <= 3) f(std::integral_constant<int, 3>());
+    else f(std::integral_constant<int, kBottomQuadLayers>());
+}
+template <int E>
+size_t quad_smem_bytes(const BottomEll& m) {
+    return sizeof(double) * (size_t)(m.nval + m.nchunk + kEllThreads * E) + sizeof(int) * (size_t)(33 * m.ngroups + 1) +
+           sizeof(unsigned short) * (size_t)m.nval;
+}
+}  // namespace
+
+bool bottom_quad_init(const BottomEll& m) {
+    if (m.layers > kBottomQuadLayers) return false;
+    bool ok = false;
+    quad_by_layers(m.layers, [&](auto e) {
+        constexpr int E = decltype(e)::value;
+        const size_t bytes = quad_smem_bytes<E>(m);
+        ok = bytes <= kQuadSmemMax;
+        if (ok && bytes > kBottomSmemBytes) {  // beyond the default: raise the limit, once and for all sizes
+            AE_CUDA_CHECK(cudaFuncSetAttribute(k_bottom_quad<double, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)kQuadSmemMax));
+            AE_CUDA_CHECK(cudaFuncSetAttribute(k_bottom_quad<float, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)kQuadSmemMax));
+        }
+    });
+    return ok;
+}
+
+template <class R>
+void launch_bottom_quad(const BottomArgs& a, const BottomEll& m, const R* b, R* x, cudaStream_t st) {
+    quad_by_layers(m.layers, [&](auto e) {
+        constexpr int E = decltype(e)::value;
+        k_bottom_quad<R, E><<<1, kEllThreads, quad_smem_bytes<E>(m), st>>>(a, m, b, x);
+    });
+    launched();
+}
+template void launch_bottom_quad<double>(const BottomArgs&, const BottomEll&, const double*, double*, cudaStream_t);
+template void launch_bottom_quad<float>(const BottomArgs&, const BottomEll&, const float*, float*, cudaStream_t);
 
 // Linear::solveaffine's right-hand side (src/Solver/Nonlocal/Linear.H:62-89): with r = 0 - A 0,
 // the negated apply of zero, rhs += r on nodes inside the domain, nothing on its boundary.

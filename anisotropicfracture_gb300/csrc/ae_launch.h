@@ -218,7 +218,7 @@ void launch_bottom(const BottomArgs& a, cudaStream_t st);
 void launch_ring_interp_fix(const Geo& gf, View<double> x, View<const float> ecrse, View<const float> efine,
                             cudaStream_t st);
 // Coarsest-level operator assembled as an FP64 CSR matrix (rows = unknowns t + c nn), used by the
-// bottom solve of the FP32 cycle.  The dense form comes first: column j of the row-major N x N
+// bottom solve.  The dense form comes first: column j of the row-major N x N
 // matrix A is the operator applied to e_j (E: N x N scratch for the unit vectors).
 struct BottomCsr {
     const int* rowptr;
@@ -236,6 +236,25 @@ struct BottomCsr {
 constexpr int kCsrChunk = 8;
 void launch_bottom_assemble(const BottomArgs& a, double* A, double* E, cudaStream_t st);
 void launch_bottom_csr(const BottomArgs& a, const BottomCsr& m, cudaStream_t st);
+// The same matrix laid out for the four-warp bottom solve (ae_bottom_ell.h): unknowns in slots of
+// 128 threads, rows cut into chunks, chunks in groups of 32.
+struct BottomEll {
+    const double* val;
+    const unsigned short* col;
+    const int* goff;   // [ngroups + 1] first entry of each group
+    const int* slot;   // [32 ngroups] chunk | (length + 1) << 16
+    const int* wgrp;   // [5] first group of each warp
+    const int* rows;   // [128 layers] first chunk | number of chunks << 16
+    const int* perm;   // [128 layers] unknown of each slot, -1: none
+    int nval, ngroups, nchunk, layers;
+};
+constexpr int kBottomQuadLayers = 6;  // unknowns per thread
+// whether the matrix fits the kernel's shared memory; call once before the first launch (it sets the
+// kernels' shared-memory attribute)
+bool bottom_quad_init(const BottomEll& m);
+// x = bottom solve of A x = b from x = 0, b and x in the cycle's precision
+template <class R>
+void launch_bottom_quad(const BottomArgs& a, const BottomEll& m, const R* b, R* x, cudaStream_t st);
 // unknowns up to which the coarsest level is assembled (dense scratch 2 N^2 doubles at set-up)
 constexpr long long kBottomCsrMaxN = 1536;
 
