@@ -88,7 +88,7 @@ struct MGLevel {
     long long nn = 0;
     double *C = nullptr, *D = nullptr, *invD = nullptr;
     double *res = nullptr, *cor = nullptr, *rescor = nullptr, *corhold = nullptr, *tmp = nullptr;
-    float *C32 = nullptr, *D32 = nullptr, *invD32 = nullptr;
+    float *C32 = nullptr, *invD32 = nullptr;
     float *res32 = nullptr, *cor32 = nullptr, *rescor32 = nullptr, *corhold32 = nullptr, *tmp32 = nullptr;
     // Voronoi stiffness (finest MG level of an AMR level, ae_op_set_model_grains): grain id per
     // node laid out like C, per-grain tables; the sweeps read these instead of C / C32
@@ -177,9 +177,7 @@ struct ae_op_s {
     ~ae_op_s() {
         for (auto& A : amr)
             for (auto& L : A.mg) {
-                if (L.split.list) cudaFree(L.split.list);
-                if (L.split.list_r) cudaFree(L.split.list_r);
-                if (L.split.gidm) cudaFree(L.split.gidm);
+                split_free(L.split);
             }
         for (void* p : allocs) cudaFree(p);
         if (stage) cudaFree(stage);
@@ -340,7 +338,6 @@ void alloc_level_fp32(ae_op* op) {
     for (auto& A : op->amr)
         for (auto& L : A.mg) {
             L.C32 = op->alloc<float>(op->ncoef * L.nn);
-            L.D32 = op->alloc<float>(3 * L.nn);
             L.invD32 = op->alloc<float>(3 * L.nn);
             L.res32 = op->alloc<float>(3 * L.nn);
             L.cor32 = op->alloc<float>(3 * L.nn);
@@ -471,7 +468,7 @@ void assemble_bottom(ae_op* op) {
     upload_bottom_ell(op, L, rp, cl, vl);
 }
 
-// FP32 copies of the stiffness and diagonal on every level (mixed-precision cycle)
+// FP32 copies of the stiffness and 1 / diagonal on every level (mixed-precision cycle)
 void prepare32(ae_op* op) {
     alloc_level_fp32(op);
     if (op->prepared32) return;
@@ -479,7 +476,6 @@ void prepare32(ae_op* op) {
         for (auto& L : A.mg) {
             const Box3 s = geo_store(L.g);
             launch_copy<float, double>(s, op->ncoef, level_view(L.g, L.C32), cview(level_view(L.g, L.C)), op->st);
-            launch_copy<float, double>(s, 3, level_view(L.g, L.D32), cview(level_view(L.g, L.D)), op->st);
             launch_copy<float, double>(s, 3, level_view(L.g, L.invD32), cview(level_view(L.g, L.invD)), op->st);
         }
     AE_CHECK(cudaStreamSynchronize(op->st));
@@ -494,7 +490,8 @@ void build_splits(ae_op* op) {
         if (!L.grains || L.split_built || (L.g.ng != 0 && L.g.ng < 2) || L.ngrains > kSplitMaxGrains ||
             !split_supported(L.g))
             continue;
-        split_build(L.g, cview(level_view(L.g, L.gid)), L.split, op->st, op->dnorm + 7);
+        split_build(L.g, op->model, cview(level_view(L.g, L.gid)), L.ngrains, L.gtab64, L.split, op->st,
+                    op->dnorm + 7);
         if (const char* e = std::getenv("AE_SPLIT_KZ")) L.split.kz = std::atoi(e);
         L.split_built = true;
     }
@@ -540,10 +537,7 @@ void prepare(ae_op* op) {
     op->amr[0].mg.back().csr_built = false;
     for (auto& A : op->amr)
         for (auto& L : A.mg) {
-            if (L.split.list) AE_CHECK(cudaFree(L.split.list));
-            if (L.split.list_r) AE_CHECK(cudaFree(L.split.list_r));
-            if (L.split.gidm) AE_CHECK(cudaFree(L.split.gidm));
-            L.split = SplitList{};
+            split_free(L.split);
             L.split_built = false;
         }
     int flag = 0;
@@ -566,21 +560,21 @@ bool use_tiled(const ae_op* op) {
     return sizeof(R) == 4 ? op->tiled32 : op->tiled64;
 }
 template <class R>
-void sweep_jacobi(ae_op* op, const Geo& g, const R* C, const R* invD, const R* D, const R* xi, const R* b, R* xo,
+void sweep_jacobi(ae_op* op, const Geo& g, const R* C, const R* invD, const R* xi, const R* b, R* xo,
                   R omega, cudaStream_t st) {
     const OpParams P = op->params(g);
     if (use_tiled<R>(op))
         launch_tiled<R>(1, P, cview(level_view(g, const_cast<R*>(C))), cview(level_view(g, const_cast<R*>(xi))),
                         cview(level_view(g, const_cast<R*>(b))), cview(level_view(g, const_cast<R*>(invD))),
-                        cview(level_view(g, const_cast<R*>(D))), level_view(g, xo), omega, st);
+                        level_view(g, xo), omega, st);
     else if (const MGLevel* sl = op->split_for<R>(C))
         launch_jacobi_split<R>(P, sl->split, cview(level_view(g, const_cast<R*>(C))),
-                               cview(level_view(g, const_cast<R*>(invD))), cview(level_view(g, const_cast<R*>(D))),
+                               cview(level_view(g, const_cast<R*>(invD))),
                                cview(level_view(g, const_cast<R*>(xi))), cview(level_view(g, const_cast<R*>(b))),
                                level_view(g, xo), omega, st, op->grains_for<R>(C), sl->ngrains, op->dflag + 2);
     else
         launch_jacobi<R>(P, cview(level_view(g, const_cast<R*>(C))), cview(level_view(g, const_cast<R*>(invD))),
-                         cview(level_view(g, const_cast<R*>(D))), cview(level_view(g, const_cast<R*>(xi))),
+                         cview(level_view(g, const_cast<R*>(xi))),
                          cview(level_view(g, const_cast<R*>(b))), level_view(g, xo), omega, st,
                          op->grains_for<R>(C));
 }
@@ -591,7 +585,7 @@ void sweep_residual(ae_op* op, const Geo& g, const R* C, const R* x, const R* b,
     if (use_tiled<R>(op))
         launch_tiled<R>(2, P, cview(level_view(g, const_cast<R*>(C))), cview(level_view(g, const_cast<R*>(x))),
                         cview(level_view(g, const_cast<R*>(b))), cview(level_view(g, const_cast<R*>(b))),
-                        cview(level_view(g, const_cast<R*>(b))), level_view(g, r), R(0), st);
+                        level_view(g, r), R(0), st);
     else if (const MGLevel* sl = op->split_for<R>(C))
         launch_residual_split<R>(P, sl->split, cview(level_view(g, const_cast<R*>(C))),
                                  cview(level_view(g, const_cast<R*>(x))), cview(level_view(g, const_cast<R*>(b))),
@@ -607,7 +601,7 @@ void sweep_fapply(ae_op* op, const Geo& g, const R* C, const R* x, R* f, cudaStr
     if (use_tiled<R>(op))
         launch_tiled<R>(0, P, cview(level_view(g, const_cast<R*>(C))), cview(level_view(g, const_cast<R*>(x))),
                         cview(level_view(g, const_cast<R*>(x))), cview(level_view(g, const_cast<R*>(x))),
-                        cview(level_view(g, const_cast<R*>(x))), level_view(g, f), R(0), st);
+                        level_view(g, f), R(0), st);
     else if (const MGLevel* sl = op->split_for<R>(C))
         launch_fapply_split<R>(P, sl->split, cview(level_view(g, const_cast<R*>(C))),
                                cview(level_view(g, const_cast<R*>(x))), level_view(g, f), st, op->grains_for<R>(C),
@@ -620,17 +614,17 @@ void sweep_fapply(ae_op* op, const Geo& g, const R* C, const R* x, R* f, cudaStr
 // ------------------------------------------------------------------ the multigrid cycle
 template <class R>
 struct LevelPtrs {
-    R *C, *D, *invD, *res, *cor, *rescor, *corhold, *tmp;
+    R *C, *invD, *res, *cor, *rescor, *corhold, *tmp;
 };
 template <class R>
 LevelPtrs<R> ptrs(MGLevel& L);
 template <>
 LevelPtrs<double> ptrs<double>(MGLevel& L) {
-    return {L.C, L.D, L.invD, L.res, L.cor, L.rescor, L.corhold, L.tmp};
+    return {L.C, L.invD, L.res, L.cor, L.rescor, L.corhold, L.tmp};
 }
 template <>
 LevelPtrs<float> ptrs<float>(MGLevel& L) {
-    return {L.C32, L.D32, L.invD32, L.res32, L.cor32, L.rescor32, L.corhold32, L.tmp32};
+    return {L.C32, L.invD32, L.res32, L.cor32, L.rescor32, L.corhold32, L.tmp32};
 }
 
 template <class R>
@@ -650,10 +644,10 @@ struct Cycle {
         for (int s = 0; s < o.sweeps; ++s) {
             if (s == 0 && from_zero)
                 launch_jacobi_zero<R>(L.g, cview(level_view(L.g, const_cast<R*>(p.invD))),
-                                      cview(level_view(L.g, const_cast<R*>(p.D))), cview(level_view(L.g, const_cast<R*>(b))),
+                                      cview(level_view(L.g, const_cast<R*>(b))),
                                       level_view(L.g, t), (R)o.omega, st);
             else
-                sweep_jacobi<R>(op, L.g, p.C, p.invD, p.D, a, b, t, (R)o.omega, st);
+                sweep_jacobi<R>(op, L.g, p.C, p.invD, a, b, t, (R)o.omega, st);
             std::swap(a, t);
         }
         if (a != x) launch_copy<R, R>(geo_store(L.g), 3, level_view(L.g, x), cview(level_view(L.g, a)), st);
@@ -1248,8 +1242,9 @@ int ae_op_set_model_grains(ae_op* op, int amrlev, const ae_fab* grain_id, int ng
         const int nc = op->ncoef;
         if (!L.gid) L.gid = op->alloc<unsigned short>(L.nn);
         if (L.gcap < ngrains) {
-            L.gtab64 = op->alloc<double>((long long)ngrains * nc);
-            L.gtab32 = op->alloc<float>((long long)ngrains * nc);
+            // 4 more: the sweeps copy the tables in whole 16 bytes
+            L.gtab64 = op->alloc<double>((long long)ngrains * nc + 4);
+            L.gtab32 = op->alloc<float>((long long)ngrains * nc + 4);
             L.gcap = ngrains;
         }
         AE_CHECK(cudaMemcpyAsync(L.gtab64, table, sizeof(double) * ngrains * nc, cudaMemcpyDefault, op->st));
@@ -1499,7 +1494,7 @@ int ae_fsmooth(ae_op* op, int amrlev, int mglev, const ae_fab* x, const ae_fab* 
             R *a = p.tmp, *t = p.rescor;
             launch_copy<R, R>(s, 3, level_view(L.g, t), cview(level_view(L.g, a)), op->st);
             for (int sw = 0; sw < nsweeps; ++sw) {
-                sweep_jacobi<R>(op, L.g, p.C, p.invD, p.D, a, p.corhold, t, (R)omega, op->st);
+                sweep_jacobi<R>(op, L.g, p.C, p.invD, a, p.corhold, t, (R)omega, op->st);
                 std::swap(a, t);
             }
             launch_copy<R, R>(need, 3, fab_view<R>(*x), cview(level_view(L.g, a)), op->st);
@@ -1866,7 +1861,7 @@ int ae_profile_kernel(ae_op* op, int which, int amrlev, int mglev, int precision
             using R = decltype(zero);
             LevelPtrs<R> p = ptrs<R>(L);
             if (which == 0) sweep_fapply<R>(op, L.g, p.C, p.cor, p.tmp, st);
-            else if (which == 1) sweep_jacobi<R>(op, L.g, p.C, p.invD, p.D, p.cor, p.res, p.tmp, R(2.0 / 3.0), st);
+            else if (which == 1) sweep_jacobi<R>(op, L.g, p.C, p.invD, p.cor, p.res, p.tmp, R(2.0 / 3.0), st);
             else if (which == 2) sweep_residual<R>(op, L.g, p.C, p.cor, p.res, p.rescor, st);
             else {
                 MGLevel& Lc = op->amr[amrlev].mg[mglev + 1];

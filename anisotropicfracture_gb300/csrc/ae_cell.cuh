@@ -32,29 +32,17 @@ __device__ __forceinline__ void cell_ijk(const int n[3], int t, int& i, int& j, 
     i = r - j * n[0];
 }
 
-// central gradient and second derivatives of the three components of U at node t
+// the value of component p of U beside node t: u(p, a, b, c) for row_interior
 template <class R>
-__device__ __forceinline__ void cell_derivs(const SCoef<R>& K, const R* __restrict__ U, int us, int t, const POff& o,
-                                            R gu[3][3], R b[3][3][3]) {
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-        const R* up = U + p * us + t;
-        const R c0 = up[0];
-        const R xm = up[o.xm], xp = up[o.xp], ym = up[o.ym], yp = up[o.yp], zm = up[o.zm], zp = up[o.zp];
-        gu[p][0] = (xp - xm) * K.h[0];
-        gu[p][1] = (yp - ym) * K.h[1];
-        gu[p][2] = (zp - zm) * K.h[2];
-        b[p][0][0] = (xp - R(2) * c0 + xm) * K.i2[0];
-        b[p][1][1] = (yp - R(2) * c0 + ym) * K.i2[1];
-        b[p][2][2] = (zp - R(2) * c0 + zm) * K.i2[2];
-        b[p][0][1] = (up[o.xp + o.yp] + up[o.xm + o.ym] - up[o.xp + o.ym] - up[o.xm + o.yp]) * K.m01;
-        b[p][0][2] = (up[o.xp + o.zp] + up[o.xm + o.zm] - up[o.xp + o.zm] - up[o.xm + o.zp]) * K.m02;
-        b[p][1][2] = (up[o.yp + o.zp] + up[o.ym + o.zm] - up[o.yp + o.zm] - up[o.ym + o.zp]) * K.m12;
-        b[p][1][0] = b[p][0][1];
-        b[p][2][0] = b[p][0][2];
-        b[p][2][1] = b[p][1][2];
+struct CellAt {
+    const R* u;
+    int us;
+    const POff& o;
+    __device__ __forceinline__ R operator()(int p, int a, int b, int c) const {
+        return u[p * us + (a > 0 ? o.xp : a < 0 ? o.xm : 0) + (b > 0 ? o.yp : b < 0 ? o.ym : 0) +
+                 (c > 0 ? o.zp : c < 0 ? o.zm : 0)];
     }
-}
+};
 
 // sum_d column d of (d_d C) : g, central differences of C over the wrapped neighbours
 template <int M, class R, bool LDG = true>
@@ -69,62 +57,56 @@ __device__ __forceinline__ void cell_gradC(const SCoef<R>& K, const R* __restric
     for (int r = 0; r < 3; ++r) out[r] = gradc_sum(c_x[r], c_y[r], c_z[r], K.h);
 }
 
-// f = A u at node t of a periodic cell
+// A u = row_factor f at node t of a periodic cell
 template <int M, class R, bool LDG = true>
 __device__ __forceinline__ void cell_apply(const SCoef<R>& K, bool uniform, const R* __restrict__ C, int cs,
                                            const R* __restrict__ U, int us, int t, const POff& o, R f[3]) {
-    constexpr int NC = NCoef<M>::value;
-    R gu[3][3], b[3][3][3];
-    cell_derivs<R>(K, U, us, t, o, gu, b);
-    {
-        R a[NC];
-#pragma unroll
-        for (int q = 0; q < NC; ++q) a[q] = ldv<LDG>(C + q * cs + t);
-        div_of<M, R>(a, b, f);
-    }
+    R gu[3][3];
+    row_interior<M, R>(K, CellAt<R>{U + t, us, o}, [&](int q) { return ldv<LDG>(C + q * cs + t); }, gu, f);
     if (!uniform) {
-        R gc[3];
-        cell_gradC<M, R, LDG>(K, C, cs, t, o, gu, gc);
+        const R* c0 = C + t;
+        R cx[3], cy[3], cz[3];
+        grad_scale(K, gu);
+        gradC_col_f<M, R>([&](int q) { return ldv<LDG>(c0 + q * cs + o.xp) - ldv<LDG>(c0 + q * cs + o.xm); }, gu, 0, cx);
+        gradC_col_f<M, R>([&](int q) { return ldv<LDG>(c0 + q * cs + o.yp) - ldv<LDG>(c0 + q * cs + o.ym); }, gu, 1, cy);
+        gradC_col_f<M, R>([&](int q) { return ldv<LDG>(c0 + q * cs + o.zp) - ldv<LDG>(c0 + q * cs + o.zm); }, gu, 2, cz);
 #pragma unroll
-        for (int r = 0; r < 3; ++r) f[r] += gc[r];
+        for (int r = 0; r < 3; ++r) f[r] = row_gradc(K, f[r], cx[r], cy[r], cz[r]);
     }
 }
 
-// f = A u at node t of a Voronoi cell stored as a grain id per node and a per-grain coefficient
-// table (tab[g * ncoef + q]).  The arithmetic is that of cell_apply on the equivalent per-node
-// field; a direction whose two neighbours lie in the same grain has an exactly zero stiffness
-// difference, so its column of the grad C term is zero and its loads are skipped.
+// cell_apply of a Voronoi cell stored as a grain id per node and a per-grain coefficient table
+// (tab[g * ncoef + q]).  The arithmetic is that of cell_apply on the equivalent per-node field; a
+// direction whose two neighbours lie in the same grain has an exactly zero stiffness difference, so
+// its column of the grad C term is zero and its loads are skipped.
 template <int M, class R>
 __device__ __forceinline__ void cell_apply_grains(const SCoef<R>& K, bool uniform,
                                                   const unsigned short* __restrict__ gid,
                                                   const R* __restrict__ tab, const R* __restrict__ U, int us, int t,
                                                   const POff& o, R f[3]) {
     constexpr int NC = NCoef<M>::value;
-    R gu[3][3], b[3][3][3];
-    cell_derivs<R>(K, U, us, t, o, gu, b);
-    {
-        const R* a0 = tab + (int)__ldg(gid + t) * NC;
-        R a[NC];
-#pragma unroll
-        for (int q = 0; q < NC; ++q) a[q] = __ldg(a0 + q);
-        div_of<M, R>(a, b, f);
-    }
+    R gu[3][3];
+    const R* a0 = tab + (int)__ldg(gid + t) * NC;
+    row_interior<M, R>(K, CellAt<R>{U + t, us, o}, [&](int q) { return __ldg(a0 + q); }, gu, f);
     if (!uniform) {
         const int gp[3] = {__ldg(gid + t + o.xp), __ldg(gid + t + o.yp), __ldg(gid + t + o.zp)};
         const int gm[3] = {__ldg(gid + t + o.xm), __ldg(gid + t + o.ym), __ldg(gid + t + o.zm)};
-        R col[3][3];
+        if (gp[0] != gm[0] || gp[1] != gm[1] || gp[2] != gm[2]) {
+            R col[3][3];
+            grad_scale(K, gu);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            if (gp[d] == gm[d]) {
-                col[d][0] = col[d][1] = col[d][2] = R(0);
-            } else {
-                const R* cp = tab + gp[d] * NC;
-                const R* cm = tab + gm[d] * NC;
-                gradC_col_f<M, R>([&](int q) { return __ldg(cp + q) - __ldg(cm + q); }, gu, d, col[d]);
+            for (int d = 0; d < 3; ++d) {
+                if (gp[d] == gm[d]) {
+                    col[d][0] = col[d][1] = col[d][2] = R(0);
+                } else {
+                    const R* cp = tab + gp[d] * NC;
+                    const R* cm = tab + gm[d] * NC;
+                    gradC_col_f<M, R>([&](int q) { return __ldg(cp + q) - __ldg(cm + q); }, gu, d, col[d]);
+                }
             }
-        }
 #pragma unroll
-        for (int r = 0; r < 3; ++r) f[r] = gradc_add(f[r], col[0][r], col[1][r], col[2][r], K.h);
+            for (int r = 0; r < 3; ++r) f[r] = row_gradc(K, f[r], col[0][r], col[1][r], col[2][r]);
+        }
     }
 }
 

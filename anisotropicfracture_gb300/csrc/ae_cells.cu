@@ -34,21 +34,6 @@ namespace {
 
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
-template <class R>
-SCoef<R> scoef_dx(const double dx[3]) {
-    SCoef<R> K;
-    for (int d = 0; d < 3; ++d) {
-        K.h[d] = (R)(0.5 / dx[d]);
-        K.id[d] = (R)(1.0 / dx[d]);
-        K.i2[d] = (R)(1.0 / (dx[d] * dx[d]));
-        K.bb[d] = (R)(-2.0 / dx[d] / dx[d]);
-    }
-    K.m01 = (R)(0.25 / (dx[0] * dx[1]));
-    K.m02 = (R)(0.25 / (dx[0] * dx[2]));
-    K.m12 = (R)(0.25 / (dx[1] * dx[2]));
-    return K;
-}
-
 int ncoef_of(int model) { return model == AE_MODEL_ISOTROPIC ? 2 : model == AE_MODEL_MAJORMINOR ? 21 : 9; }
 
 // Lays out one cell in `base` (nullptr: dry run).  Returns the bytes used.
@@ -74,8 +59,8 @@ size_t cell_layout(CellRes& c, char* base) {
         L.I64 = (double*)take(sizeof(double) * 3 * nn);
         L.C32 = (float*)take(sizeof(float) * nc * nn);
         L.I32 = (float*)take(sizeof(float) * 3 * nn);
-        L.K64 = scoef_dx<double>(dx);
-        L.K32 = scoef_dx<float>(dx);
+        L.K64 = scoef_of<double>(dx);
+        L.K32 = scoef_of<float>(dx);
         L.gid = nullptr;
         L.ngrains = 0;
         L.tab64 = nullptr;

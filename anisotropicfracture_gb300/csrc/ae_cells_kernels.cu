@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, GR>()) kb_smo
         const int ds = grains ? 1 : nn;  // component stride of invD / D
         if (ZERO) {
 #pragma unroll
-            for (int p = 0; p < 3; ++p) xout[p * nn + t] = (omega * b[p * nn + t]) * invD[p * ds];
+            for (int p = 0; p < 3; ++p) xout[p * nn + t] = jacobi_update<R>(R(0), b[p * nn + t], invD[p * ds], omega);
             continue;
         }
         int i, j, k;
@@ -110,18 +110,10 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, GR>()) kb_smo
         const POff o = cell_offsets(L.n, i, j, k);
         R f[3];
         level_apply<M, R, GR>(L, A.uniform, xin, t, o, f);
+        const R sc = row_factor(kfield<R>(L));
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
-            const R xv = xin[p * nn + t];
-            if constexpr (sizeof(R) == 8) {
-                // the reference's update, (1-w) x + w (b - (Ax - D x)) / D (Operator.cpp:154)
-                const R Dv = grains ? L.dtab64[g3 + p] : L.D64[p * nn + t];
-                const R rx = f[p] - xv * Dv;
-                xout[p * nn + t] = (R(1) - omega) * xv + omega * (b[p * nn + t] - rx) * invD[p * ds];
-            } else {
-                xout[p * nn + t] = xv + omega * (b[p * nn + t] - f[p]) * invD[p * ds];
-            }
-        }
+        for (int p = 0; p < 3; ++p)
+            xout[p * nn + t] = jacobi_update<R>(xin[p * nn + t], row_residual(b[p * nn + t], sc, f[p]), invD[p * ds], omega);
     }
 }
 
@@ -163,8 +155,9 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, GR>()) kb_res
         R f[3];
         level_apply<M, R, GR>(L, A.uniform, V.cor, t, o, f);
         R* out = inplace ? V.res : V.rescor;
+        const R sc = row_factor(kfield<R>(L));
 #pragma unroll
-        for (int p = 0; p < 3; ++p) out[p * nn + t] = V.res[p * nn + t] - f[p];
+        for (int p = 0; p < 3; ++p) out[p * nn + t] = row_residual(V.res[p * nn + t], sc, f[p]);
     }
 }
 
@@ -229,9 +222,8 @@ struct CellBottomOps {
             const POff o = cell_offsets(n, i, j, k);
             double f[3];
             cell_apply<M, double, LDG>(K, uniform, C, nn, x, nn, t, o, f);
-            out[t] = f[0];
-            out[t + nn] = f[1];
-            out[t + 2 * nn] = f[2];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) out[t + p * nn] = mul_rn(K.i2[0], f[p]);
         }
         __syncthreads();
     }
@@ -373,7 +365,7 @@ __global__ void __launch_bounds__(kCellThreads) kb_resid_top(CellArgs A, const W
             level_apply<M, double, GR>(L, A.uniform, S.x, t, o, f);
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
-                v[p] = S.b[p * nn + t] - f[p];
+                v[p] = row_residual(S.b[p * nn + t], L.K64.i2[0], f[p]);
                 S.r[p * nn + t] = v[p];
             }
         }

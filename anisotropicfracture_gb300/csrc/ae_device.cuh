@@ -29,45 +29,42 @@ __host__ __device__ constexpr int major_slot(int I, int K) {
     return I <= K ? I * 9 - I * (I - 1) / 2 + (K - I) : K * 9 - K * (K - 1) / 2 + (I - K);
 }
 
-// FP32 rows in one fixed rounding order.  The compiler fuses a product into a neighbouring
-// addition at its own discretion, and the choice can differ between kernels that inline the same
-// expression in different surroundings.  The FP32 operator's sums of products therefore go through
-// explicitly rounded operations -- additions rounded, the first product of a sum rounded and each
-// further one fused into the running sum -- so that every FP32 kernel computes a node's row to the
-// same bits.  FP64 keeps the written expressions.
-__device__ __forceinline__ float fx_sop_acc(float r) { return r; }
-template <class... T>
-__device__ __forceinline__ float fx_sop_acc(float r, float a, float x, T... rest) {
-    return fx_sop_acc(__fmaf_rn(a, x, r), rest...);
+// Rows in one fixed rounding order.  The compiler fuses a product into a neighbouring addition at its
+// own discretion, and the choice can differ between kernels that inline the same expression in
+// different surroundings.  The operator's interior rows therefore go through explicitly rounded
+// operations, so that every kernel computes a node's row to the same bits.
+__device__ __forceinline__ float mul_rn(float x, float y) { return __fmul_rn(x, y); }
+__device__ __forceinline__ double mul_rn(double x, double y) { return __dmul_rn(x, y); }
+__device__ __forceinline__ float add_rn(float x, float y) { return __fadd_rn(x, y); }
+__device__ __forceinline__ double add_rn(double x, double y) { return __dadd_rn(x, y); }
+__device__ __forceinline__ float sub_rn(float x, float y) { return __fsub_rn(x, y); }
+__device__ __forceinline__ double sub_rn(double x, double y) { return __dsub_rn(x, y); }
+__device__ __forceinline__ float fma_rn(float x, float y, float z) { return __fmaf_rn(x, y, z); }
+__device__ __forceinline__ double fma_rn(double x, double y, double z) { return __fma_rn(x, y, z); }
+template <class R>
+__device__ __forceinline__ R fx_sop_acc(R r) { return r; }
+template <class R, class... T>
+__device__ __forceinline__ R fx_sop_acc(R r, R a, R x, T... rest) {
+    return fx_sop_acc(fma_rn(a, x, r), rest...);
 }
-// a0 x0 + a1 x1 + ... in that order
-template <class... T>
-__device__ __forceinline__ float fx_sop(float a, float x, T... rest) {
-    return fx_sop_acc(__fmul_rn(a, x), rest...);
+// a0 x0 + a1 x1 + ... in that order: the first product rounded, each further one fused into the sum
+template <class R, class... T>
+__device__ __forceinline__ R fx_sop(R a, R x, T... rest) {
+    return fx_sop_acc(mul_rn(a, x), rest...);
 }
 template <class R>
-__device__ __forceinline__ R add2(R x, R y) {
-    if constexpr (sizeof(R) == 4) return __fadd_rn(x, y);
-    else return x + y;
-}
+__device__ __forceinline__ R add2(R x, R y) { return add_rn(x, y); }
 // a0 x0 + ... + a5 x5 (one row of a MajorMinor contraction)
 template <class R>
 __device__ __forceinline__ R sop6(R a0, R x0, R a1, R x1, R a2, R x2, R a3, R x3, R a4, R x4, R a5, R x5) {
-    if constexpr (sizeof(R) == 4) return fx_sop(a0, x0, a1, x1, a2, x2, a3, x3, a4, x4, a5, x5);
-    else return a0 * x0 + a1 * x1 + a2 * x2 + a3 * x3 + a4 * x4 + a5 * x5;
+    return fx_sop(a0, x0, a1, x1, a2, x2, a3, x3, a4, x4, a5, x5);
 }
 // (c0 h0 + c1 h1) + c2 h2: the grad C columns of a row scaled by the central-difference factors
 template <class R>
-__device__ __forceinline__ R gradc_sum(R c0, R c1, R c2, const R h[3]) {
-    if constexpr (sizeof(R) == 4) return fx_sop(c0, h[0], c1, h[1], c2, h[2]);
-    else return (c0 * h[0] + c1 * h[1]) + c2 * h[2];
-}
+__device__ __forceinline__ R gradc_sum(R c0, R c1, R c2, const R h[3]) { return fx_sop(c0, h[0], c1, h[1], c2, h[2]); }
 // f + the grad C term of the row
 template <class R>
-__device__ __forceinline__ R gradc_add(R f, R c0, R c1, R c2, const R h[3]) {
-    if constexpr (sizeof(R) == 4) return __fadd_rn(f, gradc_sum(c0, c1, c2, h));
-    else return f + ((c0 * h[0] + c1 * h[1]) + c2 * h[2]);
-}
+__device__ __forceinline__ R gradc_add(R f, R c0, R c1, R c2, const R h[3]) { return add_rn(f, gradc_sum(c0, c1, c2, h)); }
 
 enum BCType { DISP = 0, TRAC = 1, PERIODIC = 2, NEUMANN = 3 };
 
@@ -105,7 +102,30 @@ struct SCoef {
     R i2[3];       // 1 / dx^2   (second derivative)
     R m01, m02, m12;  // 0.25 / (dx_a dx_b)  (mixed derivative)
     R bb[3];       // -2 / dx / dx  (diagonal of the second derivative)
+    // the interior row as i2[0] times a row of unscaled differences (row_of below)
+    R q[3];        // dx_0 / dx_d
+    R sd[6];       // q factors of the differences xx, yy, zz, xy, xz, yz (1/4 of the mixed ones apart)
+    int iso;       // equal spacing: every q is 1
 };
+// fills the members for the spacing dx (host)
+template <class R>
+inline SCoef<R> scoef_of(const double dx[3]) {
+    SCoef<R> K;
+    for (int d = 0; d < 3; ++d) {
+        K.h[d] = (R)(0.5 / dx[d]);
+        K.id[d] = (R)(1.0 / dx[d]);
+        K.i2[d] = (R)(1.0 / (dx[d] * dx[d]));
+        K.bb[d] = (R)(-2.0 / dx[d] / dx[d]);
+        K.q[d] = (R)(dx[0] / dx[d]);
+    }
+    K.m01 = (R)(0.25 / (dx[0] * dx[1]));
+    K.m02 = (R)(0.25 / (dx[0] * dx[2]));
+    K.m12 = (R)(0.25 / (dx[1] * dx[2]));
+    const int a[6] = {0, 1, 2, 0, 0, 1}, b[6] = {0, 1, 2, 1, 2, 2};
+    for (int s = 0; s < 6; ++s) K.sd[s] = (R)((dx[0] / dx[a[s]]) * (dx[0] / dx[b[s]]));
+    K.iso = dx[0] == dx[1] && dx[0] == dx[2];
+    return K;
+}
 
 // BC types per face (26) and direction (3).
 struct BCP {
@@ -342,28 +362,20 @@ __device__ __forceinline__ void gradC_col(const R* __restrict__ C, long long cs,
 #pragma unroll
             for (int k = 0; k < 3; ++k)
 #pragma unroll
-                for (int l = 0; l < 3; ++l) v += DC(major_slot(3 * r + d, 3 * k + l)) * g[k][l];
+                for (int l = 0; l < 3; ++l) v = fma_rn(DC(major_slot(3 * r + d, 3 * k + l)), g[k][l], v);
             col[r] = v;
         }
     } else if (M == ISO) {
         const R dl = DC(0), dm = DC(1);
-        const R tr = dl * (g[0][0] + g[1][1] + g[2][2]);
-        if (d == 0) {
-            col[0] = tr + R(2) * dm * g[0][0];
-            col[1] = dm * (g[0][1] + g[1][0]);
-            col[2] = dm * (g[2][0] + g[0][2]);
-        } else if (d == 1) {
-            col[0] = dm * (g[0][1] + g[1][0]);
-            col[1] = tr + R(2) * dm * g[1][1];
-            col[2] = dm * (g[1][2] + g[2][1]);
-        } else {
-            col[0] = dm * (g[2][0] + g[0][2]);
-            col[1] = dm * (g[1][2] + g[2][1]);
-            col[2] = tr + R(2) * dm * g[2][2];
-        }
+        const R tr = mul_rn(dl, add_rn(add_rn(g[0][0], g[1][1]), g[2][2])), dm2 = add_rn(dm, dm);
+        const R s01 = mul_rn(dm, add_rn(g[0][1], g[1][0])), s02 = mul_rn(dm, add_rn(g[2][0], g[0][2]));
+        const R s12 = mul_rn(dm, add_rn(g[1][2], g[2][1]));
+        col[0] = d == 0 ? fma_rn(dm2, g[0][0], tr) : d == 1 ? s01 : s02;
+        col[1] = d == 0 ? s01 : d == 1 ? fma_rn(dm2, g[1][1], tr) : s12;
+        col[2] = d == 0 ? s02 : d == 1 ? s12 : fma_rn(dm2, g[2][2], tr);
     } else {
 #pragma unroll
-        for (int r = 0; r < 3; ++r) col[r] = DC(3 * r + d) * g[r][d];
+        for (int r = 0; r < 3; ++r) col[r] = mul_rn(DC(3 * r + d), g[r][d]);
     }
 #undef DC
 }
@@ -401,28 +413,20 @@ __device__ __forceinline__ void gradC_col_f(F&& dC, const R g[3][3], int d, R co
 #pragma unroll
             for (int k = 0; k < 3; ++k)
 #pragma unroll
-                for (int l = 0; l < 3; ++l) v += dC(major_slot(3 * r + d, 3 * k + l)) * g[k][l];
+                for (int l = 0; l < 3; ++l) v = fma_rn(dC(major_slot(3 * r + d, 3 * k + l)), g[k][l], v);
             col[r] = v;
         }
     } else if (M == ISO) {
         const R dl = dC(0), dm = dC(1);
-        const R tr = dl * (g[0][0] + g[1][1] + g[2][2]);
-        if (d == 0) {
-            col[0] = tr + R(2) * dm * g[0][0];
-            col[1] = dm * (g[0][1] + g[1][0]);
-            col[2] = dm * (g[2][0] + g[0][2]);
-        } else if (d == 1) {
-            col[0] = dm * (g[0][1] + g[1][0]);
-            col[1] = tr + R(2) * dm * g[1][1];
-            col[2] = dm * (g[1][2] + g[2][1]);
-        } else {
-            col[0] = dm * (g[2][0] + g[0][2]);
-            col[1] = dm * (g[1][2] + g[2][1]);
-            col[2] = tr + R(2) * dm * g[2][2];
-        }
+        const R tr = mul_rn(dl, add_rn(add_rn(g[0][0], g[1][1]), g[2][2])), dm2 = add_rn(dm, dm);
+        const R s01 = mul_rn(dm, add_rn(g[0][1], g[1][0])), s02 = mul_rn(dm, add_rn(g[2][0], g[0][2]));
+        const R s12 = mul_rn(dm, add_rn(g[1][2], g[2][1]));
+        col[0] = d == 0 ? fma_rn(dm2, g[0][0], tr) : d == 1 ? s01 : s02;
+        col[1] = d == 0 ? s01 : d == 1 ? fma_rn(dm2, g[1][1], tr) : s12;
+        col[2] = d == 0 ? s02 : d == 1 ? s12 : fma_rn(dm2, g[2][2], tr);
     } else {
 #pragma unroll
-        for (int r = 0; r < 3; ++r) col[r] = dC(3 * r + d) * g[r][d];
+        for (int r = 0; r < 3; ++r) col[r] = mul_rn(dC(3 * r + d), g[r][d]);
     }
 }
 
@@ -452,13 +456,196 @@ __device__ __forceinline__ constexpr int zslot_index(int q) {
     return -1;
 }
 
+// ------------------------------------------------------------------ the interior row
+// C : grad grad u + sum_d (d_d C : grad u) e_d, written to take few operations (GB300 issues FP64 at
+// 1/64 of its FP32 rate, so the FP64 sweeps are bound by their number):
+//   - differences are not scaled one by one: a row is i2[0] times a sum over the unscaled differences
+//     (with unequal spacing scaled by ratios of the spacings), the mixed ones times 1/4;
+//   - the products run over the differences, not over the slots: row i is the sum over k and the six
+//     (l, j) of A_ik,lj u_k,lj with A_ik,lj = C_ijkl + C_ilkj for l != j, C_ilkl for l = j, which is
+//     symmetric in i and k (36 numbers, from a table for a grain map).
+// MajorMinor: 45 + 60 FP64 operations a node on a grain map, against 154 before; the difference of a
+// pair comes first, so a smooth field's differences are exact.  FP32 keeps div_of over scaled
+// differences: it is not bound by operations, and reads 21 coefficients a node instead of 36.
+enum { kXX = 0, kYY = 1, kZZ = 2, kXY = 3, kXZ = 4, kYZ = 5 };
+
+// D: the six second differences of each component, g: its three central differences, from
+// u(p, di, dj, dk)
+template <class R, class U>
+__device__ __forceinline__ void row_diffs(const SCoef<R>&, U&& u, R D[3][6], R g[3][3]) {
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        const R c = u(p, 0, 0, 0);
+        const R xm = u(p, -1, 0, 0), xp = u(p, 1, 0, 0), ym = u(p, 0, -1, 0), yp = u(p, 0, 1, 0), zm = u(p, 0, 0, -1),
+                zp = u(p, 0, 0, 1);
+        g[p][0] = sub_rn(xp, xm);
+        g[p][1] = sub_rn(yp, ym);
+        g[p][2] = sub_rn(zp, zm);
+        D[p][kXX] = add_rn(fma_rn(R(-2), c, xp), xm);
+        D[p][kYY] = add_rn(fma_rn(R(-2), c, yp), ym);
+        D[p][kZZ] = add_rn(fma_rn(R(-2), c, zp), zm);
+        D[p][kXY] = sub_rn(sub_rn(u(p, 1, 1, 0), u(p, 1, -1, 0)), sub_rn(u(p, -1, 1, 0), u(p, -1, -1, 0)));
+        D[p][kXZ] = sub_rn(sub_rn(u(p, 1, 0, 1), u(p, -1, 0, 1)), sub_rn(u(p, 1, 0, -1), u(p, -1, 0, -1)));
+        D[p][kYZ] = sub_rn(sub_rn(u(p, 0, 1, 1), u(p, 0, -1, 1)), sub_rn(u(p, 0, 1, -1), u(p, 0, -1, -1)));
+    }
+}
+template <class R>
+__device__ __forceinline__ void row_scale(const SCoef<R>& K, R D[3][6]) {
+    if (K.iso) return;
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+#pragma unroll
+        for (int s = 1; s < 6; ++s) D[p][s] = mul_rn(D[p][s], K.sd[s]);
+}
+// (FP64: row_interior's FP32 differences are scaled already)
+template <class R>
+__device__ __forceinline__ void grad_scale(const SCoef<R>& K, R g[3][3]) {
+    if (sizeof(R) == 4 || K.iso) return;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        g[p][1] = mul_rn(g[p][1], K.q[1]);
+        g[p][2] = mul_rn(g[p][2], K.q[2]);
+    }
+}
+
+// (written without recursion, so that unrolled loops see constants)
+__host__ __device__ constexpr int pair_index(int i, int j) {
+    return (i < j ? i : j) == 0 ? (i < j ? j : i) : i + j + 1;
+}
+__host__ __device__ constexpr int pair_slot(int p, int q) {
+    return (p < q ? p : q) * 6 - (p < q ? p : q) * ((p < q ? p : q) - 1) / 2 + (p < q ? q : p) - (p < q ? p : q);
+}
+__host__ __device__ constexpr int mm_slot(int i, int j, int k, int l) {
+    return pair_slot(pair_index(i, j), pair_index(k, l));
+}
+static_assert(pair_index(1, 1) == 3 && pair_index(2, 1) == 4 && pair_index(2, 2) == 5 && mm_slot(2, 2, 2, 2) == 20 &&
+                  mm_slot(1, 0, 2, 1) == 9 && mm_slot(1, 2, 0, 0) == 4,
+              "slot order of Matrix4<3, MajorMinor>");
+template <int M>
+__host__ __device__ constexpr int slot_of(int i, int j, int k, int l) {
+    return M == MAJOR ? major_slot(3 * i + j, 3 * k + l) : mm_slot(i, j, k, l);
+}
+__host__ __device__ constexpr int ik_row(int n) { return n < 3 ? 0 : n < 5 ? 1 : 2; }
+__host__ __device__ constexpr int ik_col(int n) { return n < 3 ? n : n < 5 ? n - 2 : 2; }
+__host__ __device__ constexpr int diff_a(int s) { return s < 3 ? s : s < 5 ? 0 : 1; }
+__host__ __device__ constexpr int diff_b(int s) { return s < 3 ? s : s == 3 ? 1 : 2; }
+// coefficient 6 n + s of a row: n the pair (i, k) in the order 00 01 02 11 12 22, s the difference;
+// a(q): slot q of the stiffness
+template <int M, class A>
+__device__ __forceinline__ auto row_coef(A&& a, int n, int s) {
+    const int i = ik_row(n), k = ik_col(n), l = diff_a(s), j = diff_b(s);
+    const auto c = a(slot_of<M>(i, j, k, l));
+    return l == j ? c : add_rn(c, a(slot_of<M>(i, l, k, j)));
+}
+
+// numbers a row takes per node or grain: the 36 sums (MajorMinor, Major), or the slots themselves
+template <int M> struct RowN { static constexpr int value = 36; };
+template <> struct RowN<ISO> { static constexpr int value = 2; };
+template <> struct RowN<DIAG> { static constexpr int value = 9; };
+
+// F / i2[0] of the interior term from the differences; r(n): number n of the row
+template <int M, class A>
+__device__ __forceinline__ void row_sum(A&& r, const double D[3][6], double F[3]) {
+    if constexpr (M == ISO) {
+        const double lam = r(0), mu = r(1), lm = add_rn(lam, mu);
+        const double g0 = fma_rn(0.25, add_rn(D[1][kXY], D[2][kXZ]), D[0][kXX]);
+        const double g1 = fma_rn(0.25, add_rn(D[0][kXY], D[2][kYZ]), D[1][kYY]);
+        const double g2 = fma_rn(0.25, add_rn(D[0][kXZ], D[1][kYZ]), D[2][kZZ]);
+        const double g[3] = {g0, g1, g2};
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            F[i] = fma_rn(mu, add_rn(add_rn(D[i][kXX], D[i][kYY]), D[i][kZZ]), mul_rn(lm, g[i]));
+    } else if constexpr (M == DIAG) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) F[i] = fx_sop(r(3 * i), D[i][kXX], r(3 * i + 1), D[i][kYY], r(3 * i + 2), D[i][kZZ]);
+    } else {
+        // the mixed differences in a sum of their own, which takes the 1/4
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            double fd, fm;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int n = 6 * pair_index(i, k);
+                fd = k == 0 ? mul_rn(r(n), D[k][0]) : fma_rn(r(n), D[k][0], fd);
+                fd = fma_rn(r(n + 1), D[k][1], fd);
+                fd = fma_rn(r(n + 2), D[k][2], fd);
+                fm = k == 0 ? mul_rn(r(n + 3), D[k][3]) : fma_rn(r(n + 3), D[k][3], fm);
+                fm = fma_rn(r(n + 4), D[k][4], fm);
+                fm = fma_rn(r(n + 5), D[k][5], fm);
+            }
+            F[i] = fma_rn(0.25, fm, fd);
+        }
+    }
+}
+// number n of the row from the slots a(q)
+template <int M, class A>
+__device__ __forceinline__ auto row_number(A&& a, int n) {
+    if constexpr (M == ISO || M == DIAG) return a(n);
+    else return row_coef<M>(a, n / 6, n % 6);
+}
+// b - scale f and scale f, for the f and the factor that apply_node returns
+template <class R>
+__device__ __forceinline__ R row_residual(R b, R scale, R f) { return fma_rn(-scale, f, b); }
+// The interior term of a node and its central differences for the grad C term: FP64 as above (a row
+// over i2[0]), FP32 from the scaled differences (factor 1).  u(p, di, dj, dk); slot(q) loads a
+// coefficient (after the differences: loaded first, FP32 Fapply took 0.129 ms at 129^3, not 0.097).
+template <int M, class R, class U, class A>
+__device__ __forceinline__ void row_interior(const SCoef<R>& K, U&& u, A&& slot, R gu[3][3], R f[3]) {
+    constexpr int NC = NCoef<M>::value;
+    R a[NC];
+    if constexpr (sizeof(R) == 8) {
+        R D[3][6];
+        row_diffs<R>(K, u, D, gu);
+        row_scale(K, D);
+#pragma unroll
+        for (int q = 0; q < NC; ++q) a[q] = slot(q);
+        row_sum<M>([&](int n) { return row_number<M>([&](int q) { return a[q]; }, n); }, D, f);
+    } else {
+        R b[3][3][3];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            const R c0 = u(p, 0, 0, 0);
+            const R xm = u(p, -1, 0, 0), xp = u(p, 1, 0, 0), ym = u(p, 0, -1, 0), yp = u(p, 0, 1, 0),
+                    zm = u(p, 0, 0, -1), zp = u(p, 0, 0, 1);
+            gu[p][0] = (xp - xm) * K.h[0];
+            gu[p][1] = (yp - ym) * K.h[1];
+            gu[p][2] = (zp - zm) * K.h[2];
+            b[p][0][0] = (xp - R(2) * c0 + xm) * K.i2[0];
+            b[p][1][1] = (yp - R(2) * c0 + ym) * K.i2[1];
+            b[p][2][2] = (zp - R(2) * c0 + zm) * K.i2[2];
+            b[p][0][1] = (u(p, 1, 1, 0) + u(p, -1, -1, 0) - u(p, 1, -1, 0) - u(p, -1, 1, 0)) * K.m01;
+            b[p][0][2] = (u(p, 1, 0, 1) + u(p, -1, 0, -1) - u(p, 1, 0, -1) - u(p, -1, 0, 1)) * K.m02;
+            b[p][1][2] = (u(p, 0, 1, 1) + u(p, 0, -1, -1) - u(p, 0, 1, -1) - u(p, 0, -1, 1)) * K.m12;
+            b[p][1][0] = b[p][0][1];
+            b[p][2][0] = b[p][0][2];
+            b[p][2][1] = b[p][1][2];
+        }
+#pragma unroll
+        for (int q = 0; q < NC; ++q) a[q] = slot(q);
+        div_of<M, R>(a, b, f);
+    }
+}
+// the factor of the interior rows of row_interior
+template <class R>
+__device__ __forceinline__ R row_factor(const SCoef<R>& K) {
+    if constexpr (sizeof(R) == 8) return K.i2[0];
+    else return R(1);
+}
+// f plus its grad C columns (from row_interior's central differences)
+template <class R>
+__device__ __forceinline__ R row_gradc(const SCoef<R>& K, R f, R c0, R c1, R c2) {
+    if constexpr (sizeof(R) == 8) return fma_rn(0.25, fma_rn(c2, K.q[2], fma_rn(c1, K.q[1], c0)), f);
+    else return gradc_add(f, c0, c1, c2, K.h);
+}
+
 // ------------------------------------------------------------------ the operator at one node
 // f = A u at node (i,j,k): boundary rows through the BC table, interior rows
 // C : grad grad u + sum_d (d_d C : grad u) e_d  (src/Operator/Elastic.cpp:174-258).
 // u and C are read through views whose strides may differ.  LDG = false when C lives in
-// shared memory.
+// shared memory.  Returns the factor that A u is f times: row_factor on interior rows, 1 on boundary
+// rows (b - A u is then one fused operation a component, row_residual).
 template <int M, class R, bool LDG = true>
-__device__ __forceinline__ void apply_node(const Geo& g, const SCoef<R>& K, const BCP& bc, bool uniform,
+__device__ __forceinline__ R apply_node(const Geo& g, const SCoef<R>& K, const BCP& bc, bool uniform,
                                            const R* __restrict__ C, long long cs, long long cc,
                                            long long csy, long long csz, const R* __restrict__ U,
                                            long long usc, long long uc, long long usy, long long usz, int i, int j,
@@ -500,41 +687,21 @@ __device__ __forceinline__ void apply_node(const Geo& g, const SCoef<R>& K, cons
             else if (t[r] == NEUMANN) v = gu[r][0] * nrm[0] + gu[r][1] * nrm[1] + gu[r][2] * nrm[2];
             f[r] = v;
         }
-        return;
+        return R(1);
     }
-    R gu[3][3], b[3][3][3];
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-        const R* up = U + p * usc + uc;
-        const R c0 = up[0];
-        const R xm = up[-1], xp = up[1], ym = up[-usy], yp = up[usy], zm = up[-usz], zp = up[usz];
-        gu[p][0] = (xp - xm) * K.h[0];
-        gu[p][1] = (yp - ym) * K.h[1];
-        gu[p][2] = (zp - zm) * K.h[2];
-        b[p][0][0] = (xp - R(2) * c0 + xm) * K.i2[0];
-        b[p][1][1] = (yp - R(2) * c0 + ym) * K.i2[1];
-        b[p][2][2] = (zp - R(2) * c0 + zm) * K.i2[2];
-        b[p][0][1] = (up[1 + usy] + up[-1 - usy] - up[1 - usy] - up[-1 + usy]) * K.m01;
-        b[p][0][2] = (up[1 + usz] + up[-1 - usz] - up[1 - usz] - up[-1 + usz]) * K.m02;
-        b[p][1][2] = (up[usy + usz] + up[-usy - usz] - up[usy - usz] - up[-usy + usz]) * K.m12;
-        b[p][1][0] = b[p][0][1];
-        b[p][2][0] = b[p][0][2];
-        b[p][2][1] = b[p][1][2];
-    }
-    {
-        R a[NC];
-#pragma unroll
-        for (int q = 0; q < NC; ++q) a[q] = ldv<LDG>(C + q * cs + cc);
-        div_of<M, R>(a, b, f);
-    }
+    R gu[3][3];
+    row_interior<M, R>(K, [&](int p, int di, int dj, int dk) { return U[p * usc + uc + di + dj * usy + dk * usz]; },
+                       [&](int q) { return ldv<LDG>(C + q * cs + cc); }, gu, f);
     if (!uniform) {
         R c0[3], c1[3], c2[3];
+        grad_scale(K, gu);
         gradC_col<M, R, LDG>(C, cs, cc, 1, gu, 0, c0);
         gradC_col<M, R, LDG>(C, cs, cc, csy, gu, 1, c1);
         gradC_col<M, R, LDG>(C, cs, cc, csz, gu, 2, c2);
 #pragma unroll
-        for (int r = 0; r < 3; ++r) f[r] = gradc_add(f[r], c0[r], c1[r], c2[r], K.h);
+        for (int r = 0; r < 3; ++r) f[r] = row_gradc(K, f[r], c0[r], c1[r], c2[r]);
     }
+    return row_factor(K);
 }
 
 // apply_node for a stiffness given as a grain id per node (gid, strides gsy, gsz, node index gc)
@@ -542,7 +709,7 @@ __device__ __forceinline__ void apply_node(const Geo& g, const SCoef<R>& K, cons
 // A direction whose two neighbours lie in one grain has an exactly zero stiffness difference; its
 // grad C column is zero and its table reads are skipped.
 template <int M, class R>
-__device__ __forceinline__ void apply_node_grains(const Geo& g, const SCoef<R>& K, const BCP& bc, bool uniform,
+__device__ __forceinline__ R apply_node_grains(const Geo& g, const SCoef<R>& K, const BCP& bc, bool uniform,
                                                   const unsigned short* __restrict__ gid, long long gc,
                                                   long long gsy, long long gsz, const R* __restrict__ tab,
                                                   const R* __restrict__ U, long long usc, long long uc, long long usy,
@@ -584,50 +751,39 @@ __device__ __forceinline__ void apply_node_grains(const Geo& g, const SCoef<R>& 
             else if (t[r] == NEUMANN) v = gu[r][0] * nrm[0] + gu[r][1] * nrm[1] + gu[r][2] * nrm[2];
             f[r] = v;
         }
-        return;
+        return R(1);
     }
-    R gu[3][3], b[3][3][3];
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-        const R* up = U + p * usc + uc;
-        const R c0 = up[0];
-        const R xm = up[-1], xp = up[1], ym = up[-usy], yp = up[usy], zm = up[-usz], zp = up[usz];
-        gu[p][0] = (xp - xm) * K.h[0];
-        gu[p][1] = (yp - ym) * K.h[1];
-        gu[p][2] = (zp - zm) * K.h[2];
-        b[p][0][0] = (xp - R(2) * c0 + xm) * K.i2[0];
-        b[p][1][1] = (yp - R(2) * c0 + ym) * K.i2[1];
-        b[p][2][2] = (zp - R(2) * c0 + zm) * K.i2[2];
-        b[p][0][1] = (up[1 + usy] + up[-1 - usy] - up[1 - usy] - up[-1 + usy]) * K.m01;
-        b[p][0][2] = (up[1 + usz] + up[-1 - usz] - up[1 - usz] - up[-1 + usz]) * K.m02;
-        b[p][1][2] = (up[usy + usz] + up[-usy - usz] - up[usy - usz] - up[-usy + usz]) * K.m12;
-        b[p][1][0] = b[p][0][1];
-        b[p][2][0] = b[p][0][2];
-        b[p][2][1] = b[p][1][2];
-    }
-    {
-        R a[NC];
-#pragma unroll
-        for (int q = 0; q < NC; ++q) a[q] = __ldg(a0 + q);
-        div_of<M, R>(a, b, f);
-    }
+    R gu[3][3];
+    row_interior<M, R>(K, [&](int p, int di, int dj, int dk) { return U[p * usc + uc + di + dj * usy + dk * usz]; },
+                       [&](int q) { return __ldg(a0 + q); }, gu, f);
     if (!uniform) {
         const long long go[3] = {1, gsy, gsz};
-        R col[3][3];
+        int gp[3], gm[3];
+        bool any = false;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const int gp = __ldg(gid + gc + go[d]), gm = __ldg(gid + gc - go[d]);
-            if (gp == gm) {
-                col[d][0] = col[d][1] = col[d][2] = R(0);
-            } else {
-                const R* cp = tab + gp * NC;
-                const R* cm = tab + gm * NC;
-                gradC_col_f<M, R>([&](int q) { return __ldg(cp + q) - __ldg(cm + q); }, gu, d, col[d]);
-            }
+            gp[d] = __ldg(gid + gc + go[d]);
+            gm[d] = __ldg(gid + gc - go[d]);
+            any = any || gp[d] != gm[d];
         }
+        if (any) {
+            R col[3][3];
+            grad_scale(K, gu);
 #pragma unroll
-        for (int r = 0; r < 3; ++r) f[r] = gradc_add(f[r], col[0][r], col[1][r], col[2][r], K.h);
+            for (int d = 0; d < 3; ++d) {
+                if (gp[d] == gm[d]) {
+                    col[d][0] = col[d][1] = col[d][2] = R(0);
+                } else {
+                    const R* cp = tab + gp[d] * NC;
+                    const R* cm = tab + gm[d] * NC;
+                    gradC_col_f<M, R>([&](int q) { return __ldg(cp + q) - __ldg(cm + q); }, gu, d, col[d]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 3; ++r) f[r] = row_gradc(K, f[r], col[0][r], col[1][r], col[2][r]);
+        }
     }
+    return row_factor(K);
 }
 
 }  // namespace ae

@@ -77,26 +77,26 @@ __device__ __forceinline__ void block_max_atomic(double v, unsigned long long* o
 // otherwise through the per-node stiffness C
 // (GR: compiled for the grain tables, so each variant keeps its own register budget)
 template <int M, class R, bool GR>
-__device__ __forceinline__ void apply_any(const OpParams& P, const SCoef<R>& K, const View<const R>& C,
+__device__ __forceinline__ R apply_any(const OpParams& P, const SCoef<R>& K, const View<const R>& C,
                                           const Grains<R>& G, const View<const R>& u, int i, int j, int k, R v[3]) {
     if constexpr (GR)
-        apply_node_grains<M, R>(P.g, K, P.bc, P.uniform, G.gid, C.at(i, j, k), C.sy, C.sz, G.tab, u.p, u.sc,
+        return apply_node_grains<M, R>(P.g, K, P.bc, P.uniform, G.gid, C.at(i, j, k), C.sy, C.sz, G.tab, u.p, u.sc,
                                 u.at(i, j, k), u.sy, u.sz, i, j, k, v);
     else
-        apply_node<M, R>(P.g, K, P.bc, P.uniform, C.p, C.sc, C.at(i, j, k), C.sy, C.sz, u.p, u.sc, u.at(i, j, k),
+        return apply_node<M, R>(P.g, K, P.bc, P.uniform, C.p, C.sc, C.at(i, j, k), C.sy, C.sz, u.p, u.sc, u.at(i, j, k),
                          u.sy, u.sz, i, j, k, v);
 }
 
 // The same with the node's offsets given: oc into C (and the grain ids), ou into u
 template <int M, class R, bool GR>
-__device__ __forceinline__ void apply_at(const OpParams& P, const SCoef<R>& K, const View<const R>& C,
+__device__ __forceinline__ R apply_at(const OpParams& P, const SCoef<R>& K, const View<const R>& C,
                                          const Grains<R>& G, const View<const R>& u, int i, int j, int k,
                                          long long oc, long long ou, R v[3]) {
     if constexpr (GR)
-        apply_node_grains<M, R>(P.g, K, P.bc, P.uniform, G.gid, oc, C.sy, C.sz, G.tab, u.p, u.sc, ou, u.sy, u.sz, i,
+        return apply_node_grains<M, R>(P.g, K, P.bc, P.uniform, G.gid, oc, C.sy, C.sz, G.tab, u.p, u.sc, ou, u.sy, u.sz, i,
                                 j, k, v);
     else
-        apply_node<M, R>(P.g, K, P.bc, P.uniform, C.p, C.sc, oc, C.sy, C.sz, u.p, u.sc, ou, u.sy, u.sz, i, j, k, v);
+        return apply_node<M, R>(P.g, K, P.bc, P.uniform, C.p, C.sc, oc, C.sy, C.sz, u.p, u.sc, ou, u.sy, u.sz, i, j, k, v);
 }
 
 // true when two views index the same storage layout (same box origin and strides): the
@@ -131,11 +131,10 @@ __global__ void __launch_bounds__(kBlock) k_fapply(OpParams P, SCoef<R> K, Reg r
     int i, j, k;
     reg_ijk(reg, t, i, j, k);
     R v[3];
-    apply_any<M, R, GR>(P, K, C, G, u, i, j, k, v);
+    const R sc = apply_any<M, R, GR>(P, K, C, G, u, i, j, k, v);
     const long long o = f.at(i, j, k);
-    f.p[o] = v[0];
-    f.p[o + f.sc] = v[1];
-    f.p[o + 2 * f.sc] = v[2];
+#pragma unroll
+    for (int n = 0; n < 3; ++n) f.p[o + n * f.sc] = mul_rn(sc, v[n]);
 }
 
 // ------------------------------------------------------------------ residual (+ norm, + FP32 copy)
@@ -154,14 +153,14 @@ __global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_residual(
         // SAME: every view has the layout of x (checked by the launcher)
         const long long ox = x.at(i, j, k);
         const long long oc = SAME ? ox : C.at(i, j, k);
-        apply_at<M, R, GR>(P, K, C, G, x, i, j, k, oc, ox, v);
+        const R sc = apply_at<M, R, GR>(P, K, C, G, x, i, j, k, oc, ox, v);
         const long long ob = SAME ? ox : b.at(i, j, k), orr = SAME ? ox : r.at(i, j, k);
         const long long o32 = SAME ? ox : (R32 ? r32.at(i, j, k) : 0);
         const long long bsc = SAME ? x.sc : b.sc, rsc = SAME ? x.sc : r.sc, r32sc = SAME ? x.sc : r32.sc;
         const bool inv = in_box(P.g.vlo, P.g.vhi, i, j, k);
 #pragma unroll
         for (int n = 0; n < 3; ++n) {
-            const R rv = b.p[ob + n * bsc] - v[n];
+            const R rv = row_residual(b.p[ob + n * bsc], sc, v[n]);
             r.p[orr + n * rsc] = rv;
             if (R32) r32.p[o32 + n * r32sc] = (float)rv;
             // a NaN residual reports an infinite norm (fmax alone would drop it)
@@ -173,27 +172,16 @@ __global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_residual(
 
 // ------------------------------------------------------------------ damped Jacobi sweep
 // src/Operator/Operator.cpp:109-157 with the per-node Fapply fused in: one node (i, j, k).
-// The damped-Jacobi update of one component: x_new from x, (A x), b, D and 1/D.
-__device__ __forceinline__ double jacobi_update_impl(double xv, double ax, double b, double d, double invd,
-                                                     double omega) {
-    // the reference's update, (1-w) x + w (b - (Ax - D x)) / D (Operator.cpp:154)
-    const double dx = xv * d;
-    const double rx = ax - dx;
-    return (1.0 - omega) * xv + omega * (b - rx) * invd;
-}
-__device__ __forceinline__ float jacobi_update_impl(float xv, float ax, float b, float, float invd, float omega) {
-    // FP32 cycle: the same update written x + w (b - Ax) / D, which reads no D (rounded in one
-    // fixed order, as the FP32 rows are)
-    return __fmaf_rn(__fmul_rn(omega, __fsub_rn(b, ax)), invd, xv);
-}
+// The damped-Jacobi update of one component from r = b - A x: x + w r / D, which is the reference's
+// (1 - w) x + w (b - (A x - D x)) / D (Operator.cpp:154) without its D, in one fixed rounding order.
 template <class R>
-__device__ __forceinline__ R jacobi_update(R xv, R ax, R b, R d, R invd, R omega) {
-    return jacobi_update_impl(xv, ax, b, d, invd, omega);
+__device__ __forceinline__ R jacobi_update(R xv, R r, R invd, R omega) {
+    return fma_rn(mul_rn(omega, r), invd, xv);
 }
 
 template <int M, class R, bool GR, bool SAME>
 __device__ __forceinline__ void jacobi_node(const OpParams& P, const SCoef<R>& K, const View<const R>& C,
-                                            const Grains<R>& G, const View<const R>& invD, const View<const R>& D,
+                                            const Grains<R>& G, const View<const R>& invD,
                                             const View<const R>& xi, const View<const R>& b, const View<R>& xo,
                                             R omega, int i, int j, int k) {
     const Geo& g = P.g;
@@ -214,13 +202,13 @@ __device__ __forceinline__ void jacobi_node(const OpParams& P, const SCoef<R>& K
         return;
     }
     R v[3];
-    apply_at<M, R, GR>(P, K, C, G, xi, i, j, k, SAME ? ox : C.at(i, j, k), ox, v);
+    const R sc = apply_at<M, R, GR>(P, K, C, G, xi, i, j, k, SAME ? ox : C.at(i, j, k), ox, v);
     const long long od = SAME ? ox : invD.at(i, j, k), ob = SAME ? ox : b.at(i, j, k);
-    const long long dsc = SAME ? xsc : D.sc, isc = SAME ? xsc : invD.sc, bsc = SAME ? xsc : b.sc;
+    const long long isc = SAME ? xsc : invD.sc, bsc = SAME ? xsc : b.sc;
 #pragma unroll
     for (int n = 0; n < 3; ++n)
-        xo.p[oo + n * osc] = jacobi_update<R>(xi.p[ox + n * xsc], v[n], b.p[ob + n * bsc],
-                                              sizeof(R) == 8 ? D.p[od + n * dsc] : R(0), invD.p[od + n * isc], omega);
+        xo.p[oo + n * osc] = jacobi_update<R>(xi.p[ox + n * xsc], row_residual(b.p[ob + n * bsc], sc, v[n]),
+                                              invD.p[od + n * isc], omega);
 }
 
 // The first sweep of a smoother call whose correction starts at zero (the pre-smoothing of a
@@ -229,8 +217,8 @@ __device__ __forceinline__ void jacobi_node(const OpParams& P, const SCoef<R>& K
 // through the same update with the zeros passed in at run time (zero == 0), so the arithmetic
 // and its rounding are the full sweep's.
 template <class R>
-__global__ void __launch_bounds__(kBlock) k_jacobi_zero(Geo g, Reg reg, View<const R> invD, View<const R> D,
-                                                        View<const R> b, View<R> xo, R omega, R zero) {
+__global__ void __launch_bounds__(kBlock) k_jacobi_zero(Geo g, Reg reg, View<const R> invD, View<const R> b,
+                                                        View<R> xo, R omega, R zero) {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= reg.n) return;
     int i, j, k;
@@ -246,21 +234,21 @@ __global__ void __launch_bounds__(kBlock) k_jacobi_zero(Geo g, Reg reg, View<con
     const long long od = invD.at(i, j, k), ob = b.at(i, j, k);
 #pragma unroll
     for (int n = 0; n < 3; ++n)
-        xo.p[oo + n * xo.sc] = jacobi_update<R>(zero, zero, b.p[ob + n * b.sc], sizeof(R) == 8 ? D.p[od + n * D.sc] : R(0),
+        xo.p[oo + n * xo.sc] = jacobi_update<R>(zero, row_residual(b.p[ob + n * b.sc], R(1), zero),
                                                 invD.p[od + n * invD.sc], omega);
 }
 
 template <int M, class R, bool GR, bool SAME>
 __global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_jacobi(OpParams P, SCoef<R> K, Reg reg,
                                                                                View<const R> C, Grains<R> G,
-                                                                               View<const R> invD, View<const R> D,
+                                                                               View<const R> invD,
                                                                                View<const R> xi, View<const R> b,
                                                                                View<R> xo, R omega) {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= reg.n) return;
     int i, j, k;
     reg_ijk(reg, t, i, j, k);
-    jacobi_node<M, R, GR, SAME>(P, K, C, G, invD, D, xi, b, xo, omega, i, j, k);
+    jacobi_node<M, R, GR, SAME>(P, K, C, G, invD, xi, b, xo, omega, i, j, k);
 }
 
 // ------------------------------------------------------------------ z-marching tiled stencil sweeps
@@ -296,7 +284,7 @@ __device__ __forceinline__ void cp_async_wait() {
 template <int M, class R, int OP>
 __global__ void __launch_bounds__(TX* TY, 2) k_tiled(OpParams P, SCoef<R> K, Box3 box, View<const R> C,
                                                      View<const R> x, View<const R> b, View<const R> invD,
-                                                     View<const R> D, View<R> out, R omega) {
+                                                     View<R> out, R omega) {
     constexpr int NC = NCoef<M>::value;
     constexpr int NZ = ZSlots<M>::n;
     constexpr int NT = TX * TY;
@@ -392,7 +380,7 @@ __global__ void __launch_bounds__(TX* TY, 2) k_tiled(OpParams P, SCoef<R> K, Box
                                       k > g.dlo[2] && k < g.dhi[2];
                 if (!interior) {
                     apply_node<M, R>(g, K, P.bc, P.uniform, C.p, C.sc, C.at(i, j, k), C.sy, C.sz, x.p, x.sc,
-                                     x.at(i, j, k), x.sy, x.sz, i, j, k, f);
+                                     x.at(i, j, k), x.sy, x.sz, i, j, k, f);  // a boundary row: factor 1
                 } else {
                     R gu[3][3], bb[3][3][3];
 #pragma unroll
@@ -442,8 +430,7 @@ __global__ void __launch_bounds__(TX* TY, 2) k_tiled(OpParams P, SCoef<R> K, Box
                     const long long ob = b.at(i, j, k), od = invD.at(i, j, k);
 #pragma unroll
                     for (int n = 0; n < 3; ++n)
-                        out.p[oo + n * out.sc] = jacobi_update<R>(Uc[n * HP + idx], f[n], b.p[ob + n * b.sc],
-                                                                  sizeof(R) == 8 ? D.p[od + n * D.sc] : R(0),
+                        out.p[oo + n * out.sc] = jacobi_update<R>(Uc[n * HP + idx], b.p[ob + n * b.sc] - f[n],
                                                                   invD.p[od + n * invD.sc], omega);
                 }
             }

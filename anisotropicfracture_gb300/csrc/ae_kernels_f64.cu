@@ -571,11 +571,11 @@ struct BottomOps {
             const int k = t / sz, rem = t - k * sz;
             const int j = rem / nx, i = rem - j * nx;
             double v[3];
-            apply_node<M, double, !SMEM>(g, K, a.P.bc, a.P.uniform, Cv.p, nn, t, sy, sz, x, nn, t, sy, sz,
+            const double f = apply_node<M, double, !SMEM>(g, K, a.P.bc, a.P.uniform, Cv.p, nn, t, sy, sz, x, nn, t, sy, sz,
                                          i + g.vlo[0], j + g.vlo[1], k + g.vlo[2], v);
-            out[t] = v[0];
-            out[t + nn] = v[1];
-            out[t + 2 * nn] = v[2];
+            out[t] = f * v[0];
+            out[t + nn] = f * v[1];
+            out[t + 2 * nn] = f * v[2];
         }
         __syncthreads();
     }
@@ -716,11 +716,11 @@ __global__ void __launch_bounds__(128) k_bottom_assemble(BottomArgs a, double* A
         const int k = (int)(t / sz), rem = (int)(t - (long long)k * sz);
         const int jj = rem / nx, i = rem - jj * nx;
         double v[3];
-        apply_node<M, double, true>(g, a.K, a.P.bc, a.P.uniform, a.C, nn, t, sy, sz, e, nn, t, sy, sz, i + g.vlo[0],
+        const double f = apply_node<M, double, true>(g, a.K, a.P.bc, a.P.uniform, a.C, nn, t, sy, sz, e, nn, t, sy, sz, i + g.vlo[0],
                                     jj + g.vlo[1], k + g.vlo[2], v);
-        A[t * N + j] = v[0];
-        A[(t + nn) * N + j] = v[1];
-        A[(t + 2 * nn) * N + j] = v[2];
+        A[t * N + j] = f * v[0];
+        A[(t + nn) * N + j] = f * v[1];
+        A[(t + 2 * nn) * N + j] = f * v[2];
     }
 }
 void launch_bottom_assemble(const BottomArgs& a, double* A, double* E, cudaStream_t st) {

@@ -54,19 +54,7 @@ inline Box3 geo_apply_region(const Geo& g) {
 }
 
 template <class R>
-SCoef<R> make_scoef(const Geo& g) {
-    SCoef<R> K;
-    for (int d = 0; d < 3; ++d) {
-        K.h[d] = (R)(0.5 / g.dx[d]);
-        K.id[d] = (R)(1.0 / g.dx[d]);
-        K.i2[d] = (R)(1.0 / (g.dx[d] * g.dx[d]));
-        K.bb[d] = (R)(-2.0 / g.dx[d] / g.dx[d]);
-    }
-    K.m01 = (R)(0.25 / (g.dx[0] * g.dx[1]));
-    K.m02 = (R)(0.25 / (g.dx[0] * g.dx[2]));
-    K.m12 = (R)(0.25 / (g.dx[1] * g.dx[2]));
-    return K;
-}
+SCoef<R> make_scoef(const Geo& g) { return scoef_of<R>(g.dx); }
 
 // View over a level's storage box (the layout of every internal array).
 template <class T>
@@ -120,13 +108,13 @@ void launch_residual(const OpParams& P, View<const R> C, View<const R> x, View<c
 // One damped-Jacobi sweep: xo = (1-w) xi + w (b - (A xi - D xi)) / D on grow(valid,1)∩dom,
 // zero on the ring grow(valid,2) \ grow(valid,1), copy elsewhere.
 template <class R>
-void launch_jacobi(const OpParams& P, View<const R> C, View<const R> invD, View<const R> D, View<const R> xi,
+void launch_jacobi(const OpParams& P, View<const R> C, View<const R> invD, View<const R> xi,
                    View<const R> b, View<R> xo, R omega, cudaStream_t st, Grains<R> G = Grains<R>{});
 // Fapply (op 0), damped-Jacobi sweep (op 1) or residual (op 2) with the z-marching tiled
 // kernel, on the level's internal storage views only.  tiled_init must have run once.
 template <class R>
 void launch_tiled(int op, const OpParams& P, View<const R> C, View<const R> x, View<const R> b, View<const R> invD,
-                  View<const R> D, View<R> out, R omega, cudaStream_t st);
+                  View<R> out, R omega, cudaStream_t st);
 template <class R>
 void tiled_init();
 template <class R>
@@ -154,7 +142,7 @@ void launch_fill(const Box3& region, int ncomp, View<R> dst, R value, cudaStream
 // The first damped-Jacobi sweep from x = 0 over the level's storage box: every node as the full
 // sweep leaves it for x = 0 (x_new = w b / D where the sweep updates, 0 elsewhere), no stencil.
 template <class R>
-void launch_jacobi_zero(const Geo& g, View<const R> invD, View<const R> D, View<const R> b, View<R> xo, R omega,
+void launch_jacobi_zero(const Geo& g, View<const R> invD, View<const R> b, View<R> xo, R omega,
                         cudaStream_t st);
 // max |v| over region into *norm (bit pattern)
 template <class R>

@@ -5,15 +5,12 @@
 // only the nodes whose stencil straddles a grain boundary take -- and waits on scattered loads.
 // A sweep there is split by node:
 //
-//   k_sweep_tile   every node of the interior box I (not on the domain boundary, inside
-//                  grow(valid, 1)).  A block owns a 32 x 8 column of (i, j) and marches in k.
-//                  Per plane one elected thread loads, with TMA (cp.async.bulk.tensor) onto an
-//                  mbarrier, the x halo tile (three components), b, 1/D and the grain id/mask
-//                  tile of the next plane, so every read of the stencil and the update is a
-//                  shared-memory load at a fixed offset.  The grain table sits in shared memory.
-//                  In FP32 a thread computes the nodes of two neighbouring rows, which share the
-//                  loads of the rows between them.  The grad C term is computed only where the
-//                  node's mask says a direction's two neighbours lie in different grains.
+//   k_sweep_tile64/32  every node of the interior box I (not on the domain boundary, inside
+//                  grow(valid, 1)).  A block owns a 32 x 8 column of (i, j) and marches in k, its
+//                  planes of x, b, 1/D and the ids loaded by TMA (cp.async.bulk.tensor) ahead of
+//                  the plane being computed, the grain tables in shared memory.  The grad C term
+//                  is computed only where the node's mask says a direction's two neighbours lie in
+//                  different grains.
 //   k_*_list       every node of the sweep region outside I (domain-boundary rows, the ghost
 //                  ring, nodes outside the domain), through the per-node code.
 //
@@ -22,15 +19,15 @@
 //
 // Every node is computed by the per-node sweep's own arithmetic: where a direction's neighbours
 // share a grain the grad C column is exactly zero, and the interior and grad C expressions are
-// written operation for operation as apply_node_grains writes them (the FP32 sums of products in
-// the explicitly rounded order of ae_device.cuh), so the split sweep equals the one-pass sweep
-// bit for bit.  The list and the id/mask array are built once per level (k_split_mark), when the
+// those of ae_device.cuh in their explicitly rounded order, so the split sweep equals the one-pass
+// sweep bit for bit.  The list and the id/mask array are built once per level (k_split_mark), when the
 // operator is prepared.  TMA needs 16-byte aligned rows: the level arrays' row pitch is a
 // multiple of 4 nodes (Geo::px).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -41,54 +38,47 @@ namespace ae {
 
 namespace {
 
-constexpr int STX = 32, STY = 8, SNT = STX * STY;
-constexpr int SBW = 36;                    // box width: 32 nodes + halo + alignment shift (<= 2)
-constexpr int SXR = STY + 2;               // x tile rows (one-node halo in j)
-constexpr int SXP = SBW * SXR;             // elements per x component plane tile
-constexpr int SVP = SBW * STY;             // elements per b / 1/D / D component tile (no halo)
-constexpr int SXRING = 4, SVRING = 2;      // x planes k-1, k, k+1 + the one in flight; b, 1/D, ids
-constexpr int kWaitLimit = 1 << 20;        // try_wait polls before a wait is declared failed
-#ifndef AE_SPLIT_MIN_BLOCKS
-#define AE_SPLIT_MIN_BLOCKS 4
+constexpr int STX = 32, STY = 8;   // nodes of a tile per plane: a warp per row
+constexpr int SXR = STY + 2;       // x tile rows (one-node halo in j)
+constexpr int kWaitLimit = 1 << 20;  // try_wait polls before a wait is declared failed
+constexpr int kTileThreads = 32 * (STY + 1);  // the rows' warps and a producer
+#ifndef AE_RING
+#define AE_RING 4
 #endif
-// FP32: each thread computes the nodes of NPT consecutive rows j .. j + NPT - 1, which share the
-// loads of the rows between them in every plane: for two rows, 28 instead of 38 shared-memory
-// loads per component
-#ifndef AE_SPLIT_NPT32
-#define AE_SPLIT_NPT32 2
-#endif
-#ifndef AE_SPLIT_PAIR_BLOCKS
-#define AE_SPLIT_PAIR_BLOCKS 5
-#endif
-
+constexpr int SRING = AE_RING;     // planes in flight or in use
 __host__ __device__ constexpr int up128(int b) { return (b + 127) / 128 * 128; }
-__host__ __device__ constexpr int up16(int b) { return (b + 15) / 16 * 16; }
 
-// Shared memory of the tiled kernel, in bytes, for elements R: the x ring, the b, 1/D and (FP64
-// Jacobi: the reference's update reads D) D rings, the id ring -- every TMA destination on a
-// 128-byte boundary -- two mbarriers, the queue of the plane's nodes with a non-zero grad C
-// column (count, thread index, main-term f) and the grain table.
+// Nodes with a grad C column are put off: a warp keeps what the column needs -- the in-plane
+// differences, the two neighbours in k, the interior sum and the node's offset -- in a queue of its own
+// and computes 32 of them at a time, because a warp-wide FP64 instruction costs the same whatever lanes
+// are active.
+constexpr int QCAP = 64;  // entries per warp: at most 31 left over and 32 new ones
+constexpr int QN = 15;    // numbers per entry
+
+// Shared memory of the tiled kernel, in bytes, for elements R: per ring slot the x halo tile, the b and
+// 1/D tiles and the ids (TMA destinations on a 128-byte boundary); then the barriers, the warps' queues
+// (FP64) and the grain tables.
 template <class R>
 struct TL {
     static constexpr int E = (int)sizeof(R);
-    static constexpr int XS = up128(3 * SXP * E);  // bytes per x ring slot
-    static constexpr int VS = 3 * SVP * E;         // bytes per b / 1/D / D ring slot
-    static constexpr int GS = SVP * 4;             // bytes per id ring slot
-    static constexpr int oB = SXRING * XS;
-    static constexpr int oI = oB + SVRING * VS;
-    static constexpr int oD = oI + SVRING * VS;
-    static constexpr int oG = oD + (E == 8 ? SVRING * VS : 0);
-    static constexpr int oBar = oG + SVRING * GS;
-    static constexpr int oQ = oBar + 16;
-    static constexpr int oQt = oQ + 16;
-    static constexpr int oQf = up16(oQt + 4 * SNT);
-    static constexpr int oT = up16(oQf + 3 * SNT * E);
-    static constexpr unsigned kX = 3 * SXP * E, kV = 3 * SVP * E, kG = SVP * 4;
-    static_assert(VS % 128 == 0 && GS % 128 == 0 && oB % 128 == 0 && oI % 128 == 0 && oD % 128 == 0 &&
-                      oG % 128 == 0,
-                  "TMA slot alignment");
+    static constexpr int AL = 16 / E;              // columns per 16 bytes: TMA boxes start on such a column
+    static constexpr int BW = STX + 2 * AL;        // x box width: the tile and AL columns to each side
+    static constexpr int XP = BW * SXR;            // elements per x component plane tile
+    static constexpr int VP = STX * STY;           // elements per b / 1/D / id component plane tile
+    static constexpr int oB = up128(3 * XP * E);
+    static constexpr int oI = oB + 3 * VP * E;
+    static constexpr int oG = oI + 3 * VP * E;
+    static constexpr int kSlot = oG + VP * 4;
+    static constexpr int oBar = SRING * kSlot;
+    static constexpr int oQ = up128(oBar + 16 * SRING + 8);  // the ring's barriers and the table's
+    static constexpr int kQ = QCAP * (QN * E + 4);  // bytes per warp queue
+    static constexpr int oT = up128(oQ + STY * kQ);
+    static constexpr unsigned kX = 3 * XP * E, kV = 3 * VP * E, kG = VP * 4;
+    static_assert(oB % 128 == 0 && oI % 128 == 0 && oG % 128 == 0 && kSlot % 128 == 0, "TMA destinations");
 };
-constexpr int kTabSmemMax = 24 * 1024;  // bytes of grain table kept in shared memory
+// bytes of grain tables kept in shared memory: the rows' numbers up to kRowSmemMax, and the stiffness
+// table beside them up to kTabSmemMax in all (three FP32 blocks an SM up to 110 cubic grains)
+constexpr int kRowSmemMax = 40 * 1024, kTabSmemMax = 44 * 1024;
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -97,6 +87,9 @@ __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
 }
 __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
     unsigned ok;
@@ -121,6 +114,13 @@ __device__ __forceinline__ void tma_load4(unsigned dst, const CUtensorMap* map, 
         "[%6];\n" ::"r"(dst),
         "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(z), "r"(c), "r"(bar)
         : "memory");
+}
+
+// global -> shared memory, addresses and size multiples of 16 bytes, completing on an mbarrier
+__device__ __forceinline__ void bulk_copy(unsigned dst, const void* src, int bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
 }
 
 // packed node of a list: offsets from the storage box's low corner, 21 bits each
@@ -180,42 +180,328 @@ __global__ void __launch_bounds__(kBlock) k_split_mark(Reg reg, Box3 R, Box3 I, 
     if (FILL && f) list[base + wcnt[w] + __popc(ball & ((1u << lane) - 1u))] = code;
 }
 
+// Row numbers of every grain (RowN), in rows of whole pairs: what row_sum takes for a node of the grain.
+template <int M>
+__host__ __device__ constexpr int row_stride() { return (RowN<M>::value + 1) / 2 * 2; }
+template <int M>
+__global__ void __launch_bounds__(kBlock) k_row_table(const double* __restrict__ tab, int ngr, double* __restrict__ rows) {
+    constexpr int NC = NCoef<M>::value, NR = RowN<M>::value;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= ngr) return;
+#pragma unroll
+    for (int n = 0; n < NR; ++n) {
+        rows[(long long)g * row_stride<M>() + n] = row_number<M>([&](int q) { return __ldg(tab + (long long)g * NC + q); }, n);
+    }
+}
+
 // Tile geometry shared by the host and the kernel: tensor coordinates are offsets from the
-// storage box's low corner; the boxes of a tile start at column xa (a multiple of 4, as TMA
-// requires), and node i of the tile sits at column sh + 1 + (i - i0).
+// storage box's low corner.  Tiles start on columns that are multiples of 32 there, so a warp's rows
+// of b, 1/D, the ids and the output are aligned; the x box starts AL columns before.
 struct TileGeo {
     Box3 I;        // interior box (absolute node indices)
     int slo[3];    // storage box low corner
-    int tiles_x;   // tiles per row of I
+    int tiles_x;   // tiles per row of the storage box
     int kz;        // planes per block
-    int sh;        // column shift of the tile's first halo column inside the box
 };
 
 // One sweep over the interior box I of a grain-map level, A the interior row of
-// Elastic<T>::Fapply: OP = SPLIT_JACOBI, the damped-Jacobi update (jacobi_update: the reference's
-// form in FP64, x + w (b - A x) / D in the FP32 cycle; Operator.cpp:109-157); OP = SPLIT_RESIDUAL,
-// out = b - A x (out may alias b: every node reads only its own b); OP = SPLIT_FAPPLY, out = A x.  The grain table is staged
-// in shared memory (TABS, rows padded to 16 bytes) or read through L1.  err: set when a TMA load
-// did not complete.  NPT: rows of the tile per thread (1, 2 or 4: the thread's nodes (i, j) ..
-// (i, j + NPT - 1) take the x values of rows j - 1 .. j + NPT from one set of loads; each node's
-// arithmetic is unchanged).
+// Elastic<T>::Fapply: OP = SPLIT_JACOBI, the damped-Jacobi update (Operator.cpp:109-157);
+// OP = SPLIT_RESIDUAL, out = b - A x (out may alias b: every node reads only its own b);
+// OP = SPLIT_FAPPLY, out = A x.
+//
+// A block owns a 32 x 8 column of (i, j) and marches in k.  One producer warp keeps up to SRING planes
+// in flight by TMA (cp.async.bulk.tensor onto a full barrier per slot): the x halo tile (three
+// components) of a plane and the b, 1/D and id tiles of the plane before, which is the one that becomes
+// computable.  The other warps hold a row (FP32: two rows) each.  An x plane is read from shared memory
+// once: each node takes from it the centre value, the two in-plane central differences and the three
+// in-plane second differences; the differences across planes come from those of the planes before, in
+// registers (9 values a component).  Warps run up to a ring apart, and no block barrier is in the loop.
+//
+// The row's numbers sit in shared memory per grain (TABS: the table of k_row_table, one bulk copy) or are
+// formed from the slots in global memory.  err: set when
+// a wait ran out.
+//
+// Bound by the FP64 pipe (89 % busy): 99 operations a node on a cubic level and about 6 for the queue.
+// Fapply at 257^3 3.45 ms, with the boundary list 3.52, against 4.34 and 4.42 with the scaled rows (154
+// operations) and a queue per plane that one warp worked off behind two block barriers; residual 3.52
+// against 4.54, Jacobi 3.73 against 4.98.  A queue per block instead of per warp: 3.66.
 enum SplitOp { SPLIT_JACOBI = 0, SPLIT_RESIDUAL = 1, SPLIT_FAPPLY = 2 };
-template <int M, class R, bool TABS, int OP, int NPT>
-__global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : sizeof(R) == 4 ? AE_SPLIT_MIN_BLOCKS : 2)
-    k_sweep_tile(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_b,
-                 const __grid_constant__ CUtensorMap tm_i, const __grid_constant__ CUtensorMap tm_d,
-                 const __grid_constant__ CUtensorMap tm_g, SCoef<R> K, TileGeo T, int uniform, long long sy,
-                 long long sz, long long sc, const unsigned* __restrict__ gidm_g, const R* __restrict__ tab, int tab_n,
-                 R* __restrict__ xo, R omega, int* err) {
-    static_assert(NPT == 1 || NPT == 2 || NPT == 4, "one, two or four rows per thread");
-    static_assert(STY % NPT == 0, "whole row groups per tile");
-    constexpr int NT = SNT / NPT;  // threads per block
+// what a thread keeps of a plane, per component: centre, in-plane central differences
+template <class R>
+struct PlaneRegs {
+    R c[3], dx[3], dy[3];
+};
+template <int M, bool TABS, int OP>
+__global__ void __launch_bounds__(kTileThreads, 1)
+    k_sweep_tile64(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_b,
+                 const __grid_constant__ CUtensorMap tm_i, const __grid_constant__ CUtensorMap tm_g, SCoef<double> K, TileGeo T,
+                 int uniform, int sy, int sz, int sc, const unsigned* __restrict__ gidm,
+                 const double* __restrict__ tab, const double* __restrict__ rows, int rows_bytes, int tab_bytes,
+                 const double* __restrict__ x, const double* b, const double* __restrict__ invD, double* out, double omega,
+                 int* err) {
+    using R = double;
     using L = TL<R>;
+    constexpr int NC = NCoef<M>::value, TS = row_stride<M>();
+    extern __shared__ __align__(128) unsigned char smem[];
+    const unsigned sb = smem_u32(smem);
+    const auto full = [&](int s) { return sb + (unsigned)L::oBar + 16u * (unsigned)s; };
+    const auto empty = [&](int s) { return sb + (unsigned)L::oBar + 16u * (unsigned)s + 8u; };
+    const R* ts = reinterpret_cast<const R*>(smem + L::oT);
+    const unsigned tbar = sb + (unsigned)L::oBar + 16u * SRING;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c0 = (int)(blockIdx.x % T.tiles_x) * STX;  // the tile's first column, from slo
+    const int j0 = T.I.lo[1] + (int)(blockIdx.x / T.tiles_x) * STY;
+    const int k0 = T.I.lo[2] + (int)blockIdx.y * T.kz;
+    const int k1 = min(k0 + T.kz - 1, T.I.hi[2]);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < SRING; ++s) {
+            mbar_init(full(s), 1);
+            mbar_init(empty(s), STY);
+        }
+        mbar_init(tbar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    const int planes = k1 - k0 + 3;  // x planes k0 - 1 .. k1 + 1; with plane k0 - 1 + t come the tiles of plane k0 - 2 + t
+    if (warp == STY) {               // producer
+        if (lane == 0) {
+            int t = 0;
+            bool ok = true;
+            if (TABS) {
+                mbar_expect_tx(tbar, (unsigned)(rows_bytes + tab_bytes));
+                bulk_copy(sb + (unsigned)L::oT, rows, rows_bytes, tbar);
+                if (tab_bytes) bulk_copy(sb + (unsigned)(L::oT + rows_bytes), tab, tab_bytes, tbar);
+            }
+            for (; t < planes; ++t) {
+                const int s = t % SRING;
+                if (t >= SRING && !mbar_wait(empty(s), (unsigned)((t / SRING - 1) & 1))) {
+                    ok = false;
+                    break;
+                }
+                constexpr unsigned kTiles = (OP == SPLIT_JACOBI ? 2 : OP == SPLIT_RESIDUAL ? 1 : 0) * L::kV + L::kG;
+                const unsigned dst = sb + (unsigned)(s * L::kSlot);
+                const int y = j0 - T.slo[1], z = k0 - 1 + t - T.slo[2];
+                mbar_expect_tx(full(s), L::kX + (t >= 2 ? kTiles : 0u));
+                tma_load4(dst, &tm_x, c0 - L::AL, y - 1, z, 0, full(s));
+                if (t >= 2) {
+                    tma_load4(dst + L::oG, &tm_g, c0, y, z - 1, 0, full(s));
+                    if (OP != SPLIT_FAPPLY) tma_load4(dst + L::oB, &tm_b, c0, y, z - 1, 0, full(s));
+                    if (OP == SPLIT_JACOBI) tma_load4(dst + L::oI, &tm_i, c0, y, z - 1, 0, full(s));
+                }
+            }
+            if (!ok) atomicExch(err, 1);
+            // let the loads in flight land (bounded) before the block's memory goes
+            for (int q = max(t - SRING, 0); q < t; ++q) mbar_wait(full(q % SRING), (unsigned)((q / SRING) & 1));
+            if (TABS) mbar_wait(tbar, 0);
+        }
+        return;
+    }
+    const int i = T.slo[0] + c0 + lane, j = j0 + warp;
+    const bool act = i >= T.I.lo[0] && i <= T.I.hi[0] && j <= T.I.hi[1];
+    int o = c0 + lane + (j - T.slo[1]) * sy + (k0 - T.slo[2] - 2) * sz;  // node (i, j) of the plane computed
+    // the grains' stiffness: beside the rows in shared memory, or global
+    const R* gt = TABS && tab_bytes ? reinterpret_cast<const R*>(smem + L::oT + rows_bytes) : tab;
+    // F plus the grad C term of a node at offset on: gu its central differences, gp and gm the grains of
+    // its neighbours, mask the directions
+    const auto with_gradc = [&](unsigned mask, const unsigned (&gp)[3], const unsigned (&gm)[3], R (&gu)[3][3], R (&F)[3]) {
+        grad_scale(K, gu);
+        R col[3][3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (mask & (1u << d)) {
+                const R* cp = gt + (int)(gp[d] & 0xffffu) * NC;
+                const R* cm = gt + (int)(gm[d] & 0xffffu) * NC;
+                gradC_col_f<M, R>([&](int q) { return cp[q] - cm[q]; }, gu, d, col[d]);
+            } else {
+                col[d][0] = col[d][1] = col[d][2] = R(0);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) F[r] = row_gradc(K, F[r], col[0][r], col[1][r], col[2][r]);
+    };
+    const auto value = [&](R xc, R bc, R ic, R F) {
+        if (OP == SPLIT_JACOBI) return jacobi_update<R>(xc, row_residual(bc, K.i2[0], F), ic, omega);
+        if (OP == SPLIT_RESIDUAL) return row_residual(bc, K.i2[0], F);
+        return mul_rn(K.i2[0], F);
+    };
+    R* qv = reinterpret_cast<R*>(smem + L::oQ + warp * L::kQ);  // [QN][QCAP]
+    int* qo = reinterpret_cast<int*>(qv + QN * QCAP);
+    int qhead = 0, qcnt = 0;
+    // the first cnt (at most 32) nodes of the queue
+    const auto work_off = [&](int cnt) {
+        __syncwarp();
+        if (lane < cnt) {
+            const int e = (qhead + lane) & (QCAP - 1);
+            const int on = qo[e];
+            const int step[3] = {1, sy, sz};
+            unsigned gp[3], gm[3];
+            R xc[3], bc[3], ic[3], gu[3][3], F[3];
+            const unsigned mask = __ldg(gidm + on) >> 16;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                gp[d] = __ldg(gidm + on + step[d]);
+                gm[d] = __ldg(gidm + on - step[d]);
+            }
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                xc[r] = OP == SPLIT_JACOBI ? __ldg(x + on + r * sc) : R(0);
+                bc[r] = OP != SPLIT_FAPPLY ? b[on + r * sc] : R(0);
+                ic[r] = OP == SPLIT_JACOBI ? __ldg(invD + on + r * sc) : R(0);
+                F[r] = qv[(12 + r) * QCAP + e];
+                gu[r][0] = qv[r * QCAP + e];
+                gu[r][1] = qv[(3 + r) * QCAP + e];
+                gu[r][2] = sub_rn(qv[(6 + r) * QCAP + e], qv[(9 + r) * QCAP + e]);
+            }
+            with_gradc(mask, gp, gm, gu, F);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) out[on + r * sc] = value(xc[r], bc[r], ic[r], F[r]);
+        }
+        __syncwarp();
+        qhead = (qhead + cnt) & (QCAP - 1);
+        qcnt -= cnt;
+    };
+
+    PlaneRegs<R> even, odd;
+    R xx[3], yy[3], xy[3];                               // in-plane second differences of the middle plane
+    const int at = (warp + 1) * L::BW + L::AL + lane;    // node (i, j) inside an x component tile
+    const int av = warp * STX + lane;                    // ... inside a b / 1/D / id component tile
+    // One plane: x plane k + 1 has arrived in the slot at base.  lo holds plane k - 1 and receives plane
+    // k + 1, mid holds plane k, whose row is formed (for the block's first two planes from nothing, and
+    // not stored).
+    const auto plane = [&](PlaneRegs<R>& lo, PlaneRegs<R>& mid, const unsigned char* base, bool store) {
+        const R* xs = reinterpret_cast<const R*>(base) + at;
+        const R* vb = reinterpret_cast<const R*>(base + L::oB) + av;
+        const R* vi = reinterpret_cast<const R*>(base + L::oI) + av;
+        const unsigned gw = store ? reinterpret_cast<const unsigned*>(base + L::oG)[av] : 0u;
+        const bool wide = !uniform && (gw >> 16) != 0;  // has a grad C column
+        const unsigned ball = __ballot_sync(0xffffffffu, wide);
+        int e = -1;  // queue entry
+        if (wide) {
+            e = (qhead + qcnt + __popc(ball & ((1u << lane) - 1u))) & (QCAP - 1);
+            qo[e] = o;
+        }
+        qcnt += __popc(ball);
+        const R* tr = TABS ? ts + (int)(gw & 0xffffu) * TS : tab;
+        R D[3][6], F[3];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            const R* u = xs + p * L::XP;
+            const R c = u[0], xm = u[-1], xp = u[1], ym = u[-L::BW], yp = u[L::BW];
+            const R dx = sub_rn(xp, xm), dy = sub_rn(yp, ym);
+            D[p][kXX] = xx[p];
+            D[p][kYY] = yy[p];
+            D[p][kXY] = xy[p];
+            D[p][kZZ] = add_rn(fma_rn(R(-2), mid.c[p], c), lo.c[p]);
+            D[p][kXZ] = sub_rn(dx, lo.dx[p]);
+            D[p][kYZ] = sub_rn(dy, lo.dy[p]);
+            if (e >= 0) {
+                qv[p * QCAP + e] = mid.dx[p];
+                qv[(3 + p) * QCAP + e] = mid.dy[p];
+                qv[(6 + p) * QCAP + e] = c;
+                qv[(9 + p) * QCAP + e] = lo.c[p];
+            }
+            lo.c[p] = c;
+            lo.dx[p] = dx;
+            lo.dy[p] = dy;
+            xx[p] = add_rn(fma_rn(R(-2), c, xp), xm);
+            yy[p] = add_rn(fma_rn(R(-2), c, yp), ym);
+            xy[p] = sub_rn(sub_rn(u[1 + L::BW], u[1 - L::BW]), sub_rn(u[-1 + L::BW], u[-1 - L::BW]));
+        }
+        {
+            row_scale(K, D);
+            if constexpr (TABS) {
+                row_sum<M>([&](int q) { return tr[q]; }, D, F);
+            } else {
+                R a[NC];
+                const R* ag = tab + (int)(gw & 0xffffu) * NC;
+#pragma unroll
+                for (int q = 0; q < NC; ++q) a[q] = __ldg(ag + q);
+                row_sum<M>([&](int q) { return row_number<M>([&](int u) { return a[u]; }, q); }, D, F);
+            }
+        }
+        if (e >= 0) {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) qv[(12 + r) * QCAP + e] = F[r];
+        }
+        if (store && e < 0) {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const R bc = OP != SPLIT_FAPPLY ? vb[r * L::VP] : R(0), ic = OP == SPLIT_JACOBI ? vi[r * L::VP] : R(0);
+                out[o + r * sc] = value(mid.c[r], bc, ic, F[r]);
+            }
+        }
+    };
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        even.c[p] = even.dx[p] = even.dy[p] = odd.c[p] = odd.dx[p] = odd.dy[p] = R(0);
+        xx[p] = yy[p] = xy[p] = R(0);
+    }
+    bool failed = TABS && !__all_sync(0xffffffffu, mbar_wait(tbar, 0));
+    int s = 0;
+    unsigned phase = 0;
+    for (int t = 0; !failed && t < planes; ++t, o += sz) {  // x plane k0 - 1 + t
+        failed = !__all_sync(0xffffffffu, mbar_wait(full(s), phase));
+        if (failed) break;
+        const unsigned char* base = smem + s * L::kSlot;
+        if (t & 1) plane(odd, even, base, act && t >= 2);
+        else plane(even, odd, base, act && t >= 2);
+        // the slot has been read by every lane: hand it back
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty(s));
+        if (qcnt >= 32 || (t + 1 == planes && qcnt > 0)) work_off(min(qcnt, 32));
+        if (t + 1 == planes && qcnt > 0) work_off(qcnt);
+        if (++s == SRING) {
+            s = 0;
+            phase ^= 1u;
+        }
+    }
+    if (failed && lane == 0) atomicExch(err, 1);
+}
+
+// ------------------------------------------------------------------ FP32
+// The same sweep in FP32.  It is bound by issue and by the shared-memory data path (a word per lane and
+// cycle), no unit saturated: a block of 128 threads owns a 32 x 8 column and marches 8 planes, two rows
+// per thread, which share the loads of the rows between them in every plane (28 instead of 38 loads per
+// component).  One thread issues, per plane, the TMA loads of the x halo tile, b, 1/D and the ids one
+// stage ahead.  The rows are div_mm's 21 coefficients a node: the 36 sums of the FP64 rows would be 12
+// more words of that path.  Nodes with a grad C column (a mask in the id word) go to a queue and are
+// finished after a block barrier by the first threads.
+//
+// Jacobi at 257^3, tile and list kernels: 0.264 ms.  Slower: packed FMAs over the 36 sums, 0.290 (1/D
+// past the tiles, five blocks) and 0.296 (four); the register-marching form of the FP64 kernel, 0.315
+// at 112 registers and two blocks, 0.355 at 72 and three, two rows a thread 0.42-0.48.
+constexpr int SNT = STX * STY;
+constexpr int T32B = 36;                      // box width: 32 nodes + halo + alignment shift (<= 2)
+constexpr int T32X = T32B * SXR;              // elements per x component plane tile
+constexpr int T32V = T32B * STY;              // elements per b / 1/D / id component tile (no halo)
+#ifndef AE_SPLIT_PAIR_BLOCKS
+#define AE_SPLIT_PAIR_BLOCKS 5
+#endif
+struct TL32 {
+    static constexpr int XS = up128(3 * T32X * 4);  // bytes per x ring slot (planes k - 1, k, k + 1, one in flight)
+    static constexpr int VS = 3 * T32V * 4;         // bytes per b / 1/D ring slot (two)
+    static constexpr int GS = T32V * 4;             // bytes per id ring slot (two)
+    static constexpr int oB = 4 * XS, oI = oB + 2 * VS, oG = oI + 2 * VS, oBar = oG + 2 * GS;
+    static constexpr int oQ = oBar + 16, oQt = oQ + 16, oQf = oQt + 4 * SNT;  // queue: count, places, sums
+    static constexpr int oT = oQf + 3 * SNT * 4;
+    static constexpr unsigned kX = 3 * T32X * 4, kV = 3 * T32V * 4, kG = T32V * 4;
+    static_assert(VS % 128 == 0 && GS % 128 == 0 && oB % 128 == 0 && oT % 16 == 0, "TMA slots, table");
+};
+constexpr int kTab32SmemMax = 24 * 1024;  // bytes of grain table kept in shared memory
+template <int M, bool TABS, int OP>
+__global__ void __launch_bounds__(SNT / 2, AE_SPLIT_PAIR_BLOCKS)
+    k_sweep_tile32(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_b,
+                 const __grid_constant__ CUtensorMap tm_i, const __grid_constant__ CUtensorMap tm_g,
+                   SCoef<float> K, TileGeo T, int sh, int uniform, long long sy, long long sz, long long sc,
+                   const unsigned* __restrict__ gidm_g, const float* __restrict__ tab, int tab_n, float* __restrict__ xo,
+                   float omega, int* err) {
+    using R = float;
+    constexpr int NPT = 2, NT = SNT / NPT;  // rows per thread, threads per block
+    using L = TL32;
     constexpr int NC = NCoef<M>::value;
     // grain rows in shared memory padded to whole 16-byte vectors (four coefficients)
     constexpr int NCP = (NC + 3) / 4 * 4;
     constexpr int TS = TABS ? NCP : NC;  // row stride of the table the kernel reads
-    constexpr bool D64 = sizeof(R) == 8 && OP == SPLIT_JACOBI;
     extern __shared__ __align__(128) unsigned char smem[];
     auto xslot = [&](int k) { return reinterpret_cast<const R*>(smem + (k & 3) * L::XS); };
     const unsigned* gring = reinterpret_cast<const unsigned*>(smem + L::oG);
@@ -240,7 +526,7 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
     const bool act = i <= T.I.hi[0] && j <= T.I.hi[1];
     auto act_n = [&](int n) { return i <= T.I.hi[0] && j + n <= T.I.hi[1]; };  // node n of the thread
     // tensor coordinates of the boxes
-    const int xa = i0 - 1 - T.slo[0] - T.sh;
+    const int xa = i0 - 1 - T.slo[0] - sh;
     const int yx = j0 - 1 - T.slo[1], yv = j0 - T.slo[1];
     const unsigned sb = smem_u32(smem);
     const unsigned bar0 = sb + (unsigned)L::oBar;
@@ -259,11 +545,10 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
         const unsigned s = (unsigned)(k & 1);
         if (OP != SPLIT_FAPPLY) tma_load4(sb + (unsigned)L::oB + s * L::VS, &tm_b, xa, yv, k - T.slo[2], 0, bar);
         if (OP == SPLIT_JACOBI) tma_load4(sb + (unsigned)L::oI + s * L::VS, &tm_i, xa, yv, k - T.slo[2], 0, bar);
-        if (D64) tma_load4(sb + (unsigned)L::oD + s * L::VS, &tm_d, xa, yv, k - T.slo[2], 0, bar);
         tma_load4(sb + (unsigned)L::oG + s * L::GS, &tm_g, xa, yv, k - T.slo[2], 0, bar);
     };
-    constexpr unsigned kVTile = (OP == SPLIT_JACOBI ? (D64 ? 3 : 2) : OP == SPLIT_RESIDUAL ? 1 : 0) * L::kV + L::kG;
-    // stage 0: planes k0-1, k0, k0+1 of x and the b, 1/D (D), id tiles of plane k0
+    constexpr unsigned kVTile = (OP == SPLIT_JACOBI ? 2 : OP == SPLIT_RESIDUAL ? 1 : 0) * L::kV + L::kG;
+    // stage 0: planes k0-1, k0, k0+1 of x and the b, 1/D, id tiles of plane k0
     if (leader) {
         mbar_expect_tx(bar0, 3 * L::kX + kVTile);
         load_x(k0 - 1, bar0);
@@ -271,9 +556,9 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
         load_x(k0 + 1, bar0);
         load_v(k0, bar0);
     }
-    const int col = T.sh + 1 + tx;
-    const int cx = (ty + 1) * SBW + col;  // this node inside an x component tile
-    const int cv = ty * SBW + col;        // ... inside a b / 1/D / id component tile
+    const int col = sh + 1 + tx;
+    const int cx = (ty + 1) * T32B + col;  // this node inside an x component tile
+    const int cv = ty * T32B + col;        // ... inside a b / 1/D / id component tile
     long long o = (long long)(i - T.slo[0]) + (long long)(j - T.slo[1]) * sy + (long long)(k0 - T.slo[2]) * sz;
     bool failed = false;
     int last = 0;  // last stage issued
@@ -302,7 +587,6 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
         const R* pp = xslot(k + 1) + cx;
         const R* bv = reinterpret_cast<const R*>(smem + L::oB + vs * L::VS) + cv;
         const R* iv = reinterpret_cast<const R*>(smem + L::oI + vs * L::VS) + cv;
-        const R* dv = reinterpret_cast<const R*>(smem + L::oD + vs * L::VS) + cv;
         bool queued[NPT];
         R f[NPT][3], xv[NPT][3];
         // the 21 (9, 2, 45) coefficients of a node's grain, then its interior term div(C : grad grad x)
@@ -310,22 +594,13 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
             R a[NCP];
             const R* a0 = tb + (int)(gw & 0xffffu) * TS;
             if (TABS) {
-                if (sizeof(R) == 4) {
 #pragma unroll
-                    for (int q = 0; q < NCP; q += 4) {
-                        const float4 v = *reinterpret_cast<const float4*>(a0 + q);
-                        a[q] = (R)v.x;
-                        a[q + 1] = (R)v.y;
-                        a[q + 2] = (R)v.z;
-                        a[q + 3] = (R)v.w;
-                    }
-                } else {
-#pragma unroll
-                    for (int q = 0; q < NCP; q += 2) {
-                        const double2 v = *reinterpret_cast<const double2*>(a0 + q);
-                        a[q] = (R)v.x;
-                        a[q + 1] = (R)v.y;
-                    }
+                for (int q = 0; q < NCP; q += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(a0 + q);
+                    a[q] = v.x;
+                    a[q + 1] = v.y;
+                    a[q + 2] = v.z;
+                    a[q + 3] = v.w;
                 }
             } else {
 #pragma unroll
@@ -333,33 +608,7 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
             }
             div_of<M, R>(a, bb, fo);
         };
-        if constexpr (NPT == 1) {
-            queued[0] = false;
-            if (act) {
-                const unsigned gw = gring[vs * SVP + cv];
-                R bb[3][3][3];
-#pragma unroll
-                for (int p = 0; p < 3; ++p) {
-                    const R* um = pm + p * SXP;
-                    const R* uc = pc + p * SXP;
-                    const R* up = pp + p * SXP;
-                    const R c0 = uc[0];
-                    xv[0][p] = c0;
-                    const R xm = uc[-1], xp = uc[1], ym = uc[-SBW], yp = uc[SBW], zm = um[0], zp = up[0];
-                    bb[p][0][0] = (xp - R(2) * c0 + xm) * K.i2[0];
-                    bb[p][1][1] = (yp - R(2) * c0 + ym) * K.i2[1];
-                    bb[p][2][2] = (zp - R(2) * c0 + zm) * K.i2[2];
-                    bb[p][0][1] = (uc[1 + SBW] + uc[-1 - SBW] - uc[1 - SBW] - uc[-1 + SBW]) * K.m01;
-                    bb[p][0][2] = (up[1] + um[-1] - um[1] - up[-1]) * K.m02;
-                    bb[p][1][2] = (up[SBW] + um[-SBW] - um[SBW] - up[-SBW]) * K.m12;
-                    bb[p][1][0] = bb[p][0][1];
-                    bb[p][2][0] = bb[p][0][2];
-                    bb[p][2][1] = bb[p][1][2];
-                }
-                interior(gw, bb, f[0]);
-                queued[0] = !uniform && (gw >> 16) != 0;
-            }
-        } else {
+        {
 #pragma unroll
             for (int n = 0; n < NPT; ++n) queued[n] = false;
             if (act) {
@@ -370,18 +619,18 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
                 R h[NPT][3][6];
 #pragma unroll
                 for (int p = 0; p < 3; ++p) {
-                    const R* um = pm + p * SXP;
-                    const R* uc = pc + p * SXP;
-                    const R* up = pp + p * SXP;
+                    const R* um = pm + p * T32X;
+                    const R* uc = pc + p * T32X;
+                    const R* up = pp + p * T32X;
                     R ac[NR][3], am[NR][3], ap[NR][3];
 #pragma unroll
                     for (int r = 0; r < NR; ++r)
 #pragma unroll
                         for (int c = 0; c < 3; ++c) {
-                            ac[r][c] = uc[(r - 1) * SBW + c - 1];
+                            ac[r][c] = uc[(r - 1) * T32B + c - 1];
                             const bool need = (r >= 1 && r <= NPT) || c == 1;
-                            am[r][c] = need ? um[(r - 1) * SBW + c - 1] : R(0);
-                            ap[r][c] = need ? up[(r - 1) * SBW + c - 1] : R(0);
+                            am[r][c] = need ? um[(r - 1) * T32B + c - 1] : R(0);
+                            ap[r][c] = need ? up[(r - 1) * T32B + c - 1] : R(0);
                         }
 #pragma unroll
                     for (int n = 0; n < NPT; ++n) {
@@ -400,7 +649,7 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
 #pragma unroll
                 for (int n = 0; n < NPT; ++n) {
                     if (n > 0 && !act_n(n)) break;
-                    const unsigned gw = gring[vs * SVP + cv + n * SBW];
+                    const unsigned gw = gring[vs * T32V + cv + n * T32B];
                     R bb[3][3][3];
 #pragma unroll
                     for (int p = 0; p < 3; ++p) {
@@ -437,14 +686,13 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
             }
             if (an && !queued[n]) {
                 const long long on = o + n * sy;
-                const int vn = n * SBW;
+                const int vn = n * T32B;
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
                     if (OP == SPLIT_JACOBI)
-                        xo[on + r * sc] = jacobi_update<R>(xv[n][r], f[n][r], bv[vn + r * SVP],
-                                                           D64 ? dv[vn + r * SVP] : R(0), iv[vn + r * SVP], omega);
+                        xo[on + r * sc] = jacobi_update<R>(xv[n][r], sub_rn(bv[vn + r * T32V], f[n][r]), iv[vn + r * T32V], omega);
                     else if (OP == SPLIT_RESIDUAL)
-                        xo[on + r * sc] = bv[vn + r * SVP] - f[n][r];
+                        xo[on + r * sc] = bv[vn + r * T32V] - f[n][r];
                     else
                         xo[on + r * sc] = f[n][r];
                 }
@@ -456,7 +704,7 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
         for (int e = threadIdx.x; e < *qn; e += NT) {
             const int t = qtid[e];
             const int qx = t % STX, qy = t / STX;
-            const int qcx = (qy + 1) * SBW + T.sh + 1 + qx, qcv = qy * SBW + T.sh + 1 + qx;
+            const int qcx = (qy + 1) * T32B + sh + 1 + qx, qcv = qy * T32B + sh + 1 + qx;
             const long long qo = o + (long long)(qx - tx) + (long long)(qy - ty) * sy;
             const R* qm = xslot(k - 1) + qcx;
             const R* qc = xslot(k) + qcx;
@@ -464,17 +712,17 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
             R gu[3][3];
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
-                gu[p][0] = (qc[p * SXP + 1] - qc[p * SXP - 1]) * K.h[0];
-                gu[p][1] = (qc[p * SXP + SBW] - qc[p * SXP - SBW]) * K.h[1];
-                gu[p][2] = (qp[p * SXP] - qm[p * SXP]) * K.h[2];
+                gu[p][0] = (qc[p * T32X + 1] - qc[p * T32X - 1]) * K.h[0];
+                gu[p][1] = (qc[p * T32X + T32B] - qc[p * T32X - T32B]) * K.h[1];
+                gu[p][2] = (qp[p * T32X] - qm[p * T32X]) * K.h[2];
             }
             // neighbour ids: x from the tile, y from the tile inside it, the rest from global
-            const unsigned* gv = gring + vs * SVP + qcv;
+            const unsigned* gv = gring + vs * T32V + qcv;
             const unsigned mask = gv[0] >> 16;
             const int gid_n[3][2] = {
                 {(int)(gv[1] & 0xffffu), (int)(gv[-1] & 0xffffu)},
-                {(int)((qy + 1 < STY ? gv[SBW] : __ldg(gidm_g + qo + sy)) & 0xffffu),
-                 (int)((qy > 0 ? gv[-SBW] : __ldg(gidm_g + qo - sy)) & 0xffffu)},
+                {(int)((qy + 1 < STY ? gv[T32B] : __ldg(gidm_g + qo + sy)) & 0xffffu),
+                 (int)((qy > 0 ? gv[-T32B] : __ldg(gidm_g + qo - sy)) & 0xffffu)},
                 {(int)(__ldg(gidm_g + qo + sz) & 0xffffu), (int)(__ldg(gidm_g + qo - sz) & 0xffffu)}};
             R colv[3][3];
 #pragma unroll
@@ -489,16 +737,14 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
             }
             const R* qb = reinterpret_cast<const R*>(smem + L::oB + vs * L::VS) + qcv;
             const R* qi = reinterpret_cast<const R*>(smem + L::oI + vs * L::VS) + qcv;
-            const R* qd = reinterpret_cast<const R*>(smem + L::oD + vs * L::VS) + qcv;
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
                 R fr = qf[3 * e + r];
                 fr = gradc_add(fr, colv[0][r], colv[1][r], colv[2][r], K.h);
                 if (OP == SPLIT_JACOBI)
-                    xo[qo + r * sc] = jacobi_update<R>(qc[r * SXP], fr, qb[r * SVP], D64 ? qd[r * SVP] : R(0),
-                                                       qi[r * SVP], omega);
+                    xo[qo + r * sc] = jacobi_update<R>(qc[r * T32X], sub_rn(qb[r * T32V], fr), qi[r * T32V], omega);
                 else if (OP == SPLIT_RESIDUAL)
-                    xo[qo + r * sc] = qb[r * SVP] - fr;
+                    xo[qo + r * sc] = qb[r * T32V] - fr;
                 else
                     xo[qo + r * sc] = fr;
             }
@@ -517,13 +763,13 @@ __global__ void __launch_bounds__(SNT / NPT, NPT > 1 ? AE_SPLIT_PAIR_BLOCKS : si
 template <int M, class R, bool SAME>
 __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 4 : 2)
     k_jacobi_list(OpParams P, SCoef<R> K, const unsigned long long* __restrict__ list, long long n, Box3 S,
-                  View<const R> C, Grains<R> G, View<const R> invD, View<const R> D, View<const R> xi,
-                  View<const R> b, View<R> xo, R omega) {
+                  View<const R> C, Grains<R> G, View<const R> invD, View<const R> xi, View<const R> b, View<R> xo,
+                  R omega) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     int i, j, k;
     unpack_node(list[t], S.lo, i, j, k);
-    jacobi_node<M, R, true, SAME>(P, K, C, G, invD, D, xi, b, xo, omega, i, j, k);
+    jacobi_node<M, R, true, SAME>(P, K, C, G, invD, xi, b, xo, omega, i, j, k);
 }
 
 // r = b - A x at the listed nodes (the per-node residual, k_residual's arithmetic); r may alias b
@@ -537,12 +783,9 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 4 : 2)
     unpack_node(list[t], S.lo, i, j, k);
     R v[3];
     const long long ox = x.at(i, j, k);
-    apply_at<M, R, true>(P, K, C, G, x, i, j, k, ox, ox, v);
+    const R sc = apply_at<M, R, true>(P, K, C, G, x, i, j, k, ox, ox, v);
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        const R rv = b.p[ox + q * x.sc] - v[q];
-        r.p[ox + q * x.sc] = rv;
-    }
+    for (int q = 0; q < 3; ++q) r.p[ox + q * x.sc] = row_residual(b.p[ox + q * x.sc], sc, v[q]);
 }
 
 // f = A x at the listed nodes (k_fapply's arithmetic)
@@ -556,9 +799,9 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 4 : 2)
     unpack_node(list[t], S.lo, i, j, k);
     R v[3];
     const long long ox = x.at(i, j, k);
-    apply_at<M, R, true>(P, K, C, G, x, i, j, k, ox, ox, v);
+    const R sc = apply_at<M, R, true>(P, K, C, G, x, i, j, k, ox, ox, v);
 #pragma unroll
-    for (int q = 0; q < 3; ++q) f.p[ox + q * x.sc] = v[q];
+    for (int q = 0; q < 3; ++q) f.p[ox + q * x.sc] = mul_rn(sc, v[q]);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda)
@@ -578,8 +821,8 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 
 // Tensor map over a level array [comp][k][j][i] (storage box, row pitch px), boxes of
-// SBW x rows x 1 x ncomp elements of esize bytes.
-CUtensorMap level_tmap(const void* base, const Geo& g, int ncomp, int rows, CUtensorMapDataType type, int esize) {
+// width x rows x 1 x ncomp elements of esize bytes.
+CUtensorMap level_tmap(const void* base, const Geo& g, int ncomp, int width, int rows, CUtensorMapDataType type, int esize) {
     const Box3 s = geo_store(g);
     const cuuint64_t nx = (cuuint64_t)(s.hi[0] - s.lo[0] + 1), ny = (cuuint64_t)(s.hi[1] - s.lo[1] + 1),
                      nz = (cuuint64_t)(s.hi[2] - s.lo[2] + 1);
@@ -587,7 +830,7 @@ CUtensorMap level_tmap(const void* base, const Geo& g, int ncomp, int rows, CUte
     const cuuint64_t dims[4] = {nx, ny, nz, (cuuint64_t)ncomp};
     const cuuint64_t e = (cuuint64_t)esize;
     const cuuint64_t strides[3] = {px * e, px * ny * e, px * ny * nz * e};
-    const cuuint32_t box[4] = {(cuuint32_t)SBW, (cuuint32_t)rows, 1, (cuuint32_t)ncomp};
+    const cuuint32_t box[4] = {(cuuint32_t)width, (cuuint32_t)rows, 1, (cuuint32_t)ncomp};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     CUtensorMap m;
     const CUresult r = encode_fn()(&m, type, 4, const_cast<void*>(base), dims, strides, box, estr,
@@ -597,57 +840,82 @@ CUtensorMap level_tmap(const void* base, const Geo& g, int ncomp, int rows, CUte
     return m;
 }
 
-template <int M, class R, bool TABS, int OP, int NPT>
-void tile_smem_attr(size_t bytes) {
-    static size_t set = 0;
-    if (bytes > set) {
-        AE_CUDA_CHECK(cudaFuncSetAttribute(k_sweep_tile<M, R, TABS, OP, NPT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-        set = bytes;
-    }
+template <int M, class R, bool TABS, int OP>
+void tile_smem_attr() {
+    static std::once_flag once;
+    std::call_once(once, [] {
+        const int tables = !TABS ? 0 : sizeof(R) == 4 ? kTab32SmemMax : kTabSmemMax;
+        if constexpr (sizeof(R) == 4)
+            AE_CUDA_CHECK(cudaFuncSetAttribute(k_sweep_tile32<M, TABS, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               TL32::oT + tables));
+        else
+            AE_CUDA_CHECK(cudaFuncSetAttribute(k_sweep_tile64<M, TABS, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               TL<double>::oT + tables));
+    });
 }
 
-// the tiled kernel of one operation over I; b: the right-hand side, invD: 1/D and D (Jacobi only;
-// D read in FP64)
+// Planes per block: the split of nz planes into chunks that takes the fewest plane times, waves of
+// blocks times the planes a block goes through (two more than it computes, and about four plane times
+// to fill its ring).
+int tile_kz(long long tiles, int nz, long long wave) {
+    int best = nz;
+    long long cost = -1;
+    for (int n = 1; n <= (nz + 3) / 4; ++n) {
+        const int kz = (nz + n - 1) / n;
+        const long long c = ((tiles * ((nz + kz - 1) / kz) + wave - 1) / wave) * (kz + 6);
+        if (cost < 0 || c < cost) cost = c, best = kz;
+    }
+    return best;
+}
+
+// the tiled kernel of one operation over I; b: the right-hand side, invD: 1/D (Jacobi only)
 template <class R, int OP>
 void launch_tile(const OpParams& P, const SplitList& sl, const Box3& I, const Box3& S, View<const R> x, const R* b,
-                 const R* invD, const R* D, R* out, R omega, cudaStream_t st, Grains<R> G, int ngrains, int* err) {
-    const SCoef<R> K = make_scoef<R>(P.g);
-    const CUtensorMapDataType dt = sizeof(R) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
+                 const R* invD, R* out, R omega, cudaStream_t st, Grains<R> G, int ngrains, int* err) {
     constexpr int E = (int)sizeof(R);
+    constexpr bool F32 = E == 4;
+    const SCoef<R> K = make_scoef<R>(P.g);
+    const CUtensorMapDataType dt = F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
     dispatch_model<R>(P.model, [&](auto m) {
         constexpr int Mv = decltype(m)::value;
         TileGeo T;
         T.I = I;
         for (int q = 0; q < 3; ++q) T.slo[q] = S.lo[q];
-        const int nx = I.hi[0] - I.lo[0] + 1, ny = I.hi[1] - I.lo[1] + 1, nz = I.hi[2] - I.lo[2] + 1;
+        // FP32 tiles start at I's first column, FP64 tiles at the storage box's
+        const int nx = I.hi[0] - (F32 ? I : S).lo[0] + 1, ny = I.hi[1] - I.lo[1] + 1, nz = I.hi[2] - I.lo[2] + 1;
         T.tiles_x = (nx + STX - 1) / STX;
-        const int tiles_y = (ny + STY - 1) / STY;
-        T.kz = sl.kz > 0 ? sl.kz : 8;
-        // every tile starts 32 nodes after the previous one, so one shift serves all of them: the
-        // boxes' first column is then 16-byte aligned (x * E a multiple of 16)
-        T.sh = (I.lo[0] - 1 - S.lo[0]) & (16 / E - 1);
-        const CUtensorMap tx = level_tmap(x.p, P.g, 3, SXR, dt, E);
-        const CUtensorMap tb = level_tmap(b, P.g, 3, STY, dt, E);
-        const CUtensorMap ti = level_tmap(invD ? invD : b, P.g, 3, STY, dt, E);
-        const CUtensorMap td = level_tmap(D ? D : b, P.g, 3, STY, dt, E);
-        const CUtensorMap tg = level_tmap(sl.gidm, P.g, 1, STY, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4);
-        const dim3 grid((unsigned)(T.tiles_x * tiles_y), (unsigned)((nz + T.kz - 1) / T.kz));
-        const int tab_n = ngrains * NCoef<Mv>::value;
-        const int tab_pad = ngrains * ((NCoef<Mv>::value + 3) / 4 * 4);
-        const bool tabs = tab_pad * E <= kTabSmemMax;
-        const size_t smem = (size_t)TL<R>::oT + (tabs ? (size_t)tab_pad * E : 0);
-        constexpr int NPT = E == 4 ? AE_SPLIT_NPT32 : 1;
-        if (tabs) {
-            tile_smem_attr<Mv, R, true, OP, NPT>(smem);
-            k_sweep_tile<Mv, R, true, OP, NPT><<<grid, SNT / NPT, smem, st>>>(
-                tx, tb, ti, td, tg, K, T, P.uniform, x.sy, x.sz, x.sc, sl.gidm, G.tab, tab_n, out, omega, err);
-        } else {
-            tile_smem_attr<Mv, R, false, OP, NPT>(smem);
-            k_sweep_tile<Mv, R, false, OP, NPT><<<grid, SNT / NPT, smem, st>>>(
-                tx, tb, ti, td, tg, K, T, P.uniform, x.sy, x.sz, x.sc, sl.gidm, G.tab, tab_n, out, omega, err);
-        }
-        launched();
+        const int tiles = T.tiles_x * ((ny + STY - 1) / STY);
+        T.kz = sl.kz > 0 ? sl.kz : F32 ? 8 : tile_kz(tiles, nz, 152);
+        const int vw = F32 ? T32B : STX;
+        const CUtensorMap tx = level_tmap(x.p, P.g, 3, F32 ? T32B : TL<double>::BW, SXR, dt, E);
+        const CUtensorMap tb = level_tmap(b ? b : x.p, P.g, 3, vw, STY, dt, E);
+        const CUtensorMap ti = level_tmap(invD ? invD : x.p, P.g, 3, vw, STY, dt, E);
+        const CUtensorMap tg = level_tmap(sl.gidm, P.g, 1, vw, STY, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4);
+        const dim3 grid((unsigned)tiles, (unsigned)((nz + T.kz - 1) / T.kz));
+        const size_t rows_bytes = ((size_t)ngrains * row_stride<Mv>() * E + 15) / 16 * 16;
+        size_t tab_bytes = ((size_t)ngrains * NCoef<Mv>::value * E + 15) / 16 * 16;
+        if (rows_bytes + tab_bytes > kTabSmemMax) tab_bytes = 0;
+        // FP32: the stiffness table alone, rows padded to 16 bytes
+        const size_t pad_bytes = (size_t)ngrains * ((NCoef<Mv>::value + 3) / 4 * 4) * E;
+        const auto go = [&](auto tabs) {
+            constexpr bool TABS = decltype(tabs)::value;
+            tile_smem_attr<Mv, R, TABS, OP>();
+            if constexpr (F32) {
+                // every tile starts 32 nodes after the previous one, so one shift serves all of them: the
+                // boxes' first column is then a multiple of 4
+                const int sh = (I.lo[0] - 1 - S.lo[0]) & 3;
+                k_sweep_tile32<Mv, TABS, OP><<<grid, SNT / 2, TL32::oT + (TABS ? pad_bytes : 0), st>>>(
+                    tx, tb, ti, tg, K, T, sh, P.uniform, x.sy, x.sz, x.sc, sl.gidm, G.tab, ngrains * NCoef<Mv>::value, out, omega,
+                    err);
+            } else {
+                k_sweep_tile64<Mv, TABS, OP><<<grid, kTileThreads, TL<double>::oT + (TABS ? rows_bytes + tab_bytes : 0), st>>>(
+                    tx, tb, ti, tg, K, T, P.uniform, (int)x.sy, (int)x.sz, (int)x.sc, sl.gidm, G.tab, sl.rows64,
+                    TABS ? (int)rows_bytes : 0, TABS ? (int)tab_bytes : 0, x.p, b, invD, out, omega, err);
+            }
+            launched();
+        };
+        if (F32 ? pad_bytes <= kTab32SmemMax : rows_bytes <= kRowSmemMax) go(std::true_type());
+        else go(std::false_type());
     });
 }
 
@@ -664,11 +932,12 @@ bool split_supported(const Geo& g) {
     const Box3 S = geo_store(g);
     for (int q = 0; q < 3; ++q)
         if (S.hi[q] - S.lo[q] >= (1 << 21)) return false;
-    // the tiles' column shift (TileGeo::sh) must leave the 34 columns of a tile inside the box:
+    // the FP32 tiles' column shift (sh in launch_tile) must leave the 34 columns of a tile inside the box:
     // 0 on level 0 and on refined patches with 2 ghost layers, 1 or 2 where one touches the domain's
     // low face
     const Box3 I = split_interior(g);
-    return ((I.lo[0] - 1 - S.lo[0]) & 3) <= SBW - 34;
+    // and the tiled kernels' offsets into the three components are 32-bit
+    return ((I.lo[0] - 1 - S.lo[0]) & 3) <= T32B - 34 && 3 * geo_nn(g) < (1ll << 31);
 }
 
 // count and fill the list of region R \ I (and, with gidm, the id/mask array)
@@ -691,14 +960,29 @@ long long build_list(const Reg& reg, const Box3& R, const Box3& I, View<const un
     return (long long)n;
 }
 
-long long split_build(const Geo& g, View<const unsigned short> gid, SplitList& sl, cudaStream_t st,
-                      unsigned long long* scratch_count) {
+void split_free(SplitList& sl) {
+    cudaFree(sl.list);
+    cudaFree(sl.list_r);
+    cudaFree(sl.gidm);
+    cudaFree(sl.rows64);
+    sl = SplitList{};
+}
+
+long long split_build(const Geo& g, int model, View<const unsigned short> gid, int ngrains, const double* tab,
+                      SplitList& sl, cudaStream_t st, unsigned long long* scratch_count) {
     if (!split_supported(g)) throw std::runtime_error("split sweep: level layout not supported");
     const Box3 S = geo_store(g);
     const Reg reg = make_reg(S);
     const Box3 I = split_interior(g);
     AE_CUDA_CHECK(cudaMalloc(&sl.gidm, sizeof(unsigned) * (size_t)geo_nn(g)));
     AE_CUDA_CHECK(cudaMemsetAsync(sl.gidm, 0, sizeof(unsigned) * (size_t)geo_nn(g), st));
+    dispatch_model<double>(model, [&](auto m) {
+        constexpr int M = decltype(m)::value;
+        const size_t n = (size_t)ngrains * row_stride<M>() + 4;  // the bulk copy takes whole 16 bytes
+        AE_CUDA_CHECK(cudaMalloc(&sl.rows64, n * sizeof(double)));
+        k_row_table<M><<<nblocks((unsigned)ngrains), kBlock, 0, st>>>(tab, ngrains, sl.rows64);
+        launched();
+    });
     // the Jacobi sweep writes the whole storage box, the residual the apply region
     sl.n = build_list(reg, S, I, gid, sl.gidm, &sl.list, st, scratch_count);
     sl.n_r = build_list(reg, geo_apply_region(g), I, gid, nullptr, &sl.list_r, st, scratch_count);
@@ -706,22 +990,21 @@ long long split_build(const Geo& g, View<const unsigned short> gid, SplitList& s
 }
 
 template <class R>
-void launch_jacobi_split(const OpParams& P, const SplitList& sl, View<const R> C, View<const R> invD, View<const R> D,
-                         View<const R> xi, View<const R> b, View<R> xo, R omega, cudaStream_t st, Grains<R> G,
+void launch_jacobi_split(const OpParams& P, const SplitList& sl, View<const R> C, View<const R> invD, View<const R> xi,
+                         View<const R> b, View<R> xo, R omega, cudaStream_t st, Grains<R> G,
                          int ngrains, int* err) {
     const Box3 S = geo_store(P.g);
     const Box3 I = split_interior(P.g);
-    const bool same = same_layout(xi, C) && same_layout(xi, invD) && same_layout(xi, D) && same_layout(xi, b) &&
+    const bool same = same_layout(xi, C) && same_layout(xi, invD) && same_layout(xi, b) &&
                       same_layout(xi, xo);
     if (!same || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
     if (!box_empty(I))
-        launch_tile<R, SPLIT_JACOBI>(P, sl, I, S, xi, b.p, invD.p, sizeof(R) == 8 ? D.p : nullptr, xo.p, omega, st, G,
-                                     ngrains, err);
+        launch_tile<R, SPLIT_JACOBI>(P, sl, I, S, xi, b.p, invD.p, xo.p, omega, st, G, ngrains, err);
     if (sl.n > 0) {
         const SCoef<R> K = make_scoef<R>(P.g);
         dispatch_model<R>(P.model, [&](auto m) {
             k_jacobi_list<decltype(m)::value, R, true><<<(unsigned)((sl.n + kBlock - 1) / kBlock), kBlock, 0, st>>>(
-                P, K, sl.list, sl.n, S, C, G, invD, D, xi, b, xo, omega);
+                P, K, sl.list, sl.n, S, C, G, invD, xi, b, xo, omega);
         });
         launched();
     }
@@ -735,7 +1018,7 @@ void launch_residual_split(const OpParams& P, const SplitList& sl, View<const R>
     const bool same = same_layout(x, C) && same_layout(x, b) && same_layout(x, r);
     if (!same || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
     if (!box_empty(I))
-        launch_tile<R, SPLIT_RESIDUAL>(P, sl, I, S, x, b.p, nullptr, nullptr, r.p, R(0), st, G, ngrains, err);
+        launch_tile<R, SPLIT_RESIDUAL>(P, sl, I, S, x, b.p, nullptr, r.p, R(0), st, G, ngrains, err);
     if (sl.n_r > 0) {
         const SCoef<R> K = make_scoef<R>(P.g);
         dispatch_model<R>(P.model, [&](auto m) {
@@ -753,7 +1036,7 @@ void launch_fapply_split(const OpParams& P, const SplitList& sl, View<const R> C
     const Box3 I = split_interior(P.g);
     const bool same = same_layout(x, C) && same_layout(x, f);
     if (!same || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
-    if (!box_empty(I)) launch_tile<R, SPLIT_FAPPLY>(P, sl, I, S, x, x.p, nullptr, nullptr, f.p, R(0), st, G, ngrains, err);
+    if (!box_empty(I)) launch_tile<R, SPLIT_FAPPLY>(P, sl, I, S, x, (const R*)nullptr, nullptr, f.p, R(0), st, G, ngrains, err);
     if (sl.n_r > 0) {
         const SCoef<R> K = make_scoef<R>(P.g);
         dispatch_model<R>(P.model, [&](auto m) {
@@ -769,11 +1052,11 @@ template void launch_fapply_split<float>(const OpParams&, const SplitList&, View
 template void launch_fapply_split<double>(const OpParams&, const SplitList&, View<const double>, View<const double>,
                                           View<double>, cudaStream_t, Grains<double>, int, int*);
 template void launch_jacobi_split<float>(const OpParams&, const SplitList&, View<const float>, View<const float>,
-                                         View<const float>, View<const float>, View<const float>, View<float>, float,
+                                         View<const float>, View<const float>, View<float>, float,
                                          cudaStream_t, Grains<float>, int, int*);
 template void launch_jacobi_split<double>(const OpParams&, const SplitList&, View<const double>, View<const double>,
-                                          View<const double>, View<const double>, View<const double>, View<double>,
-                                          double, cudaStream_t, Grains<double>, int, int*);
+                                          View<const double>, View<const double>, View<double>, double,
+                                          cudaStream_t, Grains<double>, int, int*);
 template void launch_residual_split<float>(const OpParams&, const SplitList&, View<const float>, View<const float>,
                                            View<const float>, View<float>, cudaStream_t, Grains<float>, int, int*);
 template void launch_residual_split<double>(const OpParams&, const SplitList&, View<const double>, View<const double>,

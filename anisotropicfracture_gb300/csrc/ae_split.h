@@ -14,7 +14,8 @@ struct SplitList {
     unsigned long long* list_r = nullptr;  // the same for the residual's region grow(valid,1) ∩ domain
     long long n_r = 0;
     unsigned* gidm = nullptr;            // per stored node: grain id | grad C directions << 16
-    int kz = 0;                          // planes per block of the tiled kernel (0: default 8)
+    double* rows64 = nullptr;            // per grain: the numbers of its interior row (FP64 sweeps)
+    int kz = 0;                          // planes per block of the tiled kernel (0: chosen by its rule)
 };
 // grain ids the split sweep can carry next to its 3-bit direction mask
 constexpr int kSplitMaxGrains = 1 << 16;
@@ -25,15 +26,17 @@ Box3 split_interior(const Geo& g);
 // whether a level's layout allows the split sweep (row pitch a multiple of 4 nodes)
 bool split_supported(const Geo& g);
 // Build the node list and the id/mask array of a grain-map level (gid laid out like the level's
-// storage, at most kSplitMaxGrains grains); allocates sl.list and sl.gidm with cudaMalloc and
-// returns the list's length.  scratch_count: one device counter.  Synchronises the stream.
-long long split_build(const Geo& g, View<const unsigned short> gid, SplitList& sl, cudaStream_t st,
-                      unsigned long long* scratch_count);
+// storage, at most kSplitMaxGrains grains) and the grains' row numbers; allocates sl's arrays with
+// cudaMalloc and returns the list's length.  scratch_count: one device counter.  Synchronises the
+// stream.
+long long split_build(const Geo& g, int model, View<const unsigned short> gid, int ngrains, const double* tab,
+                      SplitList& sl, cudaStream_t st, unsigned long long* scratch_count);
+void split_free(SplitList& sl);
 // One damped-Jacobi sweep (FP32 or FP64) of a grain-map level: the tiled interior kernel, then the
 // list.  *err is set (device) when a TMA load of the tiled kernel did not complete.
 template <class R>
-void launch_jacobi_split(const OpParams& P, const SplitList& sl, View<const R> C, View<const R> invD, View<const R> D,
-                         View<const R> xi, View<const R> b, View<R> xo, R omega, cudaStream_t st, Grains<R> G,
+void launch_jacobi_split(const OpParams& P, const SplitList& sl, View<const R> C, View<const R> invD, View<const R> xi,
+                         View<const R> b, View<R> xo, R omega, cudaStream_t st, Grains<R> G,
                          int ngrains, int* err);
 // f = A x on the apply region of a grain-map level, the same split (f other than x).
 template <class R>
