@@ -643,8 +643,9 @@ __device__ __forceinline__ R row_gradc(const SCoef<R>& K, R f, R c0, R c1, R c2)
 // C : grad grad u + sum_d (d_d C : grad u) e_d  (src/Operator/Elastic.cpp:174-258).
 // u and C are read through views whose strides may differ.  LDG = false when C lives in
 // shared memory.  Returns the factor that A u is f times: row_factor on interior rows, 1 on boundary
-// rows (b - A u is then one fused operation a component, row_residual).
-template <int M, class R, bool LDG = true>
+// rows (b - A u is then one fused operation a component, row_residual).  IN: the node is known to be
+// inside the domain's boundary.
+template <int M, class R, bool LDG = true, bool IN = false>
 __device__ __forceinline__ R apply_node(const Geo& g, const SCoef<R>& K, const BCP& bc, bool uniform,
                                            const R* __restrict__ C, long long cs, long long cc,
                                            long long csy, long long csz, const R* __restrict__ U,
@@ -652,7 +653,7 @@ __device__ __forceinline__ R apply_node(const Geo& g, const SCoef<R>& K, const B
                                            int k, R f[3]) {
     constexpr int NC = NCoef<M>::value;
     R nrm[3];
-    const int face = classify<R>(g, i, j, k, nrm);
+    const int face = IN ? -1 : classify<R>(g, i, j, k, nrm);
     if (face >= 0) {
         // one-sided first derivatives: Hi stencil on the lo face, Lo on the hi face
         const int ci[3] = {i, j, k};
@@ -708,7 +709,7 @@ __device__ __forceinline__ R apply_node(const Geo& g, const SCoef<R>& K, const B
 // and a per-grain coefficient table (tab[g * ncoef + q]): the same arithmetic on the same values.
 // A direction whose two neighbours lie in one grain has an exactly zero stiffness difference; its
 // grad C column is zero and its table reads are skipped.
-template <int M, class R>
+template <int M, class R, bool IN = false>
 __device__ __forceinline__ R apply_node_grains(const Geo& g, const SCoef<R>& K, const BCP& bc, bool uniform,
                                                   const unsigned short* __restrict__ gid, long long gc,
                                                   long long gsy, long long gsz, const R* __restrict__ tab,
@@ -717,7 +718,7 @@ __device__ __forceinline__ R apply_node_grains(const Geo& g, const SCoef<R>& K, 
     constexpr int NC = NCoef<M>::value;
     const R* a0 = tab + (int)__ldg(gid + gc) * NC;
     R nrm[3];
-    const int face = classify<R>(g, i, j, k, nrm);
+    const int face = IN ? -1 : classify<R>(g, i, j, k, nrm);
     if (face >= 0) {
         const int ci[3] = {i, j, k};
         const long long os[3] = {1, usy, usz};

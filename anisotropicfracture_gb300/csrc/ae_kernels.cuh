@@ -45,6 +45,65 @@ __device__ __forceinline__ void reg_ijk(const Reg& r, unsigned t, int& i, int& j
     j = r.lo[1] + (int)jj;
     k = r.lo[2] + (int)kk;
 }
+// A region as the part inside a box, and the slabs around that part.  Per-node sweeps run the inside
+// first and the slabs in further blocks of the same launch: a warp that mixes a boundary row's one-sided
+// gradient and stress with interior rows pays for both, and with rows of 65 nodes nearly every warp did
+// (in FP64 about 70 operations on top of 100).  65^3 isotropic solve, all levels: Jacobi 28.6 -> 21.1 us a
+// sweep, residual 27.8 -> 20.3; 97 x 81 x 113 cubic Jacobi 470 -> 407; FP32 unchanged (129^3 Fapply 97).
+struct Parts {
+    Reg in;               // n == 0: none
+    Reg slab[6];
+    unsigned end[6];      // nodes of slabs 0 .. q
+    unsigned in_blocks;
+};
+inline Parts make_parts(const Box3& r, Box3 inside) {
+    Parts P;
+    inside = box_isect(inside, r);
+    Box3 rest = r;
+    Box3 s[6];
+    for (Box3& b : s) {
+        b = r;
+        b.hi[0] = b.lo[0] - 1;  // empty
+    }
+    if (box_empty(inside)) {
+        s[0] = r;
+        inside = s[5];
+    } else {
+        for (int d = 2, q = 0; d >= 0; --d, q += 2) {
+            s[q] = s[q + 1] = rest;
+            s[q].hi[d] = inside.lo[d] - 1;
+            s[q + 1].lo[d] = inside.hi[d] + 1;
+            rest.lo[d] = inside.lo[d];
+            rest.hi[d] = inside.hi[d];
+        }
+    }
+    P.in = make_reg(inside);
+    unsigned n = 0;
+    for (int q = 0; q < 6; ++q) {
+        P.slab[q] = make_reg(s[q]);
+        n += P.slab[q].n;
+        P.end[q] = n;
+    }
+    P.in_blocks = (P.in.n + kBlock - 1) / kBlock;
+    return P;
+}
+inline unsigned parts_blocks(const Parts& P) { return P.in_blocks + (P.end[5] + kBlock - 1) / kBlock; }
+// this thread's node; false: none.  The whole block is inside or outside.
+__device__ __forceinline__ bool parts_ijk(const Parts& P, bool inside, int& i, int& j, int& k) {
+    if (inside) {
+        const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+        if (t >= P.in.n) return false;
+        reg_ijk(P.in, t, i, j, k);
+        return true;
+    }
+    unsigned t = (blockIdx.x - P.in_blocks) * blockDim.x + threadIdx.x;
+    if (t >= P.end[5]) return false;
+    int q = 0;
+    unsigned before = 0;
+    while (t >= P.end[q]) before = P.end[q++];
+    reg_ijk(P.slab[q], t - before, i, j, k);
+    return true;
+}
 inline unsigned nblocks(unsigned n) { return (n + kBlock - 1) / kBlock; }
 
 // after every kernel launch: surface launch errors and count the launch
@@ -76,27 +135,27 @@ __device__ __forceinline__ void block_max_atomic(double v, unsigned long long* o
 // f = A u at one node: through the grain tables when the level has them (G.gid laid out like C),
 // otherwise through the per-node stiffness C
 // (GR: compiled for the grain tables, so each variant keeps its own register budget)
-template <int M, class R, bool GR>
+template <int M, class R, bool GR, bool IN>
 __device__ __forceinline__ R apply_any(const OpParams& P, const SCoef<R>& K, const View<const R>& C,
                                           const Grains<R>& G, const View<const R>& u, int i, int j, int k, R v[3]) {
     if constexpr (GR)
-        return apply_node_grains<M, R>(P.g, K, P.bc, P.uniform, G.gid, C.at(i, j, k), C.sy, C.sz, G.tab, u.p, u.sc,
+        return apply_node_grains<M, R, IN>(P.g, K, P.bc, P.uniform, G.gid, C.at(i, j, k), C.sy, C.sz, G.tab, u.p, u.sc,
                                 u.at(i, j, k), u.sy, u.sz, i, j, k, v);
     else
-        return apply_node<M, R>(P.g, K, P.bc, P.uniform, C.p, C.sc, C.at(i, j, k), C.sy, C.sz, u.p, u.sc, u.at(i, j, k),
+        return apply_node<M, R, true, IN>(P.g, K, P.bc, P.uniform, C.p, C.sc, C.at(i, j, k), C.sy, C.sz, u.p, u.sc, u.at(i, j, k),
                          u.sy, u.sz, i, j, k, v);
 }
 
 // The same with the node's offsets given: oc into C (and the grain ids), ou into u
-template <int M, class R, bool GR>
+template <int M, class R, bool GR, bool IN = false>
 __device__ __forceinline__ R apply_at(const OpParams& P, const SCoef<R>& K, const View<const R>& C,
                                          const Grains<R>& G, const View<const R>& u, int i, int j, int k,
                                          long long oc, long long ou, R v[3]) {
     if constexpr (GR)
-        return apply_node_grains<M, R>(P.g, K, P.bc, P.uniform, G.gid, oc, C.sy, C.sz, G.tab, u.p, u.sc, ou, u.sy, u.sz, i,
+        return apply_node_grains<M, R, IN>(P.g, K, P.bc, P.uniform, G.gid, oc, C.sy, C.sz, G.tab, u.p, u.sc, ou, u.sy, u.sz, i,
                                 j, k, v);
     else
-        return apply_node<M, R>(P.g, K, P.bc, P.uniform, C.p, C.sc, oc, C.sy, C.sz, u.p, u.sc, ou, u.sy, u.sz, i, j, k, v);
+        return apply_node<M, R, true, IN>(P.g, K, P.bc, P.uniform, C.p, C.sc, oc, C.sy, C.sz, u.p, u.sc, ou, u.sy, u.sz, i, j, k, v);
 }
 
 // true when two views index the same storage layout (same box origin and strides): the
@@ -124,14 +183,14 @@ constexpr int sweep_min_blocks() {
 
 // ------------------------------------------------------------------ Fapply
 template <int M, class R, bool GR>
-__global__ void __launch_bounds__(kBlock) k_fapply(OpParams P, SCoef<R> K, Reg reg, View<const R> C, Grains<R> G,
+__global__ void __launch_bounds__(kBlock) k_fapply(OpParams P, SCoef<R> K, Parts parts, View<const R> C, Grains<R> G,
                                                    View<const R> u, View<R> f) {
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= reg.n) return;
+    const bool inside = blockIdx.x < parts.in_blocks;
     int i, j, k;
-    reg_ijk(reg, t, i, j, k);
+    if (!parts_ijk(parts, inside, i, j, k)) return;
     R v[3];
-    const R sc = apply_any<M, R, GR>(P, K, C, G, u, i, j, k, v);
+    const R sc = inside ? apply_any<M, R, GR, true>(P, K, C, G, u, i, j, k, v)
+                        : apply_any<M, R, GR, false>(P, K, C, G, u, i, j, k, v);
     const long long o = f.at(i, j, k);
 #pragma unroll
     for (int n = 0; n < 3; ++n) f.p[o + n * f.sc] = mul_rn(sc, v[n]);
@@ -139,21 +198,21 @@ __global__ void __launch_bounds__(kBlock) k_fapply(OpParams P, SCoef<R> K, Reg r
 
 // ------------------------------------------------------------------ residual (+ norm, + FP32 copy)
 template <int M, class R, bool NORM, bool R32, bool GR, bool SAME>
-__global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_residual(OpParams P, SCoef<R> K, Reg reg,
+__global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_residual(OpParams P, SCoef<R> K, Parts parts,
                                                                                  View<const R> C, Grains<R> G,
                                                                                  View<const R> x, View<const R> b,
                                                                                  View<R> r, unsigned long long* norm,
                                                                                  View<float> r32) {
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool inside = blockIdx.x < parts.in_blocks;
     double mx = 0.0;
-    if (t < reg.n) {
-        int i, j, k;
-        reg_ijk(reg, t, i, j, k);
+    int i, j, k;
+    if (parts_ijk(parts, inside, i, j, k)) {
         R v[3];
         // SAME: every view has the layout of x (checked by the launcher)
         const long long ox = x.at(i, j, k);
         const long long oc = SAME ? ox : C.at(i, j, k);
-        const R sc = apply_at<M, R, GR>(P, K, C, G, x, i, j, k, oc, ox, v);
+        const R sc = inside ? apply_at<M, R, GR, true>(P, K, C, G, x, i, j, k, oc, ox, v)
+                            : apply_at<M, R, GR, false>(P, K, C, G, x, i, j, k, oc, ox, v);
         const long long ob = SAME ? ox : b.at(i, j, k), orr = SAME ? ox : r.at(i, j, k);
         const long long o32 = SAME ? ox : (R32 ? r32.at(i, j, k) : 0);
         const long long bsc = SAME ? x.sc : b.sc, rsc = SAME ? x.sc : r.sc, r32sc = SAME ? x.sc : r32.sc;
@@ -179,7 +238,7 @@ __device__ __forceinline__ R jacobi_update(R xv, R r, R invd, R omega) {
     return fma_rn(mul_rn(omega, r), invd, xv);
 }
 
-template <int M, class R, bool GR, bool SAME>
+template <int M, class R, bool GR, bool SAME, bool IN = false>
 __device__ __forceinline__ void jacobi_node(const OpParams& P, const SCoef<R>& K, const View<const R>& C,
                                             const Grains<R>& G, const View<const R>& invD,
                                             const View<const R>& xi, const View<const R>& b, const View<R>& xo,
@@ -189,20 +248,20 @@ __device__ __forceinline__ void jacobi_node(const OpParams& P, const SCoef<R>& K
     const long long ox = xi.at(i, j, k), oo = SAME ? ox : xo.at(i, j, k);
     const long long xsc = xi.sc, osc = SAME ? xsc : xo.sc;
     // outside the domain: untouched
-    if (!in_box(g.dlo, g.dhi, i, j, k)) {
+    if (!IN && !in_box(g.dlo, g.dhi, i, j, k)) {
 #pragma unroll
         for (int n = 0; n < 3; ++n) xo.p[oo + n * osc] = xi.p[ox + n * xsc];
         return;
     }
     // outermost ring of grow(valid, 2): zero
-    if (g.ng >= 2 && (i == g.vlo[0] - 2 || i == g.vhi[0] + 2 || j == g.vlo[1] - 2 || j == g.vhi[1] + 2 ||
-                      k == g.vlo[2] - 2 || k == g.vhi[2] + 2)) {
+    if (!IN && g.ng >= 2 && (i == g.vlo[0] - 2 || i == g.vhi[0] + 2 || j == g.vlo[1] - 2 || j == g.vhi[1] + 2 ||
+                             k == g.vlo[2] - 2 || k == g.vhi[2] + 2)) {
 #pragma unroll
         for (int n = 0; n < 3; ++n) xo.p[oo + n * osc] = R(0);
         return;
     }
     R v[3];
-    const R sc = apply_at<M, R, GR>(P, K, C, G, xi, i, j, k, SAME ? ox : C.at(i, j, k), ox, v);
+    const R sc = apply_at<M, R, GR, IN>(P, K, C, G, xi, i, j, k, SAME ? ox : C.at(i, j, k), ox, v);
     const long long od = SAME ? ox : invD.at(i, j, k), ob = SAME ? ox : b.at(i, j, k);
     const long long isc = SAME ? xsc : invD.sc, bsc = SAME ? xsc : b.sc;
 #pragma unroll
@@ -239,16 +298,16 @@ __global__ void __launch_bounds__(kBlock) k_jacobi_zero(Geo g, Reg reg, View<con
 }
 
 template <int M, class R, bool GR, bool SAME>
-__global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_jacobi(OpParams P, SCoef<R> K, Reg reg,
+__global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_jacobi(OpParams P, SCoef<R> K, Parts parts,
                                                                                View<const R> C, Grains<R> G,
                                                                                View<const R> invD,
                                                                                View<const R> xi, View<const R> b,
                                                                                View<R> xo, R omega) {
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= reg.n) return;
+    const bool inside = blockIdx.x < parts.in_blocks;
     int i, j, k;
-    reg_ijk(reg, t, i, j, k);
-    jacobi_node<M, R, GR, SAME>(P, K, C, G, invD, xi, b, xo, omega, i, j, k);
+    if (!parts_ijk(parts, inside, i, j, k)) return;
+    if (inside) jacobi_node<M, R, GR, SAME, true>(P, K, C, G, invD, xi, b, xo, omega, i, j, k);
+    else jacobi_node<M, R, GR, SAME, false>(P, K, C, G, invD, xi, b, xo, omega, i, j, k);
 }
 
 // ------------------------------------------------------------------ z-marching tiled stencil sweeps

@@ -56,6 +56,14 @@ inline Box3 geo_apply_region(const Geo& g) {
 template <class R>
 SCoef<R> make_scoef(const Geo& g) { return scoef_of<R>(g.dx); }
 
+// Nodes with an interior row: grow(valid, 1) without the domain's boundary nodes, with a one-node halo
+// inside the storage box.
+inline Box3 geo_interior(const Geo& g) {
+    Box3 d = geo_domain(g);
+    for (int q = 0; q < 3; ++q) { d.lo[q] += 1; d.hi[q] -= 1; }
+    return box_isect(box_isect(box_grow(geo_valid(g), 1), d), box_grow(geo_store(g), -1));
+}
+
 // View over a level's storage box (the layout of every internal array).
 template <class T>
 View<T> level_view(const Geo& g, T* p) {

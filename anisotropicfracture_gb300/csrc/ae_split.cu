@@ -921,12 +921,6 @@ void launch_tile(const OpParams& P, const SplitList& sl, const Box3& I, const Bo
 
 }  // namespace
 
-Box3 split_interior(const Geo& g) {
-    Box3 d = geo_domain(g);
-    for (int q = 0; q < 3; ++q) { d.lo[q] += 1; d.hi[q] -= 1; }
-    return box_isect(box_isect(box_grow(geo_valid(g), 1), d), box_grow(geo_store(g), -1));
-}
-
 bool split_supported(const Geo& g) {
     if (g.px <= 0 || g.px % 4 != 0) return false;
     const Box3 S = geo_store(g);
@@ -935,7 +929,7 @@ bool split_supported(const Geo& g) {
     // the FP32 tiles' column shift (sh in launch_tile) must leave the 34 columns of a tile inside the box:
     // 0 on level 0 and on refined patches with 2 ghost layers, 1 or 2 where one touches the domain's
     // low face
-    const Box3 I = split_interior(g);
+    const Box3 I = geo_interior(g);
     // and the tiled kernels' offsets into the three components are 32-bit
     return ((I.lo[0] - 1 - S.lo[0]) & 3) <= T32B - 34 && 3 * geo_nn(g) < (1ll << 31);
 }
@@ -973,7 +967,7 @@ long long split_build(const Geo& g, int model, View<const unsigned short> gid, i
     if (!split_supported(g)) throw std::runtime_error("split sweep: level layout not supported");
     const Box3 S = geo_store(g);
     const Reg reg = make_reg(S);
-    const Box3 I = split_interior(g);
+    const Box3 I = geo_interior(g);
     AE_CUDA_CHECK(cudaMalloc(&sl.gidm, sizeof(unsigned) * (size_t)geo_nn(g)));
     AE_CUDA_CHECK(cudaMemsetAsync(sl.gidm, 0, sizeof(unsigned) * (size_t)geo_nn(g), st));
     dispatch_model<double>(model, [&](auto m) {
@@ -994,7 +988,7 @@ void launch_jacobi_split(const OpParams& P, const SplitList& sl, View<const R> C
                          View<const R> b, View<R> xo, R omega, cudaStream_t st, Grains<R> G,
                          int ngrains, int* err) {
     const Box3 S = geo_store(P.g);
-    const Box3 I = split_interior(P.g);
+    const Box3 I = geo_interior(P.g);
     const bool same = same_layout(xi, C) && same_layout(xi, invD) && same_layout(xi, b) &&
                       same_layout(xi, xo);
     if (!same || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
@@ -1014,7 +1008,7 @@ template <class R>
 void launch_residual_split(const OpParams& P, const SplitList& sl, View<const R> C, View<const R> x, View<const R> b,
                            View<R> r, cudaStream_t st, Grains<R> G, int ngrains, int* err) {
     const Box3 S = geo_store(P.g);
-    const Box3 I = split_interior(P.g);
+    const Box3 I = geo_interior(P.g);
     const bool same = same_layout(x, C) && same_layout(x, b) && same_layout(x, r);
     if (!same || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
     if (!box_empty(I))
@@ -1033,7 +1027,7 @@ template <class R>
 void launch_fapply_split(const OpParams& P, const SplitList& sl, View<const R> C, View<const R> x, View<R> f,
                          cudaStream_t st, Grains<R> G, int ngrains, int* err) {
     const Box3 S = geo_store(P.g);
-    const Box3 I = split_interior(P.g);
+    const Box3 I = geo_interior(P.g);
     const bool same = same_layout(x, C) && same_layout(x, f);
     if (!same || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
     if (!box_empty(I)) launch_tile<R, SPLIT_FAPPLY>(P, sl, I, S, x, (const R*)nullptr, nullptr, f.p, R(0), st, G, ngrains, err);

@@ -20,9 +20,6 @@ struct SplitList {
 // grain ids the split sweep can carry next to its 3-bit direction mask
 constexpr int kSplitMaxGrains = 1 << 16;
 
-// Interior box of the tiled kernel: grow(valid, 1) without the domain's boundary nodes, with a
-// one-node halo inside the storage box.
-Box3 split_interior(const Geo& g);
 // whether a level's layout allows the split sweep (row pitch a multiple of 4 nodes)
 bool split_supported(const Geo& g);
 // Build the node list and the id/mask array of a grain-map level (gid laid out like the level's
