@@ -17,6 +17,17 @@ std::atomic<long long> g_kernel_launches{0};
 AE_INST_COPY(double, double)
 AE_INST_COPY(double, float)
 
+// a / d from inv = 1 / d: the product and one correction by its remainder
+__device__ __forceinline__ double div_by(double a, double d, double inv) {
+    const double q = a * inv;
+    const double c = fma(fma(-d, q, a), inv, q);
+    // outside the range where the remainder is exact, or with infinities, divide
+    const unsigned e = ((unsigned)__double2hiint(c) >> 20) & 0x7ff, ed = ((unsigned)__double2hiint(d) >> 20) & 0x7ff,
+                   ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ff;
+    const bool zero = (__double_as_longlong(a) << 1) == 0;
+    return ed - 64u < 0x780u && (zero || (e - 64u < 0x780u && ea - 64u < 0x780u)) ? c : a / d;
+}
+
 // ------------------------------------------------------------------ BC::Operator::Elastic::Init
 // src/BC/Operator/Elastic.H:106-181: boundary values into the rhs on every domain-boundary node.
 struct BCVal {
@@ -84,8 +95,13 @@ void launch_grains_box(const Box3& region, View<const int> ids, View<unsigned sh
 // Affine::Cubic::Combine (src/Model/Solid/Affine/Cubic.H:70-82): the weight of phase n at a node
 // is its mean over the four cells (i-1..i, j-1..j) of cell layer k, divided by the sum of those
 // means; stiffness slots and eigenstrain are the weighted sums of the per-phase tables.
-template <int NC>
-__global__ void __launch_bounds__(kBlock) k_model_mixture(Reg reg, View<const double> eta, int np,
+// NP: the number of phases, 0 for more than kMixPhases.  Bound by FP64 operations: the means are kept
+// instead of formed twice, and the weights are one division and three operations each (the product with
+// the reciprocal corrected by its remainder) instead of a division each.  129^3 nodes, three phases with
+// eigenstrains: 0.52 -> 0.475 ms.
+constexpr int kMixPhases = 6;
+template <int NC, int NP>
+__global__ void __launch_bounds__(kBlock) k_model_mixture(Reg reg, View<const double> eta, int np_,
                                                           const double* __restrict__ tab,
                                                           const double* __restrict__ f0tab, View<double> C,
                                                           View<double> F0, int* bad) {
@@ -93,44 +109,69 @@ __global__ void __launch_bounds__(kBlock) k_model_mixture(Reg reg, View<const do
     if (t >= reg.n) return;
     int i, j, k;
     reg_ijk(reg, t, i, j, k);
+    const int np = NP ? NP : np_;
     const long long o00 = eta.at(i, j, k), o01 = eta.at(i, j - 1, k);
     const long long o10 = eta.at(i - 1, j, k), o11 = eta.at(i - 1, j - 1, k);
-    double sum = 0.0;
-    for (int n = 0; n < np; ++n) {
+    const auto mean = [&](int n) {
         const double* e = eta.p + n * eta.sc;
-        sum += 0.25 * (e[o00] + e[o01] + e[o10] + e[o11]);
+        return 0.25 * (e[o00] + e[o01] + e[o10] + e[o11]);
+    };
+    double sum = 0.0, m[NP ? NP : 1];
+#pragma unroll
+    for (int n = 0; n < np; ++n) {
+        const double v = mean(n);
+        if (NP) m[NP ? n : 0] = v;
+        sum += v;
     }
     if (sum == 0.0 || isnan(sum)) {
         atomicExch(bad, 1);
         return;
     }
+    const double inv = 1.0 / sum;
     double acc[NC], f[9];
     for (int q = 0; q < NC; ++q) acc[q] = 0.0;
     for (int r = 0; r < 9; ++r) f[r] = 0.0;
+#pragma unroll
     for (int n = 0; n < np; ++n) {
-        const double* e = eta.p + n * eta.sc;
-        const double w = 0.25 * (e[o00] + e[o01] + e[o10] + e[o11]) / sum;
-        for (int q = 0; q < NC; ++q) acc[q] += tab[n * NC + q] * w;
+        const double w = div_by(NP ? m[NP ? n : 0] : mean(n), sum, inv);
+#pragma unroll
+        for (int q = 0; q < NC; ++q) acc[q] += __ldg(tab + n * NC + q) * w;
         if (F0.p)
-            for (int r = 0; r < 9; ++r) f[r] += f0tab[n * 9 + r] * w;
+#pragma unroll
+            for (int r = 0; r < 9; ++r) f[r] += __ldg(f0tab + n * 9 + r) * w;
     }
     const long long o = C.at(i, j, k);
+#pragma unroll
     for (int q = 0; q < NC; ++q) C.p[o + q * C.sc] = acc[q];
     if (F0.p) {
         const long long of = F0.at(i, j, k);
+#pragma unroll
         for (int r = 0; r < 9; ++r) F0.p[of + r * F0.sc] = f[r];
+    }
+}
+template <int NC>
+void mixture_nc(const Reg& reg, View<const double> eta, int np, const double* tab, const double* f0tab, View<double> C,
+                View<double> F0, int* bad, cudaStream_t st) {
+    const auto go = [&](auto n) {
+        k_model_mixture<NC, decltype(n)::value><<<nblocks(reg.n), kBlock, 0, st>>>(reg, eta, np, tab, f0tab, C, F0, bad);
+    };
+    switch (np) {
+        case 1: go(std::integral_constant<int, 1>()); break;
+        case 2: go(std::integral_constant<int, 2>()); break;
+        case 3: go(std::integral_constant<int, 3>()); break;
+        case 4: go(std::integral_constant<int, 4>()); break;
+        case 5: go(std::integral_constant<int, 5>()); break;
+        case kMixPhases: go(std::integral_constant<int, kMixPhases>()); break;
+        default: go(std::integral_constant<int, 0>());
     }
 }
 void launch_model_mixture(const Box3& region, int nc, View<const double> eta, int np, const double* tab,
                           const double* f0tab, View<double> C, View<double> F0, int* bad, cudaStream_t st) {
     const Reg reg = make_reg(region);
     if (reg.n == 0) return;
-    if (nc == 2)
-        k_model_mixture<2><<<nblocks(reg.n), kBlock, 0, st>>>(reg, eta, np, tab, f0tab, C, F0, bad);
-    else if (nc == 9)
-        k_model_mixture<9><<<nblocks(reg.n), kBlock, 0, st>>>(reg, eta, np, tab, f0tab, C, F0, bad);
-    else
-        k_model_mixture<21><<<nblocks(reg.n), kBlock, 0, st>>>(reg, eta, np, tab, f0tab, C, F0, bad);
+    if (nc == 2) mixture_nc<2>(reg, eta, np, tab, f0tab, C, F0, bad, st);
+    else if (nc == 9) mixture_nc<9>(reg, eta, np, tab, f0tab, C, F0, bad, st);
+    else mixture_nc<21>(reg, eta, np, tab, f0tab, C, F0, bad, st);
     launched();
 }
 
@@ -988,16 +1029,6 @@ __device__ __forceinline__ void div2(double a, double b, double c, double d, int
     q0 = __shfl_sync(0xffffffffu, q, 0);
     q1 = __shfl_sync(0xffffffffu, q, 1);
 }
-// a / d from inv = 1 / d: the product and one correction by its remainder
-__device__ __forceinline__ double div_by(double a, double d, double inv) {
-    const double q = a * inv;
-    const double c = fma(fma(-d, q, a), inv, q);
-    // outside the range where the remainder is exact, or with infinities, divide
-    const unsigned e = ((unsigned)__double2hiint(c) >> 20) & 0x7ff, ed = ((unsigned)__double2hiint(d) >> 20) & 0x7ff,
-                   ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ff;
-    return e - 64u < 0x780u && ed - 64u < 0x780u && ea - 64u < 0x780u ? c : a / d;
-}
-
 template <class R, int E>
 __global__ void __launch_bounds__(kEllThreads) k_bottom_quad(BottomArgs a, BottomEll m, const R* __restrict__ bg,
                                                              R* __restrict__ xg) {
