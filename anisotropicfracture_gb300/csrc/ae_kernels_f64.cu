@@ -219,30 +219,40 @@ void launch_model_degraded(const Box3& region, const Box3& valid, View<const dou
 }
 
 // ------------------------------------------------------------------ Strain / Stress / Energy
-// src/Operator/Elastic.cpp:399-572 (valid box, boundary-aware first derivatives)
+// src/Operator/Elastic.cpp:399-572 (valid box, boundary-aware first derivatives).  inside: no face of
+// the domain at this node.
 __device__ __forceinline__ void grad_at(const Geo& g, const SCoef<double>& K, const View<const double>& u, int i,
-                                        int j, int k, double gu[3][3]) {
+                                        int j, int k, double gu[3][3], bool inside = false) {
     const int ci[3] = {i, j, k};
     const long long os[3] = {1, u.sy, u.sz};
     const long long o = u.at(i, j, k);
+#pragma unroll
     for (int p = 0; p < 3; ++p) {
         const double* up = u.p + o + p * u.sc;
+#pragma unroll
         for (int d = 0; d < 3; ++d) {
             const long long s = os[d];
-            if (ci[d] == g.dlo[d]) gu[p][d] = (up[s] - up[0]) * K.id[d];
+            if (inside) gu[p][d] = (up[s] - up[-s]) * K.h[d];
+            else if (ci[d] == g.dlo[d]) gu[p][d] = (up[s] - up[0]) * K.id[d];
             else if (ci[d] == g.dhi[d]) gu[p][d] = (up[0] - up[-s]) * K.id[d];
             else gu[p][d] = (up[s] - up[-s]) * K.h[d];
         }
     }
 }
-__global__ void __launch_bounds__(kBlock) k_strain(Geo g, SCoef<double> K, Reg reg, View<const double> u,
+// valid nodes, those off the domain's boundary apart
+inline Parts post_parts(const Geo& g) {
+    Box3 in = geo_domain(g);
+    for (int q = 0; q < 3; ++q) { in.lo[q] += 1; in.hi[q] -= 1; }
+    return make_parts(box_isect(geo_valid(g), geo_domain(g)), in);
+}
+__global__ void __launch_bounds__(kBlock) k_strain(Geo g, SCoef<double> K, Parts parts, View<const double> u,
                                                    View<double> e, int voigt) {
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= reg.n) return;
+    const bool inside = blockIdx.x < parts.in_blocks;
     int i, j, k;
-    reg_ijk(reg, t, i, j, k);
+    if (!parts_ijk(parts, inside, i, j, k)) return;
     double gu[3][3];
-    grad_at(g, K, u, i, j, k, gu);
+    if (inside) grad_at(g, K, u, i, j, k, gu, true);
+    else grad_at(g, K, u, i, j, k, gu);
     double s[3][3];
     for (int a = 0; a < 3; ++a)
         for (int b = 0; b < 3; ++b) s[a][b] = 0.5 * (gu[a][b] + gu[b][a]);
@@ -255,30 +265,40 @@ __global__ void __launch_bounds__(kBlock) k_strain(Geo g, SCoef<double> K, Reg r
             for (int b = 0; b < 3; ++b) e.p[o + (3 * a + b) * e.sc] = s[a][b];
     }
 }
+// Bound by FP64 operations (57 for a cubic stress, 6 more for the energy).  129^3 cubic nodes: 0.377 ms
+// either, now 0.245: interior blocks without the boundary's selections, and the energy
+// W(grad u) + sum 1/2 sigma : eps as sigma : grad u where sigma is symmetric.
 template <int M>
-__global__ void __launch_bounds__(kBlock) k_stress(Geo g, SCoef<double> K, Reg reg, View<const double> C,
+__global__ void __launch_bounds__(kBlock) k_stress(Geo g, SCoef<double> K, Parts parts, View<const double> C,
                                                    View<const double> u, View<double> sg, int voigt, int energy) {
     constexpr int NC = NCoef<M>::value;
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= reg.n) return;
+    const bool inside = blockIdx.x < parts.in_blocks;
     int i, j, k;
-    reg_ijk(reg, t, i, j, k);
+    if (!parts_ijk(parts, inside, i, j, k)) return;
     double gu[3][3], s[3][3], a[NC];
-    grad_at(g, K, u, i, j, k, gu);
+    if (inside) grad_at(g, K, u, i, j, k, gu, true);
+    else grad_at(g, K, u, i, j, k, gu);
     const long long cc = C.at(i, j, k);
+#pragma unroll
     for (int q = 0; q < NC; ++q) a[q] = C.p[cc + q * C.sc];
     stress_of<M, double>(a, gu, s);
     const long long o = sg.at(i, j, k);
     if (energy) {
         // W(gradu) = trace(0.5 gradu^T (C gradu)), then += sum 0.5 sig:eps (Elastic.cpp:557-569)
-        double w = 0.0;
-        for (int ii = 0; ii < 3; ++ii) {
-            double tt = 0.0;
-            for (int jj = 0; jj < 3; ++jj) tt += gu[jj][ii] * s[jj][ii];
-            w += 0.5 * tt;
+        double w;
+        if (M == DIAG) {
+            w = 0.0;
+            for (int ii = 0; ii < 3; ++ii) {
+                double tt = 0.0;
+                for (int jj = 0; jj < 3; ++jj) tt += gu[jj][ii] * s[jj][ii];
+                w += 0.5 * tt;
+            }
+            for (int m = 0; m < 3; ++m)
+                for (int n = 0; n < 3; ++n) w += .5 * s[m][n] * (.5 * (gu[m][n] + gu[n][m]));
+        } else {
+            w = s[0][0] * gu[0][0] + s[1][1] * gu[1][1] + s[2][2] * gu[2][2] + s[0][1] * (gu[0][1] + gu[1][0]) +
+                s[0][2] * (gu[0][2] + gu[2][0]) + s[1][2] * (gu[1][2] + gu[2][1]);
         }
-        for (int m = 0; m < 3; ++m)
-            for (int n = 0; n < 3; ++n) w += .5 * s[m][n] * (.5 * (gu[m][n] + gu[n][m]));
         sg.p[o] = w;
     } else if (voigt) {
         const double v[6] = {s[0][0], s[1][1], s[2][2], s[1][2], s[2][0], s[0][1]};
@@ -289,29 +309,28 @@ __global__ void __launch_bounds__(kBlock) k_stress(Geo g, SCoef<double> K, Reg r
     }
 }
 void launch_strain(const Geo& g, View<const double> u, View<double> e, int voigt, cudaStream_t st) {
-    const Reg reg = make_reg(box_isect(geo_valid(g), geo_domain(g)));
-    if (reg.n == 0) return;
-    k_strain<<<nblocks(reg.n), kBlock, 0, st>>>(g, make_scoef<double>(g), reg, u, e, voigt);
+    const Parts parts = post_parts(g);
+    const unsigned nb = parts_blocks(parts);
+    if (nb == 0) return;
+    k_strain<<<nb, kBlock, 0, st>>>(g, make_scoef<double>(g), parts, u, e, voigt);
+    launched();
+}
+static void launch_stress_energy(const OpParams& P, View<const double> C, View<const double> u, View<double> s, int voigt,
+                                 int energy, cudaStream_t st) {
+    const Parts parts = post_parts(P.g);
+    const unsigned nb = parts_blocks(parts);
+    if (nb == 0) return;
+    dispatch_model<double>(P.model, [&](auto m) {
+        k_stress<decltype(m)::value><<<nb, kBlock, 0, st>>>(P.g, make_scoef<double>(P.g), parts, C, u, s, voigt, energy);
+    });
     launched();
 }
 void launch_stress(const OpParams& P, View<const double> C, View<const double> u, View<double> s, int voigt,
                    cudaStream_t st) {
-    const Reg reg = make_reg(box_isect(geo_valid(P.g), geo_domain(P.g)));
-    if (reg.n == 0) return;
-    dispatch_model<double>(P.model, [&](auto m) {
-        k_stress<decltype(m)::value><<<nblocks(reg.n), kBlock, 0, st>>>(P.g, make_scoef<double>(P.g), reg, C, u, s,
-                                                                        voigt, 0);
-    });
-    launched();
+    launch_stress_energy(P, C, u, s, voigt, 0, st);
 }
 void launch_energy(const OpParams& P, View<const double> C, View<const double> u, View<double> w, cudaStream_t st) {
-    const Reg reg = make_reg(box_isect(geo_valid(P.g), geo_domain(P.g)));
-    if (reg.n == 0) return;
-    dispatch_model<double>(P.model, [&](auto m) {
-        k_stress<decltype(m)::value><<<nblocks(reg.n), kBlock, 0, st>>>(P.g, make_scoef<double>(P.g), reg, C, u, w,
-                                                                        0, 1);
-    });
-    launched();
+    launch_stress_energy(P, C, u, w, 0, 1, st);
 }
 
 // ------------------------------------------------------------------ Solver::Nonlocal::Newton<T>
