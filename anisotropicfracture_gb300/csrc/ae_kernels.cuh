@@ -49,7 +49,9 @@ __device__ __forceinline__ void reg_ijk(const Reg& r, unsigned t, int& i, int& j
 // first and the slabs in further blocks of the same launch: a warp that mixes a boundary row's one-sided
 // gradient and stress with interior rows pays for both, and with rows of 65 nodes nearly every warp did
 // (in FP64 about 70 operations on top of 100).  65^3 isotropic solve, all levels: Jacobi 28.6 -> 21.1 us a
-// sweep, residual 27.8 -> 20.3; 97 x 81 x 113 cubic Jacobi 470 -> 407; FP32 unchanged (129^3 Fapply 97).
+// sweep, residual 27.8 -> 20.3; 97 x 81 x 113 cubic Jacobi 470 -> 407.  In FP32 the operations
+// do not bound: 129^3 cubic Fapply 97.7 -> 94.9, but the coarse levels' Jacobi 25.7 -> 27.5 and residual 25.9 ->
+// 26.5 us, so those two keep all their nodes in one part there.
 struct Parts {
     Reg in;               // n == 0: none
     Reg slab[6];
@@ -86,6 +88,12 @@ inline Parts make_parts(const Box3& r, Box3 inside) {
     }
     P.in_blocks = (P.in.n + kBlock - 1) / kBlock;
     return P;
+}
+// the inside for the FP64 Jacobi sweep and residual; empty in FP32
+template <class R>
+inline Box3 parts_inside(const Geo& g) {
+    if (sizeof(R) == 8) return geo_interior(g);
+    return Box3{{1, 1, 1}, {0, 0, 0}};
 }
 inline unsigned parts_blocks(const Parts& P) { return P.in_blocks + (P.end[5] + kBlock - 1) / kBlock; }
 // this thread's node; false: none.  The whole block is inside or outside.
@@ -203,7 +211,7 @@ __global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_residual(
                                                                                  View<const R> x, View<const R> b,
                                                                                  View<R> r, unsigned long long* norm,
                                                                                  View<float> r32) {
-    const bool inside = blockIdx.x < parts.in_blocks;
+    const bool inside = sizeof(R) == 8 && blockIdx.x < parts.in_blocks;
     double mx = 0.0;
     int i, j, k;
     if (parts_ijk(parts, inside, i, j, k)) {
@@ -266,8 +274,9 @@ __device__ __forceinline__ void jacobi_node(const OpParams& P, const SCoef<R>& K
     const long long isc = SAME ? xsc : invD.sc, bsc = SAME ? xsc : b.sc;
 #pragma unroll
     for (int n = 0; n < 3; ++n)
-        xo.p[oo + n * osc] = jacobi_update<R>(xi.p[ox + n * xsc], row_residual(b.p[ob + n * bsc], sc, v[n]),
-                                              invD.p[od + n * isc], omega);
+        v[n] = jacobi_update<R>(xi.p[ox + n * xsc], row_residual(b.p[ob + n * bsc], sc, v[n]), invD.p[od + n * isc], omega);
+#pragma unroll
+    for (int n = 0; n < 3; ++n) xo.p[oo + n * osc] = v[n];
 }
 
 // The first sweep of a smoother call whose correction starts at zero (the pre-smoothing of a
@@ -291,10 +300,12 @@ __global__ void __launch_bounds__(kBlock) k_jacobi_zero(Geo g, Reg reg, View<con
         return;
     }
     const long long od = invD.at(i, j, k), ob = b.at(i, j, k);
+    R v[3];
 #pragma unroll
     for (int n = 0; n < 3; ++n)
-        xo.p[oo + n * xo.sc] = jacobi_update<R>(zero, row_residual(b.p[ob + n * b.sc], R(1), zero),
-                                                invD.p[od + n * invD.sc], omega);
+        v[n] = jacobi_update<R>(zero, row_residual(b.p[ob + n * b.sc], R(1), zero), invD.p[od + n * invD.sc], omega);
+#pragma unroll
+    for (int n = 0; n < 3; ++n) xo.p[oo + n * xo.sc] = v[n];
 }
 
 template <int M, class R, bool GR, bool SAME>
@@ -303,7 +314,7 @@ __global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_jacobi(Op
                                                                                View<const R> invD,
                                                                                View<const R> xi, View<const R> b,
                                                                                View<R> xo, R omega) {
-    const bool inside = blockIdx.x < parts.in_blocks;
+    const bool inside = sizeof(R) == 8 && blockIdx.x < parts.in_blocks;
     int i, j, k;
     if (!parts_ijk(parts, inside, i, j, k)) return;
     if (inside) jacobi_node<M, R, GR, SAME, true>(P, K, C, G, invD, xi, b, xo, omega, i, j, k);
@@ -670,9 +681,14 @@ __device__ __forceinline__ T interp_at(const View<const R>& crse, int i, int j, 
 // a, b, c in {0, 1}, that lie in the fine region fr.  The parity of each of those nodes is known
 // at compile time, so a warp runs no divergent branches and the coarse values are loaded once
 // for the 8 nodes.  Each node's value is the expression of interp_at for its parity.
-template <class R>
-__global__ void __launch_bounds__(kBlock) k_interp_add8(Reg cb, Box3 fr, int ncomp, View<R> fine,
-                                                        View<const R> crse) {
+// Bound by the fine level's traffic: all 16 values are loaded before any is stored, a component per
+// blockIdx.y.  FP32 F-cycles of 257^3 nodes, all levels: 57 -> 26 us a call.
+template <class T>
+struct alignas(2 * sizeof(T)) Vec2 {
+    T v[2];
+};
+template <class R, bool VEC>
+__global__ void __launch_bounds__(kBlock) k_interp_add8(Reg cb, Box3 fr, View<R> fine, View<const R> crse) {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= cb.n) return;
     int I, J, Kc;
@@ -680,21 +696,60 @@ __global__ void __launch_bounds__(kBlock) k_interp_add8(Reg cb, Box3 fr, int nco
     const long long sy = crse.sy, sz = crse.sz;
     const bool x1 = 2 * I + 1 <= fr.hi[0], y1 = 2 * J + 1 <= fr.hi[1], z1 = 2 * Kc + 1 <= fr.hi[2];
     const bool x0 = 2 * I >= fr.lo[0], y0 = 2 * J >= fr.lo[1], z0 = 2 * Kc >= fr.lo[2];
-    for (int n = 0; n < ncomp; ++n) {
-        const R* __restrict__ c = crse.p + crse.at(I, J, Kc) + n * crse.sc;
-        R* __restrict__ f = fine.p + fine.at(2 * I, 2 * J, 2 * Kc) + n * fine.sc;
-        const long long fy = fine.sy, fz = fine.sz;
-        // (a, b, c) = (0, 0, 0): the coincident node
-        if (x0 && y0 && z0) f[0] += c[0];
-        if (x1 && y0 && z0) f[1] += R(0.5) * (c[0] + c[1]);
-        if (x0 && y1 && z0) f[fy] += R(0.5) * (c[0] + c[sy]);
-        if (x0 && y0 && z1) f[fz] += R(0.5) * (c[0] + c[sz]);
-        if (x0 && y1 && z1) f[fy + fz] += R(0.25) * (c[0] + c[sy] + c[sz] + c[sy + sz]);
-        if (x1 && y0 && z1) f[1 + fz] += R(0.25) * (c[0] + c[sz] + c[1] + c[1 + sz]);
-        if (x1 && y1 && z0) f[1 + fy] += R(0.25) * (c[0] + c[1] + c[sy] + c[1 + sy]);
-        if (x1 && y1 && z1)
-            f[1 + fy + fz] +=
-                R(0.125) * (c[0] + c[1] + c[sy] + c[sz] + c[sy + sz] + c[1 + sz] + c[1 + sy] + c[1 + sy + sz]);
+    const int n = blockIdx.y;
+    const R* __restrict__ c = crse.p + crse.at(I, J, Kc) + n * crse.sc;
+    R* __restrict__ f = fine.p + fine.at(2 * I, 2 * J, 2 * Kc) + n * fine.sc;
+    // coarse corner and fine node (a, b, c), when that fine node is in the region (a corner is one of a
+    // node that needs it); VEC: the fine pair along x is one aligned access when both are
+    R cv[8], fv[8];
+    const bool pair = VEC && x0 && x1;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int a = q & 1, bq = (q >> 1) & 1, d = q >> 2;
+        const bool need = (!a || x1) && (!bq || y1) && (!d || z1);
+        cv[q] = need ? c[a + bq * sy + d * sz] : R(0);
+    }
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const int bq = h & 1, d = h >> 1;
+        const bool row = (bq ? y1 : y0) && (d ? z1 : z0);
+        R* fr_ = f + bq * fine.sy + d * fine.sz;
+        fv[2 * h] = fv[2 * h + 1] = R(0);
+        if (row) {
+            if (pair) {
+                const Vec2<R> w = *reinterpret_cast<const Vec2<R>*>(fr_);
+                fv[2 * h] = w.v[0];
+                fv[2 * h + 1] = w.v[1];
+            } else {
+                if (x0) fv[2 * h] = fr_[0];
+                if (x1) fv[2 * h + 1] = fr_[1];
+            }
+        }
+    }
+    fv[0] += cv[0];
+    fv[1] += R(0.5) * (cv[0] + cv[1]);
+    fv[2] += R(0.5) * (cv[0] + cv[2]);
+    fv[4] += R(0.5) * (cv[0] + cv[4]);
+    fv[6] += R(0.25) * (cv[0] + cv[2] + cv[4] + cv[6]);
+    fv[5] += R(0.25) * (cv[0] + cv[4] + cv[1] + cv[5]);
+    fv[3] += R(0.25) * (cv[0] + cv[1] + cv[2] + cv[3]);
+    fv[7] += R(0.125) * (cv[0] + cv[1] + cv[2] + cv[4] + cv[6] + cv[5] + cv[3] + cv[7]);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const int bq = h & 1, d = h >> 1;
+        const bool row = (bq ? y1 : y0) && (d ? z1 : z0);
+        R* fr_ = f + bq * fine.sy + d * fine.sz;
+        if (row) {
+            if (pair) {
+                Vec2<R> w;
+                w.v[0] = fv[2 * h];
+                w.v[1] = fv[2 * h + 1];
+                *reinterpret_cast<Vec2<R>*>(fr_) = w;
+            } else {
+                if (x0) fr_[0] = fv[2 * h];
+                if (x1) fr_[1] = fv[2 * h + 1];
+            }
+        }
     }
 }
 
@@ -710,14 +765,46 @@ __global__ void __launch_bounds__(kBlock) k_inject(Reg reg, int ncomp, View<R> c
 }
 
 // ------------------------------------------------------------------ elementwise
-template <class Ro, class Ri>
+// Copies and updates are bound by bytes in flight: a thread takes U nodes and loads them all before it
+// stores any (the compiler may not, since the views could overlap).  193 x 161 x 225 nodes of three
+// FP32 components between a field and a level array: 55 -> 31 us.
+template <class Ro, class Ri, int U>
 __global__ void __launch_bounds__(kBlock) k_copy(Reg reg, int ncomp, View<Ro> dst, View<const Ri> src) {
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= reg.n) return;
-    int i, j, k;
-    reg_ijk(reg, t, i, j, k);
-    const long long od = dst.at(i, j, k), os = src.at(i, j, k);
-    for (int n = 0; n < ncomp; ++n) dst.p[od + n * dst.sc] = (Ro)src.p[os + n * src.sc];
+    const unsigned t0 = blockIdx.x * (blockDim.x * U) + threadIdx.x;
+    long long od[U], os[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+        const unsigned t = t0 + q * blockDim.x;
+        if (t >= reg.n) break;
+        int i, j, k;
+        reg_ijk(reg, t, i, j, k);
+        od[q] = dst.at(i, j, k);
+        os[q] = src.at(i, j, k);
+    }
+    int n = 0;
+    for (; n + 3 <= ncomp; n += 3) {
+        Ri v[U][3];
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (t0 + q * blockDim.x < reg.n)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) v[q][c] = src.p[os[q] + (n + c) * src.sc];
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (t0 + q * blockDim.x < reg.n)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) dst.p[od[q] + (n + c) * dst.sc] = (Ro)v[q][c];
+    }
+    for (; n < ncomp; ++n)
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (t0 + q * blockDim.x < reg.n) dst.p[od[q] + n * dst.sc] = (Ro)src.p[os[q] + n * src.sc];
+}
+// nodes a thread of k_copy takes: four once that still gives every SM of 152 its eight blocks
+template <class F>
+inline void dispatch_copy(unsigned n, F&& f) {
+    if (n >= 152u * 8u * kBlock * 4u) f(std::integral_constant<int, 4>());
+    else f(std::integral_constant<int, 1>());
 }
 template <class Ro, class Ri>
 __global__ void __launch_bounds__(kBlock) k_axpy(Reg reg, int ncomp, View<Ro> dst, double alpha, View<const Ri> src) {
@@ -741,10 +828,24 @@ __global__ void __launch_bounds__(kBlock) k_fill(Reg reg, int ncomp, View<R> dst
 // common case: level-wide vectors): the components are one contiguous run of n values, so a
 // grid-stride loop streams it with no index arithmetic.  ADD: alpha == 1, where the general form
 // dst + (Ro)(1.0 * (double)src) is exactly dst + (Ro)src (no FP64 multiply).
+// Four elements a thread and turn, as 16-byte accesses (the launcher checks that both runs begin on a
+// 16-byte boundary; the remainder of the run, or a run that does not, goes element by element).
+template <class T>
+struct alignas(16) Vec4 {
+    T v[4];
+};
 template <class Ro, class Ri>
-__global__ void __launch_bounds__(kBlock) k_flat_copy(long long n, Ro* __restrict__ dst, const Ri* __restrict__ src) {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-        dst[t] = (Ro)src[t];
+__global__ void __launch_bounds__(kBlock) k_flat_copy(long long n, bool vec, Ro* __restrict__ dst, const Ri* __restrict__ src) {
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+    const long long n4 = vec ? n / 4 : 0;
+    for (long long t = t0; t < n4; t += nt) {
+        const Vec4<Ri> s = reinterpret_cast<const Vec4<Ri>*>(src)[t];
+        Vec4<Ro> d;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) d.v[q] = (Ro)s.v[q];
+        reinterpret_cast<Vec4<Ro>*>(dst)[t] = d;
+    }
+    for (long long t = 4 * n4 + t0; t < n; t += nt) dst[t] = (Ro)src[t];
 }
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_flat_fill(long long n, R* __restrict__ dst, R value) {
@@ -752,13 +853,21 @@ __global__ void __launch_bounds__(kBlock) k_flat_fill(long long n, R* __restrict
         dst[t] = value;
 }
 template <class Ro, class Ri, bool ADD>
-__global__ void __launch_bounds__(kBlock) k_flat_axpy(long long n, Ro* __restrict__ dst, double alpha,
+__global__ void __launch_bounds__(kBlock) k_flat_axpy(long long n, bool vec, Ro* __restrict__ dst, double alpha,
                                                       const Ri* __restrict__ src) {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        if (ADD) dst[t] += (Ro)src[t];
-        else dst[t] += (Ro)(alpha * (double)src[t]);
+    const auto sum = [&](Ro d, Ri s) { return d + (ADD ? (Ro)s : (Ro)(alpha * (double)s)); };
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+    const long long n4 = vec ? n / 4 : 0;
+    for (long long t = t0; t < n4; t += nt) {
+        const Vec4<Ri> s = reinterpret_cast<const Vec4<Ri>*>(src)[t];
+        Vec4<Ro> d = reinterpret_cast<const Vec4<Ro>*>(dst)[t];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) d.v[q] = sum(d.v[q], s.v[q]);
+        reinterpret_cast<Vec4<Ro>*>(dst)[t] = d;
     }
+    for (long long t = 4 * n4 + t0; t < n; t += nt) dst[t] = sum(dst[t], src[t]);
 }
+inline bool vec4_aligned(const void* a, const void* b) { return (((uintptr_t)a | (uintptr_t)b) & 15) == 0; }
 // true when region, taken over ncomp components, covers whole rows and planes of v's storage
 // from its first node, so that the elements from there on form one contiguous run (row padding
 // included: padding is never read by the stencil kernels, and the level arrays hold it)

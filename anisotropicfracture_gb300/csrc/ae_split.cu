@@ -71,7 +71,7 @@ struct TL {
     static constexpr int kSlot = oG + VP * 4;
     static constexpr int oBar = SRING * kSlot;
     static constexpr int oQ = up128(oBar + 16 * SRING + 8);  // the ring's barriers and the table's
-    static constexpr int kQ = QCAP * (QN * E + 4);  // bytes per warp queue
+    static constexpr int kQ = QCAP * (QN * E + 8);  // bytes per warp queue
     static constexpr int oT = up128(oQ + STY * kQ);
     static constexpr unsigned kX = 3 * XP * E, kV = 3 * VP * E, kG = VP * 4;
     static_assert(oB % 128 == 0 && oI % 128 == 0 && oG % 128 == 0 && kSlot % 128 == 0, "TMA destinations");
@@ -237,8 +237,8 @@ __global__ void __launch_bounds__(kTileThreads, 1)
                  const __grid_constant__ CUtensorMap tm_i, const __grid_constant__ CUtensorMap tm_g, SCoef<double> K, TileGeo T,
                  int uniform, int sy, int sz, int sc, const unsigned* __restrict__ gidm,
                  const double* __restrict__ tab, const double* __restrict__ rows, int rows_bytes, int tab_bytes,
-                 const double* __restrict__ x, const double* b, const double* __restrict__ invD, double* out, double omega,
-                 int* err) {
+                 const double* __restrict__ x, const double* b, const double* __restrict__ invD, double* out, int osy, int osz,
+                 int osc, double omega, int* err) {
     using R = double;
     using L = TL<R>;
     constexpr int NC = NCoef<M>::value, TS = row_stride<M>();
@@ -299,6 +299,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     const int i = T.slo[0] + c0 + lane, j = j0 + warp;
     const bool act = i >= T.I.lo[0] && i <= T.I.hi[0] && j <= T.I.hi[1];
     int o = c0 + lane + (j - T.slo[1]) * sy + (k0 - T.slo[2] - 2) * sz;  // node (i, j) of the plane computed
+    int oo = c0 + lane + (j - T.slo[1]) * osy + (k0 - T.slo[2] - 2) * osz;  // ... in the output
     // the grains' stiffness: beside the rows in shared memory, or global
     const R* gt = TABS && tab_bytes ? reinterpret_cast<const R*>(smem + L::oT + rows_bytes) : tab;
     // F plus the grad C term of a node at offset on: gu its central differences, gp and gm the grains of
@@ -325,14 +326,14 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         return mul_rn(K.i2[0], F);
     };
     R* qv = reinterpret_cast<R*>(smem + L::oQ + warp * L::kQ);  // [QN][QCAP]
-    int* qo = reinterpret_cast<int*>(qv + QN * QCAP);
+    int* qo = reinterpret_cast<int*>(qv + QN * QCAP);  // the node, and its place in the output
     int qhead = 0, qcnt = 0;
     // the first cnt (at most 32) nodes of the queue
     const auto work_off = [&](int cnt) {
         __syncwarp();
         if (lane < cnt) {
             const int e = (qhead + lane) & (QCAP - 1);
-            const int on = qo[e];
+            const int on = qo[e], ow = qo[QCAP + e];
             const int step[3] = {1, sy, sz};
             unsigned gp[3], gm[3];
             R xc[3], bc[3], ic[3], gu[3][3], F[3];
@@ -354,7 +355,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
             }
             with_gradc(mask, gp, gm, gu, F);
 #pragma unroll
-            for (int r = 0; r < 3; ++r) out[on + r * sc] = value(xc[r], bc[r], ic[r], F[r]);
+            for (int r = 0; r < 3; ++r) out[ow + r * osc] = value(xc[r], bc[r], ic[r], F[r]);
         }
         __syncwarp();
         qhead = (qhead + cnt) & (QCAP - 1);
@@ -379,6 +380,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         if (wide) {
             e = (qhead + qcnt + __popc(ball & ((1u << lane) - 1u))) & (QCAP - 1);
             qo[e] = o;
+            qo[QCAP + e] = oo;
         }
         qcnt += __popc(ball);
         const R* tr = TABS ? ts + (int)(gw & 0xffffu) * TS : tab;
@@ -427,7 +429,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
                 const R bc = OP != SPLIT_FAPPLY ? vb[r * L::VP] : R(0), ic = OP == SPLIT_JACOBI ? vi[r * L::VP] : R(0);
-                out[o + r * sc] = value(mid.c[r], bc, ic, F[r]);
+                out[oo + r * osc] = value(mid.c[r], bc, ic, F[r]);
             }
         }
     };
@@ -439,7 +441,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     bool failed = TABS && !__all_sync(0xffffffffu, mbar_wait(tbar, 0));
     int s = 0;
     unsigned phase = 0;
-    for (int t = 0; !failed && t < planes; ++t, o += sz) {  // x plane k0 - 1 + t
+    for (int t = 0; !failed && t < planes; ++t, o += sz, oo += osz) {  // x plane k0 - 1 + t
         failed = !__all_sync(0xffffffffu, mbar_wait(full(s), phase));
         if (failed) break;
         const unsigned char* base = smem + s * L::kSlot;
@@ -494,7 +496,7 @@ __global__ void __launch_bounds__(SNT / 2, AE_SPLIT_PAIR_BLOCKS)
                  const __grid_constant__ CUtensorMap tm_i, const __grid_constant__ CUtensorMap tm_g,
                    SCoef<float> K, TileGeo T, int sh, int uniform, long long sy, long long sz, long long sc,
                    const unsigned* __restrict__ gidm_g, const float* __restrict__ tab, int tab_n, float* __restrict__ xo,
-                   float omega, int* err) {
+                   long long osy, long long osz, long long osc, float omega, int* err) {
     using R = float;
     constexpr int NPT = 2, NT = SNT / NPT;  // rows per thread, threads per block
     using L = TL32;
@@ -559,10 +561,11 @@ __global__ void __launch_bounds__(SNT / 2, AE_SPLIT_PAIR_BLOCKS)
     const int col = sh + 1 + tx;
     const int cx = (ty + 1) * T32B + col;  // this node inside an x component tile
     const int cv = ty * T32B + col;        // ... inside a b / 1/D / id component tile
-    long long o = (long long)(i - T.slo[0]) + (long long)(j - T.slo[1]) * sy + (long long)(k0 - T.slo[2]) * sz;
+    // node (i, j, k) in the output
+    long long o = (long long)(i - T.slo[0]) + (long long)(j - T.slo[1]) * osy + (long long)(k0 - T.slo[2]) * osz;
     bool failed = false;
     int last = 0;  // last stage issued
-    for (int k = k0; k <= k1; ++k, o += sz) {
+    for (int k = k0; k <= k1; ++k, o += osz) {
         const int s = k - k0;
         // stage s + 1: plane k + 2 of x and the tiles of plane k + 1; their ring slots were last
         // read in iteration k - 1, which the barrier at its end closed
@@ -685,16 +688,16 @@ __global__ void __launch_bounds__(SNT / 2, AE_SPLIT_PAIR_BLOCKS)
                 }
             }
             if (an && !queued[n]) {
-                const long long on = o + n * sy;
+                const long long on = o + n * osy;
                 const int vn = n * T32B;
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
                     if (OP == SPLIT_JACOBI)
-                        xo[on + r * sc] = jacobi_update<R>(xv[n][r], sub_rn(bv[vn + r * T32V], f[n][r]), iv[vn + r * T32V], omega);
+                        xo[on + r * osc] = jacobi_update<R>(xv[n][r], sub_rn(bv[vn + r * T32V], f[n][r]), iv[vn + r * T32V], omega);
                     else if (OP == SPLIT_RESIDUAL)
-                        xo[on + r * sc] = bv[vn + r * T32V] - f[n][r];
+                        xo[on + r * osc] = bv[vn + r * T32V] - f[n][r];
                     else
-                        xo[on + r * sc] = f[n][r];
+                        xo[on + r * osc] = f[n][r];
                 }
             }
         }
@@ -705,7 +708,8 @@ __global__ void __launch_bounds__(SNT / 2, AE_SPLIT_PAIR_BLOCKS)
             const int t = qtid[e];
             const int qx = t % STX, qy = t / STX;
             const int qcx = (qy + 1) * T32B + sh + 1 + qx, qcv = qy * T32B + sh + 1 + qx;
-            const long long qo = o + (long long)(qx - tx) + (long long)(qy - ty) * sy;
+            const long long qo = (long long)(i0 + qx - T.slo[0]) + (long long)(j0 + qy - T.slo[1]) * sy + (long long)(k - T.slo[2]) * sz;
+            const long long ow = o + (long long)(qx - tx) + (long long)(qy - ty) * osy;
             const R* qm = xslot(k - 1) + qcx;
             const R* qc = xslot(k) + qcx;
             const R* qp = xslot(k + 1) + qcx;
@@ -742,11 +746,11 @@ __global__ void __launch_bounds__(SNT / 2, AE_SPLIT_PAIR_BLOCKS)
                 R fr = qf[3 * e + r];
                 fr = gradc_add(fr, colv[0][r], colv[1][r], colv[2][r], K.h);
                 if (OP == SPLIT_JACOBI)
-                    xo[qo + r * sc] = jacobi_update<R>(qc[r * T32X], sub_rn(qb[r * T32V], fr), qi[r * T32V], omega);
+                    xo[ow + r * osc] = jacobi_update<R>(qc[r * T32X], sub_rn(qb[r * T32V], fr), qi[r * T32V], omega);
                 else if (OP == SPLIT_RESIDUAL)
-                    xo[qo + r * sc] = qb[r * T32V] - fr;
+                    xo[ow + r * osc] = qb[r * T32V] - fr;
                 else
-                    xo[qo + r * sc] = fr;
+                    xo[ow + r * osc] = fr;
             }
         }
         __syncthreads();
@@ -800,8 +804,9 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 4 : 2)
     R v[3];
     const long long ox = x.at(i, j, k);
     const R sc = apply_at<M, R, true>(P, K, C, G, x, i, j, k, ox, ox, v);
+    const long long of = f.at(i, j, k);
 #pragma unroll
-    for (int q = 0; q < 3; ++q) f.p[ox + q * x.sc] = mul_rn(sc, v[q]);
+    for (int q = 0; q < 3; ++q) f.p[of + q * f.sc] = mul_rn(sc, v[q]);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda)
@@ -871,10 +876,11 @@ int tile_kz(long long tiles, int nz, long long wave) {
 // the tiled kernel of one operation over I; b: the right-hand side, invD: 1/D (Jacobi only)
 template <class R, int OP>
 void launch_tile(const OpParams& P, const SplitList& sl, const Box3& I, const Box3& S, View<const R> x, const R* b,
-                 const R* invD, R* out, R omega, cudaStream_t st, Grains<R> G, int ngrains, int* err) {
+                 const R* invD, View<R> out, R omega, cudaStream_t st, Grains<R> G, int ngrains, int* err) {
     constexpr int E = (int)sizeof(R);
     constexpr bool F32 = E == 4;
     const SCoef<R> K = make_scoef<R>(P.g);
+    R* const po = out.p + out.at(S.lo[0], S.lo[1], S.lo[2]);
     const CUtensorMapDataType dt = F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
     dispatch_model<R>(P.model, [&](auto m) {
         constexpr int Mv = decltype(m)::value;
@@ -905,12 +911,13 @@ void launch_tile(const OpParams& P, const SplitList& sl, const Box3& I, const Bo
                 // boxes' first column is then a multiple of 4
                 const int sh = (I.lo[0] - 1 - S.lo[0]) & 3;
                 k_sweep_tile32<Mv, TABS, OP><<<grid, SNT / 2, TL32::oT + (TABS ? pad_bytes : 0), st>>>(
-                    tx, tb, ti, tg, K, T, sh, P.uniform, x.sy, x.sz, x.sc, sl.gidm, G.tab, ngrains * NCoef<Mv>::value, out, omega,
-                    err);
+                    tx, tb, ti, tg, K, T, sh, P.uniform, x.sy, x.sz, x.sc, sl.gidm, G.tab, ngrains * NCoef<Mv>::value, po,
+                    out.sy, out.sz, out.sc, omega, err);
             } else {
                 k_sweep_tile64<Mv, TABS, OP><<<grid, kTileThreads, TL<double>::oT + (TABS ? rows_bytes + tab_bytes : 0), st>>>(
                     tx, tb, ti, tg, K, T, P.uniform, (int)x.sy, (int)x.sz, (int)x.sc, sl.gidm, G.tab, sl.rows64,
-                    TABS ? (int)rows_bytes : 0, TABS ? (int)tab_bytes : 0, x.p, b, invD, out, omega, err);
+                    TABS ? (int)rows_bytes : 0, TABS ? (int)tab_bytes : 0, x.p, b, invD, po, (int)out.sy,
+                    (int)out.sz, (int)out.sc, omega, err);
             }
             launched();
         };
@@ -989,16 +996,17 @@ void launch_jacobi_split(const OpParams& P, const SplitList& sl, View<const R> C
                          int ngrains, int* err) {
     const Box3 S = geo_store(P.g);
     const Box3 I = geo_interior(P.g);
-    const bool same = same_layout(xi, C) && same_layout(xi, invD) && same_layout(xi, b) &&
-                      same_layout(xi, xo);
-    if (!same || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
+    const bool in = same_layout(xi, C) && same_layout(xi, invD) && same_layout(xi, b), same = in && same_layout(xi, xo);
+    if (!in || !split_out(xo) || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
     if (!box_empty(I))
-        launch_tile<R, SPLIT_JACOBI>(P, sl, I, S, xi, b.p, invD.p, xo.p, omega, st, G, ngrains, err);
+        launch_tile<R, SPLIT_JACOBI>(P, sl, I, S, xi, b.p, invD.p, xo, omega, st, G, ngrains, err);
     if (sl.n > 0) {
         const SCoef<R> K = make_scoef<R>(P.g);
         dispatch_model<R>(P.model, [&](auto m) {
-            k_jacobi_list<decltype(m)::value, R, true><<<(unsigned)((sl.n + kBlock - 1) / kBlock), kBlock, 0, st>>>(
-                P, K, sl.list, sl.n, S, C, G, invD, xi, b, xo, omega);
+            constexpr int Mv = decltype(m)::value;
+            const unsigned nb = (unsigned)((sl.n + kBlock - 1) / kBlock);
+            if (same) k_jacobi_list<Mv, R, true><<<nb, kBlock, 0, st>>>(P, K, sl.list, sl.n, S, C, G, invD, xi, b, xo, omega);
+            else k_jacobi_list<Mv, R, false><<<nb, kBlock, 0, st>>>(P, K, sl.list, sl.n, S, C, G, invD, xi, b, xo, omega);
         });
         launched();
     }
@@ -1012,7 +1020,7 @@ void launch_residual_split(const OpParams& P, const SplitList& sl, View<const R>
     const bool same = same_layout(x, C) && same_layout(x, b) && same_layout(x, r);
     if (!same || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
     if (!box_empty(I))
-        launch_tile<R, SPLIT_RESIDUAL>(P, sl, I, S, x, b.p, nullptr, r.p, R(0), st, G, ngrains, err);
+        launch_tile<R, SPLIT_RESIDUAL>(P, sl, I, S, x, b.p, nullptr, r, R(0), st, G, ngrains, err);
     if (sl.n_r > 0) {
         const SCoef<R> K = make_scoef<R>(P.g);
         dispatch_model<R>(P.model, [&](auto m) {
@@ -1028,9 +1036,8 @@ void launch_fapply_split(const OpParams& P, const SplitList& sl, View<const R> C
                          cudaStream_t st, Grains<R> G, int ngrains, int* err) {
     const Box3 S = geo_store(P.g);
     const Box3 I = geo_interior(P.g);
-    const bool same = same_layout(x, C) && same_layout(x, f);
-    if (!same || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
-    if (!box_empty(I)) launch_tile<R, SPLIT_FAPPLY>(P, sl, I, S, x, (const R*)nullptr, nullptr, f.p, R(0), st, G, ngrains, err);
+    if (!same_layout(x, C) || !split_out(f) || !split_supported(P.g)) throw std::runtime_error("split sweep needs the level's internal arrays");
+    if (!box_empty(I)) launch_tile<R, SPLIT_FAPPLY>(P, sl, I, S, x, (const R*)nullptr, nullptr, f, R(0), st, G, ngrains, err);
     if (sl.n_r > 0) {
         const SCoef<R> K = make_scoef<R>(P.g);
         dispatch_model<R>(P.model, [&](auto m) {

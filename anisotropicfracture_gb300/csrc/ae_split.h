@@ -22,6 +22,11 @@ constexpr int kSplitMaxGrains = 1 << 16;
 
 // whether a level's layout allows the split sweep (row pitch a multiple of 4 nodes)
 bool split_supported(const Geo& g);
+// whether the split sweep can write a view: offsets into its three components are 32-bit
+template <class R>
+bool split_out(const View<R>& v) {
+    return 3 * v.sc < (1ll << 31);
+}
 // Build the node list and the id/mask array of a grain-map level (gid laid out like the level's
 // storage, at most kSplitMaxGrains grains) and the grains' row numbers; allocates sl's arrays with
 // cudaMalloc and returns the list's length.  scratch_count: one device counter.  Synchronises the
@@ -30,12 +35,13 @@ long long split_build(const Geo& g, int model, View<const unsigned short> gid, i
                       SplitList& sl, cudaStream_t st, unsigned long long* scratch_count);
 void split_free(SplitList& sl);
 // One damped-Jacobi sweep (FP32 or FP64) of a grain-map level: the tiled interior kernel, then the
-// list.  *err is set (device) when a TMA load of the tiled kernel did not complete.
+// list.  *err is set (device) when a TMA load of the tiled kernel did not complete.  Inputs are the
+// level's arrays; the result goes to any view over the storage box (split_out).
 template <class R>
 void launch_jacobi_split(const OpParams& P, const SplitList& sl, View<const R> C, View<const R> invD, View<const R> xi,
                          View<const R> b, View<R> xo, R omega, cudaStream_t st, Grains<R> G,
                          int ngrains, int* err);
-// f = A x on the apply region of a grain-map level, the same split (f other than x).
+// f = A x on the apply region of a grain-map level, the same split (f other than x, any view over the region).
 template <class R>
 void launch_fapply_split(const OpParams& P, const SplitList& sl, View<const R> C, View<const R> x, View<R> f,
                          cudaStream_t st, Grains<R> G, int ngrains, int* err);
