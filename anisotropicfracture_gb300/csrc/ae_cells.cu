@@ -65,7 +65,7 @@ size_t cell_layout(CellRes& c, char* base) {
         L.ngrains = 0;
         L.tab64 = nullptr;
         L.tab32 = nullptr;
-        L.dtab64 = nullptr;
+        L.rows64 = nullptr;
         L.itab64 = nullptr;
         L.itab32 = nullptr;
         for (int d = 0; d < 3; ++d) { n[d] /= 2; dx[d] *= 2.0; }
@@ -165,6 +165,7 @@ CellEngine::~CellEngine() {
     for (auto& a : tall)
         for (auto& t : a) t.release();
     tred.release();
+    tmarch.release();
     tsub.release();
     for (auto& t : tcell) t.release();
     if (dcells) cudaFree(dcells);
@@ -198,6 +199,7 @@ CellArgs CellEngine::args(const ae_solver_opts& o) const {
     A.uniform = 0;
     A.sweeps = o.sweeps;
     A.omega = o.omega;
+    A.omega32 = (float)o.omega;
     return A;
 }
 
@@ -248,9 +250,9 @@ void CellEngine::set_grains(CellRes* c, int ng, const double* seeds, const doubl
     CellLevelDev& L = c->lv[0];
     if (c->gtab) AEH_CHECK(cudaFreeAsync(c->gtab, st));
     c->gtab = nullptr;
-    // tables: stiffness FP64 and FP32, diagonal FP64, 1/diagonal FP64 and FP32
-    const size_t n64 = (size_t)ng * nc, n32 = n64;
-    const size_t bytes = align256(8 * n64) + align256(4 * n32) + 3 * align256(8 * 3 * (size_t)ng);
+    // tables: stiffness FP64 and FP32, row numbers FP64, 1/diagonal FP64 and FP32
+    const size_t n64 = (size_t)ng * nc, n32 = n64, nrow = (size_t)ng * cell_row_numbers(nc);
+    const size_t bytes = align256(8 * n64) + align256(4 * n32) + align256(8 * nrow) + 2 * align256(8 * 3 * (size_t)ng);
     void* mem = nullptr;
     AEH_CHECK(cudaMallocAsync(&mem, bytes, st));
     c->gtab = mem;
@@ -259,8 +261,8 @@ void CellEngine::set_grains(CellRes* c, int ng, const double* seeds, const doubl
     p += align256(8 * n64);
     L.tab32 = (float*)p;
     p += align256(4 * n32);
-    L.dtab64 = (double*)p;
-    p += align256(8 * 3 * (size_t)ng);
+    L.rows64 = (double*)p;
+    p += align256(8 * nrow);
     L.itab64 = (double*)p;
     p += align256(8 * 3 * (size_t)ng);
     L.itab32 = (float*)p;
@@ -283,7 +285,7 @@ void CellEngine::set_field(CellRes* c, const void* C) {
     L.ngrains = 0;
     L.tab64 = nullptr;
     L.tab32 = nullptr;
-    L.dtab64 = nullptr;
+    L.rows64 = nullptr;
     L.itab64 = nullptr;
     L.itab32 = nullptr;
     if (c->gtab) AEH_CHECK(cudaFreeAsync(c->gtab, st));
@@ -316,7 +318,7 @@ void CellEngine::rebuild() {
             hsolves.push_back(s);
         }
         maxL = std::max(maxL, r->nlev);
-        reps0 |= r->lv[0].gid ? 2 : 1;
+        reps0 |= !r->lv[0].gid ? kRepNode : cell_marches(r->lv[0]) ? kRepMarch : kRepGrains;
     }
     nsolves = (int)hsolves.size();
     if ((size_t)ncell > cap_cells || !dcells) {
@@ -362,6 +364,22 @@ void CellEngine::rebuild() {
         for (int t0 = 0; t0 < r->lv[0].nn; t0 += kRedChunk) tred.h.push_back(Work{s, t0});
     }
     tred.upload(st);
+    // marching runs: as many planes each as leave every resident block two of them, at most 8 (the two
+    // planes loaded beside those computed cost a quarter of them then)
+    long long nodes = 0;
+    for (int c = 0; c < ncell; ++c)
+        if (cell_marches(live[c]->lv[0])) nodes += (long long)live[c]->lv[0].nn * live[c]->nrhs;
+    march_kz = (int)std::max(2ll, std::min(8ll, nodes / (2ll * kMarchNodes * nsm * kMarchBlocks)));
+    tmarch.h.clear();
+    for (int c = 0; c < ncell; ++c) {
+        const CellLevelDev& L = live[c]->lv[0];
+        if (!cell_marches(L)) continue;
+        const int sz = L.n[0] * L.n[1];
+        for (int z = 0; z < L.n[2]; z += march_kz)
+            for (int c0 = 0; c0 < sz; c0 += kMarchNodes)
+                for (int k = 0; k < live[c]->nrhs; ++k) tmarch.h.push_back(Work{solve_base[c] + k, z * sz + c0});
+    }
+    tmarch.upload(st);
     for (int m = 0; m < kMaxCellLevels; ++m) {
         Table& T = tcell[m];
         T.h.clear();
@@ -457,7 +475,7 @@ void CellEngine::smooth_phase(int prec, int m, int calls, bool zero, const ae_so
     }
     int from2 = 0;
     for (int s = 0; s < total; ++s) {
-        cells_launch_smooth(model, prec, zero && s == 0, A, T.d, T.n, sh, m, from2, reps(m), st);
+        cells_launch_smooth(model, prec, zero && s == 0, A, T.d, T.n, sh, m, from2, reps(m), march(), st);
         from2 ^= 1;
     }
     if (from2) cells_launch_copy2(prec, A, T.d, T.n, sh, m, st);
@@ -467,7 +485,7 @@ void CellEngine::vcycle(int prec, const ae_solver_opts& o) {
     const CellArgs A = args(o);
     for (int m = 0; m + 1 < maxL; ++m) {
         smooth_phase(prec, m, o.nu1, true, o, A);
-        cells_launch_rescor(model, prec, A, table(m).d, table(m).n, shape(m), m, 0, reps(m), st);
+        cells_launch_rescor(model, prec, A, table(m).d, table(m).n, shape(m), m, 0, reps(m), march(), st);
         cells_launch_restrict(prec, A, table(m + 1).d, table(m + 1).n, shape(m + 1), m, st);
     }
     const KrylovParams kp{o.bottom, o.bottom_max_iter, o.bottom_reltol, o.nuf};
@@ -485,7 +503,7 @@ void CellEngine::iteration_body(int prec, const ae_solver_opts& o, double tol_re
     for (int c = 0; c < inner; ++c) {
         vcycle(prec, o);
         cells_launch_update(prec, A, tred.d, tred.n, st);
-        if (c + 1 < inner) cells_launch_rescor(model, prec, A, table(0).d, table(0).n, shape(0), 0, 1, reps0, st);
+        if (c + 1 < inner) cells_launch_rescor(model, prec, A, table(0).d, table(0).n, shape(0), 0, 1, reps0, march(), st);
     }
     cells_launch_resid_top(model, A, tred.d, tred.n, reps0, st);
     cells_launch_mean(A, nullptr, nsolves, 0, 0, st);
@@ -640,6 +658,8 @@ void CellEngine::tune(int prec, const ae_solver_opts& o) {
     const int mults[] = {0, 2, 4, 8, 16, 32};
     for (int m = 0; m + 1 < maxL; ++m) {
         if (forced[m]) continue;
+        // marching sweeps do not take the shape: time the first sweep of a cycle there
+        const bool zero = prec && reps(m) == kRepMarch;
         float best = 1e30f;
         int bc = 1, bg = 0;
         for (int ci = 0; ci < 2; ++ci) {
@@ -650,10 +670,10 @@ void CellEngine::tune(int prec, const ae_solver_opts& o) {
                 sh.chunk = ci == 0 ? 128 : 256;
                 sh.grid = mu == 0 ? T.n : std::min(T.n, nsm * mu);
                 if (mu != 0 && sh.grid == T.n) continue;
-                cells_launch_smooth(model, prec, false, A, T.d, T.n, sh, m, 0, reps(m), st);  // warm
+                cells_launch_smooth(model, prec, zero, A, T.d, T.n, sh, m, 0, reps(m), march(), st);  // warm
                 AEH_CHECK(cudaEventRecord(e0, st));
                 for (int r = 0; r < 3; ++r)
-                    cells_launch_smooth(model, prec, false, A, T.d, T.n, sh, m, 0, reps(m), st);
+                    cells_launch_smooth(model, prec, zero, A, T.d, T.n, sh, m, 0, reps(m), march(), st);
                 AEH_CHECK(cudaEventRecord(e1, st));
                 AEH_CHECK(cudaEventSynchronize(e1));
                 float ms = 0.f;

@@ -30,16 +30,18 @@ struct CellLevelDev {
     SCoef<double> K64;
     SCoef<float> K32;
     // Voronoi cells, finest level only: grain id per node and per-grain tables of the stiffness
-    // (ncoef), diagonal and 1/diagonal (3).  gid == nullptr: per-node arrays only.  The kernels of
+    // (ncoef), the FP64 row's numbers (cell_row_numbers) and 1/diagonal (3).  gid == nullptr: per-node arrays only.  The kernels of
     // the finest level read these instead of the per-node arrays (same values, far fewer bytes).
     unsigned short* gid;
     int ngrains;
     double* tab64;
     float* tab32;
-    double* dtab64;
+    double* rows64;
     double* itab64;
     float* itab32;
 };
+// numbers of an FP64 row for a model of ncoef slots (RowN)
+inline int cell_row_numbers(int ncoef) { return ncoef == 21 ? 36 : ncoef; }
 struct CellDev {
     int nlev;
     int pad_;
@@ -93,6 +95,7 @@ struct CellArgs {
     int uniform;
     int sweeps;
     double omega;
+    float omega32;
 };
 
 // launch shape of one table: nodes per entry (= threads per block) and grid size
@@ -101,17 +104,30 @@ struct Shape {
     int grid;
 };
 
+// Grain-map cells whose FP32 finest-level sweeps march (kb_grain_march): whole rows of a plane and the
+// grains' numbers fit its shared memory.
+constexpr int kMarchX = 64, kMarchGrains = 96;
+constexpr int kMarchNodes = 256, kMarchBlocks = 4;  // nodes of a plane a block takes, resident blocks per SM
+__host__ __device__ inline bool cell_marches(const CellLevelDev& L) {
+    return L.gid != nullptr && L.n[0] <= kMarchX && L.ngrains <= kMarchGrains;
+}
+// their work: entry start = first node of a run of nodes in plane z, kz planes from there on
+struct MarchTab {
+    const Work* tab;
+    int n, kz, grid;
+};
+
 // ---- launchers (ae_cells_kernels.cu); model 0 ISO, 1 MM, 2 DIAG
-// reps (stencil launchers): bit 0 runs the per-node variant, bit 1 the grain-table variant; on
-// the finest level each entry is served by the variant that matches its cell, coarser levels
-// always take the per-node variant (reps = 1).
+// reps (stencil launchers): the finest-level representations present; each entry is served by the
+// variant that matches its cell, coarser levels always take the per-node variant.
+constexpr int kRepNode = 1, kRepGrains = 2, kRepMarch = 4;
 void cells_launch_smooth(int model, int prec, bool zero, const CellArgs& A, const Work* tab, int ntab, Shape sh,
-                         int m, int from2, int reps, cudaStream_t st);
+                         int m, int from2, int reps, const MarchTab& mt, cudaStream_t st);
 void cells_launch_copy2(int prec, const CellArgs& A, const Work* tab, int ntab, Shape sh, int m, cudaStream_t st);
 void cells_launch_fill0(int prec, const CellArgs& A, const Work* tab, int ntab, Shape sh, int m, cudaStream_t st);
 // rescor_m = res_m - A cor_m (inplace: res_m -= A cor_m)
 void cells_launch_rescor(int model, int prec, const CellArgs& A, const Work* tab, int ntab, Shape sh, int m,
-                         int inplace, int reps, cudaStream_t st);
+                         int inplace, int reps, const MarchTab& mt, cudaStream_t st);
 // res_{m+1} = R rescor_m, tab over level m+1 nodes
 void cells_launch_restrict(int prec, const CellArgs& A, const Work* tab, int ntab, Shape sh, int m, cudaStream_t st);
 // cor_m += I cor_{m+1}, tab over level m nodes

@@ -59,12 +59,15 @@ struct CellEngine {
     SolveDev* dsolves = nullptr;
     size_t cap_solves = 0;
     int nsolves = 0, maxL = 0;
-    int reps0 = 1;  // finest-level representations present (bit 0 per-node, bit 1 grain tables)
-    int reps(int m) const { return m == 0 ? reps0 : 1; }
+    int reps0 = kRepNode;  // finest-level representations present
+    int reps(int m) const { return m == 0 ? reps0 : kRepNode; }
     std::vector<int> solve_base;  // first solve slot of each cell slot
     // tables: per chunk option (128, 256) and level, solves; level-0 reduction runs; cells
     Table tall[2][kMaxCellLevels];
     Table tred;
+    Table tmarch;
+    int march_kz = 1;
+    MarchTab march() const { return MarchTab{tmarch.d, tmarch.n, march_kz, nsm * kMarchBlocks}; }
     Table tcell[kMaxCellLevels];
     // launch shapes per level (chunk option index and grid); forced[m] set by the caller
     int chunk_idx[kMaxCellLevels];

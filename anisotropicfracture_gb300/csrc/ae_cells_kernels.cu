@@ -2,6 +2,8 @@
 // grid-stride loop (a persistent grid sized by the tuner); each entry is a run of `chunk`
 // consecutive nodes of one solve's level, one node per thread.  Entries of solves that are not
 // active (converged, failed, or without that level) are skipped by the whole block.
+#include <algorithm>
+#include <mutex>
 #include <type_traits>
 
 #include "ae_cell.cuh"
@@ -43,6 +45,13 @@ __device__ __forceinline__ const R* itabfield(const CellLevelDev& L) {
     else return L.itab32;
 }
 
+// (converted on the host: a conversion holds the FP64 pipe for 64 clocks a warp)
+template <class R>
+__device__ __forceinline__ R omega_of(const CellArgs& A) {
+    if constexpr (sizeof(R) == 8) return A.omega;
+    else return A.omega32;
+}
+
 // Which finest-level representation a launch serves: GR = true the grain tables (entries of
 // cells without them are skipped), GR = false the per-node arrays (on the finest level, entries
 // of cells with grain tables are skipped).  Coarser levels always use the per-node arrays.
@@ -51,11 +60,10 @@ __device__ __forceinline__ bool rep_skips(bool GR, int m, const CellLevelDev& L)
 }
 
 // f = A u at node t of level m
-template <int M, class R, bool GR>
+template <int M, class R>
 __device__ __forceinline__ void level_apply(const CellLevelDev& L, int uniform, const R* U, int t, const POff& o,
                                             R f[3]) {
-    if constexpr (GR) cell_apply_grains<M, R>(kfield<R>(L), uniform, L.gid, tabfield<R>(L), U, L.nn, t, o, f);
-    else cell_apply<M, R>(kfield<R>(L), uniform, cfield<R>(L), L.nn, U, L.nn, t, o, f);
+    cell_apply<M, R>(kfield<R>(L), uniform, cfield<R>(L), L.nn, U, L.nn, t, o, f);
 }
 
 constexpr int kCellThreads = 256;
@@ -67,6 +75,9 @@ constexpr int kCellThreads = 256;
 //     with the compiler's 118 registers.
 #ifndef AE_CELL_SMOOTH_BLOCKS
 #define AE_CELL_SMOOTH_BLOCKS 4
+#endif
+#ifndef AE_CELL_GRAIN64_BLOCKS
+#define AE_CELL_GRAIN64_BLOCKS 2
 #endif
 #ifndef AE_CELL_SMOOTH_BLOCKS_PERNODE
 #define AE_CELL_SMOOTH_BLOCKS_PERNODE 3
@@ -94,7 +105,7 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, GR>()) kb_smo
         const R* __restrict__ xin = from2 ? V.cor2 : V.cor;
         R* __restrict__ xout = from2 ? V.cor : V.cor2;
         const R* __restrict__ b = V.res;
-        const R omega = (R)A.omega;
+        const R omega = omega_of<R>(A);
         // grain tables on the finest level of a Voronoi cell, per-node arrays otherwise
         constexpr bool grains = GR;
         const int g3 = grains ? 3 * (int)__ldg(L.gid + t) : 0;
@@ -109,7 +120,7 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, GR>()) kb_smo
         cell_ijk(L.n, t, i, j, k);
         const POff o = cell_offsets(L.n, i, j, k);
         R f[3];
-        level_apply<M, R, GR>(L, A.uniform, xin, t, o, f);
+        level_apply<M, R>(L, A.uniform, xin, t, o, f);
         const R sc = row_factor(kfield<R>(L));
 #pragma unroll
         for (int p = 0; p < 3; ++p)
@@ -134,8 +145,8 @@ __global__ void __launch_bounds__(kCellThreads) kb_copy2(CellArgs A, const Work*
 }
 
 // rescor = res - A cor at level m (inplace: into res)
-template <int M, class R, bool GR>
-__global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, GR>()) kb_rescor(CellArgs A, const Work* __restrict__ tab, int ntab, int m,
+template <int M, class R>
+__global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, false>()) kb_rescor(CellArgs A, const Work* __restrict__ tab, int ntab, int m,
                                                           int inplace) {
     for (int e = blockIdx.x; e < ntab; e += gridDim.x) {
         const Work w = tab[e];
@@ -144,7 +155,7 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, GR>()) kb_res
         // (top level) also runs on single-level cells
         if ((!inplace && m >= S.nlev - 1) || !S.st->active) continue;
         const CellLevelDev& L = A.cells[S.cell].lv[m];
-        if (rep_skips(GR, m, L)) continue;
+        if (rep_skips(false, m, L)) continue;
         const int t = w.start + threadIdx.x;
         const int nn = L.nn;
         if (t >= nn) continue;
@@ -153,7 +164,7 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, GR>()) kb_res
         cell_ijk(L.n, t, i, j, k);
         const POff o = cell_offsets(L.n, i, j, k);
         R f[3];
-        level_apply<M, R, GR>(L, A.uniform, V.cor, t, o, f);
+        level_apply<M, R>(L, A.uniform, V.cor, t, o, f);
         R* out = inplace ? V.res : V.rescor;
         const R sc = row_factor(kfield<R>(L));
 #pragma unroll
@@ -346,14 +357,14 @@ __device__ __forceinline__ void block_partials(double (&v)[NQ], double* dst) {
 }
 
 // r = b - A x at level 0 with per-chunk sums of r (tab: one kRedChunk run per entry)
-template <int M, bool GR>
+template <int M>
 __global__ void __launch_bounds__(kCellThreads) kb_resid_top(CellArgs A, const Work* __restrict__ tab, int ntab) {
     for (int e = blockIdx.x; e < ntab; e += gridDim.x) {
         const Work w = tab[e];
         const SolveDev& S = A.solves[w.id];
         if (!S.st->active) continue;
         const CellLevelDev& L = A.cells[S.cell].lv[0];
-        if (rep_skips(GR, 0, L)) continue;
+        if (rep_skips(false, 0, L)) continue;
         const int t = w.start + threadIdx.x;
         const int nn = L.nn;
         double v[3] = {0.0, 0.0, 0.0};
@@ -362,7 +373,7 @@ __global__ void __launch_bounds__(kCellThreads) kb_resid_top(CellArgs A, const W
             cell_ijk(L.n, t, i, j, k);
             const POff o = cell_offsets(L.n, i, j, k);
             double f[3];
-            level_apply<M, double, GR>(L, A.uniform, S.x, t, o, f);
+            level_apply<M, double>(L, A.uniform, S.x, t, o, f);
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
                 v[p] = row_residual(S.b[p * nn + t], L.K64.i2[0], f[p]);
@@ -370,6 +381,341 @@ __global__ void __launch_bounds__(kCellThreads) kb_resid_top(CellArgs A, const W
             }
         }
         block_partials<3>(v, S.part + (size_t)(w.start / kRedChunk) * kPartStride);
+    }
+}
+
+// ------------------------------------------------------------------ finest level on a grain map
+// The smoother, the correction residual and the top residual of Voronoi cells.  A block takes its run of
+// nodes in two passes: every node's row without the grad C term, then, packed into as few warps as hold
+// them, the nodes whose neighbours lie in different grains, which get that term added.  In one pass nearly
+// every warp holds such a node and pays three columns of gathers (FP32) or operations (FP64) for all its
+// lanes.  The grains' numbers are in shared memory (up to kGrainTabs<R>; loaded when a block comes to
+// another cell): rows of an odd number of words, so that lanes in different grains hit different banks.
+// FP64 takes the row's 36 numbers from a table instead of forming them from the 21 slots (60 operations).
+// The arithmetic is that of cell_apply on the equivalent per-node field; a direction whose two neighbours
+// lie in the same grain has an exactly zero stiffness difference, so its column is zero.
+//
+// 128 cells of 16 to 64 nodes an edge: FP64 residual 5.14 -> 3.71 ms a call.  The FP32 sweeps gain nothing
+// by this alone (0.415 against 0.444 ms: 690 instructions a node, mostly wrapped addresses); they march below,
+// and this form serves the cells that do not fit there.
+template <class R>
+constexpr int kGrainTabs = sizeof(R) == 8 ? 56 : kMarchGrains;
+template <int M, class R>
+constexpr int grain_words() {  // slots, 1 / D, row numbers
+    const int n = NCoef<M>::value + 3 + (sizeof(R) == 8 ? RowN<M>::value : 0);
+    return n | 1;
+}
+enum CellOp { CELL_SMOOTH, CELL_RESCOR, CELL_RESID };
+template <int M, class R, int OP>
+__global__ void __launch_bounds__(kCellThreads, sizeof(R) == 4 ? AE_CELL_SMOOTH_BLOCKS : AE_CELL_GRAIN64_BLOCKS)
+    kb_grain_sweep(CellArgs A, const Work* __restrict__ tab, int ntab, int flag) {
+    constexpr int NC = NCoef<M>::value, TS = grain_words<M, R>();
+    __shared__ R ts[kGrainTabs<R> * TS];
+    __shared__ R qf[3][kCellThreads];
+    __shared__ unsigned char qt[kCellThreads];
+    __shared__ int qn;
+    int have = -1;  // the cell whose numbers are in ts
+    for (int e = blockIdx.x; e < ntab; e += gridDim.x) {
+        const Work w = tab[e];
+        const SolveDev& S = A.solves[w.id];
+        if ((OP == CELL_SMOOTH || (OP == CELL_RESCOR && !flag)) && S.nlev <= 1) continue;
+        if (!S.st->active) continue;
+        const CellLevelDev& L = A.cells[S.cell].lv[0];
+        if (rep_skips(true, 0, L)) continue;
+        if (sizeof(R) == 4 && cell_marches(L)) continue;
+        const int nn = L.nn;
+        const bool in_smem = L.ngrains <= kGrainTabs<R>;
+        __syncthreads();  // the block is done with the queue and the numbers
+        if (threadIdx.x == 0) qn = 0;
+        if (in_smem && have != S.cell) {
+            for (int q = threadIdx.x; q < L.ngrains * TS; q += blockDim.x) {
+                const int g = q / TS, c = q - g * TS;
+                if (c < NC) ts[q] = tabfield<R>(L)[g * NC + c];
+                else if (c < NC + 3) ts[q] = itabfield<R>(L)[3 * g + c - NC];
+                else if constexpr (sizeof(R) == 8)
+                    if (c < NC + 3 + RowN<M>::value) ts[q] = L.rows64[g * RowN<M>::value + c - NC - 3];
+            }
+            have = S.cell;
+        }
+        __syncthreads();
+        const CellVec<R>& V = vec_of<R>(S, 0);
+        const R *u, *b;
+        R* out;
+        if constexpr (OP == CELL_RESID) {
+            u = S.x;
+            b = S.b;
+            out = S.r;
+        } else {
+            u = OP == CELL_SMOOTH && flag ? V.cor2 : V.cor;
+            b = V.res;
+            out = OP == CELL_SMOOTH ? (flag ? V.cor : V.cor2) : flag ? V.res : V.rescor;
+        }
+        const SCoef<R>& K = kfield<R>(L);
+        const R sc = row_factor(K), omega = omega_of<R>(A);
+        const auto body = [&](auto smem) {
+            constexpr bool SM = decltype(smem)::value;
+            const auto slot = [&](int g, int q) { return SM ? ts[g * TS + q] : __ldg(tabfield<R>(L) + g * NC + q); };
+            const auto finish = [&](int t, int g, const R (&f)[3]) {
+                R v[3];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    v[p] = row_residual(b[p * nn + t], sc, f[p]);
+                    if (OP == CELL_SMOOTH) {
+                        const R id = SM ? ts[g * TS + NC + p] : __ldg(itabfield<R>(L) + 3 * g + p);
+                        v[p] = jacobi_update<R>(u[p * nn + t], v[p], id, omega);
+                    }
+                }
+#pragma unroll
+                for (int p = 0; p < 3; ++p) out[p * nn + t] = v[p];
+            };
+            const int t = w.start + (int)threadIdx.x;
+            bool wide = false;  // has a grad C column
+            R f[3];
+            if (t < nn) {
+                int i, j, k;
+                cell_ijk(L.n, t, i, j, k);
+                const POff o = cell_offsets(L.n, i, j, k);
+                const unsigned short* gid = L.gid + t;
+                const int g = __ldg(gid);
+                if (!A.uniform)
+                    wide = __ldg(gid + o.xp) != __ldg(gid + o.xm) || __ldg(gid + o.yp) != __ldg(gid + o.ym) ||
+                           __ldg(gid + o.zp) != __ldg(gid + o.zm);
+                R gu[3][3];
+                const CellAt<R> at{u + t, nn, o};
+                if constexpr (sizeof(R) == 8) {
+                    R D[3][6];
+                    row_diffs<R>(K, at, D, gu);
+                    row_scale(K, D);
+                    row_sum<M>([&](int n) { return SM ? ts[g * TS + NC + 3 + n] : __ldg(L.rows64 + g * RowN<M>::value + n); }, D, f);
+                } else {
+                    row_interior<M, R>(K, at, [&](int q) { return slot(g, q); }, gu, f);
+                }
+                if (!wide) finish(t, g, f);
+            }
+            const unsigned ball = __ballot_sync(0xffffffffu, wide);
+            if (ball) {
+                const int lane = threadIdx.x & 31, lead = __ffs(ball) - 1;
+                int at = 0;
+                if (lane == lead) at = atomicAdd(&qn, __popc(ball));
+                at = __shfl_sync(0xffffffffu, at, lead) + __popc(ball & ((1u << lane) - 1u));
+                if (wide) {
+                    qt[at] = (unsigned char)threadIdx.x;
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) qf[p][at] = f[p];
+                }
+            }
+            __syncthreads();
+            if ((int)threadIdx.x < qn) {
+                const int tq = w.start + (int)qt[threadIdx.x];
+                int i, j, k;
+                cell_ijk(L.n, tq, i, j, k);
+                const POff o = cell_offsets(L.n, i, j, k);
+                const unsigned short* gid = L.gid + tq;
+                const int off[3][2] = {{o.xp, o.xm}, {o.yp, o.ym}, {o.zp, o.zm}};
+                R gu[3][3], col[3][3];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    f[p] = qf[p][threadIdx.x];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        gu[p][d] = node_diff(K, d, u[p * nn + tq + off[d][0]], u[p * nn + tq + off[d][1]]);
+                }
+                grad_scale(K, gu);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const int gp = __ldg(gid + off[d][0]), gm = __ldg(gid + off[d][1]);
+                    if (gp == gm) {
+                        col[d][0] = col[d][1] = col[d][2] = R(0);
+                    } else {
+                        gradC_col_f<M, R>([&](int q) { return slot(gp, q) - slot(gm, q); }, gu, d, col[d]);
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < 3; ++r) f[r] = row_gradc(K, f[r], col[0][r], col[1][r], col[2][r]);
+                finish(tq, __ldg(gid), f);
+            }
+        };
+        if (in_smem) body(std::true_type());
+        else body(std::false_type());
+        if constexpr (OP == CELL_RESID) {
+            __syncthreads();
+            const int t = w.start + (int)threadIdx.x;
+            double v[3] = {0.0, 0.0, 0.0};
+            if (t < nn)
+#pragma unroll
+                for (int p = 0; p < 3; ++p) v[p] = out[p * nn + t];
+            block_partials<3>(v, S.part + (size_t)(w.start / kRedChunk) * kPartStride);
+        }
+    }
+}
+
+// The FP32 sweeps of those cells (cell_marches): a block takes kMarchNodes consecutive nodes of a plane
+// and marches up to kz planes in k.  A ring of four planes in shared memory holds the whole rows the
+// block's nodes touch, wrapped in y and z as they are loaded (cp.async, one plane ahead), so that a
+// displacement is read from global memory once a block and no address in the row is wrapped but along x;
+// the walk over solve, cell and level descriptors is paid once per kz planes.  A plane's nodes with a grad C
+// column go to a queue, and the block's first threads finish them from the ring.  Any n[0] up to kMarchX
+// fills the lanes: the nodes of a plane are taken in linear order.
+//
+// Bound by latency and by the shared-memory data path together.  128 cells of 16 to 64 nodes an edge:
+// smoother sweep 0.415 -> 0.314 ms, residual of the correction 0.417 -> 0.300.  A queue per warp over several
+// planes, its neighbours read from global memory, took 0.333; two planes a thread, 96 registers and five
+// blocks of 128 threads, 0.356; five blocks of this form (spills) 0.367.
+constexpr int kMarchW = kMarchNodes - 1 + 4 * kMarchX;  // words a component's rows take at most
+constexpr int kMarchRing = 4;                            // planes k - 1, k, k + 1 and the next
+template <int M>
+constexpr size_t march_smem() {
+    return sizeof(float) * (kMarchRing * 3 * kMarchW + kGrainTabs<float> * grain_words<M, float>() + 4 * kMarchNodes + 2);
+}
+template <int M, int OP>
+__global__ void __launch_bounds__(kMarchNodes, kMarchBlocks)
+    kb_grain_march(CellArgs A, const Work* __restrict__ tab, int ntab, int kz, int flag) {
+    using R = float;
+    constexpr int NC = NCoef<M>::value, TS = grain_words<M, R>();
+    extern __shared__ __align__(16) unsigned char march_mem[];
+    R* const ring = reinterpret_cast<R*>(march_mem);  // [kMarchRing][3][kMarchW]
+    R* const ts = ring + kMarchRing * 3 * kMarchW;
+    const int lane = threadIdx.x & 31;
+    R* const qf = ts + kGrainTabs<R> * TS;  // [3][kMarchNodes]: a queued node's row so far
+    int* const qt = reinterpret_cast<int*>(qf + 3 * kMarchNodes);  // its thread
+    int* const qn = qt + kMarchNodes;                                // entries, of even and odd planes
+    int have = -1;  // the cell whose numbers are in ts
+    for (int e = blockIdx.x; e < ntab; e += gridDim.x) {
+        const Work w = tab[e];
+        const SolveDev& S = A.solves[w.id];
+        if ((OP == CELL_SMOOTH || !flag) && S.nlev <= 1) continue;
+        if (!S.st->active) continue;
+        const CellLevelDev& L = A.cells[S.cell].lv[0];
+        const int n0 = L.n[0], n1 = L.n[1], n2 = L.n[2], nn = L.nn, sz = n0 * n1;
+        const CellVec<R>& V = S.v32[0];
+        const R* const u = OP == CELL_SMOOTH && flag ? V.cor2 : V.cor;
+        const R* const b = V.res;
+        R* const out = OP == CELL_SMOOTH ? (flag ? V.cor : V.cor2) : flag ? V.res : V.rescor;
+        const unsigned short* const gids = L.gid;
+        const SCoef<R>& K = L.K32;
+        const R sc = row_factor(K), omega = omega_of<R>(A);
+        const int z0 = w.start / sz, c0 = w.start - z0 * sz, z1 = min(z0 + kz, n2);  // planes z0 .. z1 - 1
+        const int cm = min(c0 + (int)threadIdx.x, sz - 1);
+        const bool act = c0 + (int)threadIdx.x < sz;
+        const int j = cm / n0, i = cm - j * n0;
+        // the rows j0 - 1 .. j1 + 1 of a plane, one after another
+        const int j0 = c0 / n0, j1 = min(c0 + kMarchNodes - 1, sz - 1) / n0;
+        const int words = (j1 - j0 + 3) * n0;
+        const int at = (j - j0 + 1) * n0 + i, xp = i == n0 - 1 ? 1 - n0 : 1, xm = i == 0 ? n0 - 1 : -1;
+        __syncthreads();  // the block is done with the ring and the numbers
+        constexpr int kLoads = (kMarchW + kMarchNodes - 1) / kMarchNodes;
+        int from[kLoads];  // the thread's words of a plane: their place in the cell's plane, or none
+#pragma unroll
+        for (int l = 0; l < kLoads; ++l) {
+            const int q = threadIdx.x + l * kMarchNodes, r = q / n0;
+            int jj = j0 - 1 + r;
+            jj = jj < 0 ? jj + n1 : jj >= n1 ? jj - n1 : jj;
+            from[l] = q < words ? jj * n0 + (q - r * n0) : -1;
+        }
+        const auto load = [&](int k) {  // plane k, z0 - 1 <= k <= z1
+            const R* src = u + (k < 0 ? k + n2 : k >= n2 ? k - n2 : k) * sz;
+            R* dst = ring + (k & (kMarchRing - 1)) * (3 * kMarchW) + threadIdx.x;
+#pragma unroll
+            for (int l = 0; l < kLoads; ++l)
+                if (from[l] >= 0)
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) cp_async<4>(dst + p * kMarchW + l * kMarchNodes, src + from[l] + p * nn);
+            cp_async_commit();
+        };
+        load(z0 - 1);
+        load(z0);
+        load(z0 + 1);
+        if (threadIdx.x < 2) qn[threadIdx.x] = 0;
+        if (have != S.cell) {
+            for (int q = threadIdx.x; q < L.ngrains * TS; q += kMarchNodes) {
+                const int g = q / TS, c = q - g * TS;
+                if (c < NC) ts[q] = L.tab32[g * NC + c];
+                else if (c < NC + 3) ts[q] = L.itab32[3 * g + c - NC];
+            }
+            have = S.cell;
+        }
+        const auto finish = [&](int t, int g, const R (&xc)[3], const R (&f)[3]) {
+            R v[3];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                v[p] = row_residual(b[p * nn + t], sc, f[p]);
+                if (OP == CELL_SMOOTH) v[p] = jacobi_update<R>(xc[p], v[p], ts[g * TS + NC + p], omega);
+            }
+#pragma unroll
+            for (int p = 0; p < 3; ++p) out[p * nn + t] = v[p];
+        };
+        const int yo = j == n1 - 1 ? (1 - n1) * n0 : n0, ym = j == 0 ? (n1 - 1) * n0 : -n0;
+        for (int k = z0; k < z1; ++k) {
+            cp_async_wait<0>();
+            __syncthreads();
+            if (k + 1 < z1) load(k + 2);
+            const auto slot = [&](int kk) { return ring + (kk & (kMarchRing - 1)) * (3 * kMarchW); };
+            const R* pl[3] = {slot(k - 1) + at, slot(k) + at, slot(k + 1) + at};
+            const int t = cm + k * sz;
+            const int up = k == n2 - 1 ? (1 - n2) * sz : sz, down = k == 0 ? (n2 - 1) * sz : -sz;
+            const unsigned short* gid = gids + t;
+            const int g = __ldg(gid);
+            bool wide = false;  // has a grad C column
+            if (act && !A.uniform)
+                wide = __ldg(gid + xp) != __ldg(gid + xm) || __ldg(gid + yo) != __ldg(gid + ym) ||
+                       __ldg(gid + up) != __ldg(gid + down);
+            R f[3], gu[3][3];
+            row_interior<M, R>(
+                K,
+                [&](int p, int a, int bb, int c) {
+                    return pl[c + 1][p * kMarchW + (a > 0 ? xp : a < 0 ? xm : 0) + (bb > 0 ? n0 : bb < 0 ? -n0 : 0)];
+                },
+                [&](int q) { return ts[g * TS + q]; }, gu, f);
+            if (act && !wide) {
+                const R xc[3] = {pl[1][0], pl[1][kMarchW], pl[1][2 * kMarchW]};
+                finish(t, g, xc, f);
+            }
+            int* const n = qn + (k & 1);
+            const unsigned ball = __ballot_sync(0xffffffffu, wide);
+            if (ball) {
+                const int lead = __ffs(ball) - 1;
+                int q = 0;
+                if (lane == lead) q = atomicAdd(n, __popc(ball));
+                q = __shfl_sync(0xffffffffu, q, lead) + __popc(ball & ((1u << lane) - 1u));
+                if (wide) {
+                    qt[q] = threadIdx.x;
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) qf[p * kMarchNodes + q] = f[p];
+                }
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) qn[(k + 1) & 1] = 0;  // read last before this plane's first barrier
+            if ((int)threadIdx.x < *n) {
+                const int c = c0 + qt[threadIdx.x], jj = c / n0, ii = c - jj * n0, tq = c + k * sz;
+                const int aq = (jj - j0 + 1) * n0 + ii;
+                const int qxp = ii == n0 - 1 ? 1 - n0 : 1, qxm = ii == 0 ? n0 - 1 : -1;
+                const int goff[3][2] = {{qxp, qxm},
+                                        {jj == n1 - 1 ? (1 - n1) * n0 : n0, jj == 0 ? (n1 - 1) * n0 : -n0}, {up, down}};
+                const R *qm = slot(k - 1) + aq, *qc = slot(k) + aq, *qp = slot(k + 1) + aq;
+                R gv[3][3], col[3][3], fq[3];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    fq[p] = qf[p * kMarchNodes + threadIdx.x];
+                    gv[p][0] = node_diff(K, 0, qc[p * kMarchW + qxp], qc[p * kMarchW + qxm]);
+                    gv[p][1] = node_diff(K, 1, qc[p * kMarchW + n0], qc[p * kMarchW - n0]);
+                    gv[p][2] = node_diff(K, 2, qp[p * kMarchW], qm[p * kMarchW]);
+                }
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const int gp = __ldg(gids + tq + goff[d][0]), gm = __ldg(gids + tq + goff[d][1]);
+                    if (gp == gm) {
+                        col[d][0] = col[d][1] = col[d][2] = R(0);
+                    } else {
+                        const R *cp = ts + gp * TS, *cq = ts + gm * TS;
+                        gradC_col_f<M, R>([&](int u_) { return cp[u_] - cq[u_]; }, gv, d, col[d]);
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < 3; ++r) fq[r] = row_gradc(K, fq[r], col[0][r], col[1][r], col[2][r]);
+                const R xc[3] = {qc[0], qc[kMarchW], qc[2 * kMarchW]};
+                finish(tq, __ldg(gids + tq), xc, fq);
+            }
+        }
     }
 }
 
@@ -681,7 +1027,7 @@ __global__ void __launch_bounds__(kCellThreads) kb_grains(CellLevelDev L, double
     for (int q = 0; q < NC; ++q) L.C64[q * L.nn + t] = table[best * NC + q];
 }
 
-// per-grain FP32 stiffness, diagonal and 1/diagonal (the values kb_diag gives the grain's nodes)
+// per-grain FP32 stiffness, FP64 row numbers and 1/diagonal (the values kb_diag gives the grain's nodes)
 template <int M>
 __global__ void kb_grain_tables(CellLevelDev L) {
     constexpr int NC = NCoef<M>::value;
@@ -691,11 +1037,13 @@ __global__ void kb_grain_tables(CellLevelDev L) {
     cell_diag<M, double>(L.K64, L.tab64 + g * NC, 1, 0, d);
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-        L.dtab64[3 * g + p] = d[p];
         L.itab64[3 * g + p] = 1.0 / d[p];
         L.itab32[3 * g + p] = (float)(1.0 / d[p]);
     }
     for (int q = 0; q < NC; ++q) L.tab32[g * NC + q] = (float)L.tab64[g * NC + q];
+#pragma unroll
+    for (int n = 0; n < RowN<M>::value; ++n)
+        L.rows64[g * RowN<M>::value + n] = row_number<M>([&](int q) { return L.tab64[g * NC + q]; }, n);
 }
 
 inline int grid_of(int ntab, Shape sh) { return ntab < sh.grid ? ntab : sh.grid; }
@@ -709,26 +1057,52 @@ void by_prec(int prec, F&& f) {
 }  // namespace
 
 // ------------------------------------------------------------------ launchers
-// reps: bit 0 launch the per-node variant, bit 1 the grain-table variant (finest level)
+// the variants of a stencil kernel that the cells present need: f(true) on grain maps, f(false) per node
 template <class F>
 void by_rep(int reps, F&& f) {
-    if (reps & 1) f(std::false_type());
-    if (reps & 2) f(std::true_type());
+    if (reps & kRepNode) f(std::false_type());
+    if (reps & (kRepGrains | kRepMarch)) f(std::true_type());
+}
+// grain maps, smoother and correction residual: marching cells in FP32 apart from the others
+template <int M, class R, int OP>
+void launch_grain_sweep(const CellArgs& A, const Work* tab, int ntab, Shape sh, int flag, int reps, const MarchTab& mt,
+                        cudaStream_t st) {
+    if (reps & (sizeof(R) == 4 ? kRepGrains : kRepGrains | kRepMarch)) {
+        kb_grain_sweep<M, R, OP><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, flag);
+        launched();
+    }
+    if constexpr (sizeof(R) == 4) {
+        if (reps & kRepMarch) {
+            constexpr size_t smem = march_smem<M>();
+            static std::once_flag once;
+            std::call_once(once, [] {
+                AE_CUDA_CHECK(cudaFuncSetAttribute(kb_grain_march<M, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            });
+            kb_grain_march<M, OP><<<std::min(mt.n, mt.grid), kMarchNodes, smem, st>>>(A, mt.tab, mt.n, mt.kz, flag);
+            launched();
+        }
+    }
 }
 
 void cells_launch_smooth(int model, int prec, bool zero, const CellArgs& A, const Work* tab, int ntab, Shape sh,
-                         int m, int from2, int reps, cudaStream_t st) {
+                         int m, int from2, int reps, const MarchTab& mt, cudaStream_t st) {
     if (ntab == 0) return;
     dispatch_model<double>(model, [&](auto mm) {
         constexpr int M = decltype(mm)::value;
         by_prec(prec, [&](auto r) {
             using R = decltype(r);
-            by_rep(reps, [&](auto gr) {
-                constexpr bool GR = decltype(gr)::value;
-                if (zero) kb_smooth<M, R, true, GR><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, m, from2);
-                else kb_smooth<M, R, false, GR><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, m, from2);
+            if (zero) {
+                by_rep(reps, [&](auto gr) {
+                    kb_smooth<M, R, true, decltype(gr)::value><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, m, from2);
+                    launched();
+                });
+                return;
+            }
+            if (reps & kRepNode) {
+                kb_smooth<M, R, false, false><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, m, from2);
                 launched();
-            });
+            }
+            launch_grain_sweep<M, R, CELL_SMOOTH>(A, tab, ntab, sh, from2, reps, mt, st);
         });
     });
 }
@@ -743,16 +1117,17 @@ void cells_launch_fill0(int prec, const CellArgs& A, const Work* tab, int ntab, 
     launched();
 }
 void cells_launch_rescor(int model, int prec, const CellArgs& A, const Work* tab, int ntab, Shape sh, int m,
-                         int inplace, int reps, cudaStream_t st) {
+                         int inplace, int reps, const MarchTab& mt, cudaStream_t st) {
     if (ntab == 0) return;
     dispatch_model<double>(model, [&](auto mm) {
         constexpr int M = decltype(mm)::value;
         by_prec(prec, [&](auto r) {
-            by_rep(reps, [&](auto gr) {
-                kb_rescor<M, decltype(r), decltype(gr)::value><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, m,
-                                                                                                       inplace);
+            using R = decltype(r);
+            if (reps & kRepNode) {
+                kb_rescor<M, R><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, m, inplace);
                 launched();
-            });
+            }
+            launch_grain_sweep<M, R, CELL_RESCOR>(A, tab, ntab, sh, inplace, reps, mt, st);
         });
     });
 }
@@ -781,7 +1156,9 @@ void cells_launch_resid_top(int model, const CellArgs& A, const Work* tab, int n
     if (ntab == 0) return;
     dispatch_model<double>(model, [&](auto mm) {
         by_rep(reps, [&](auto gr) {
-            kb_resid_top<decltype(mm)::value, decltype(gr)::value><<<ntab, kRedChunk, 0, st>>>(A, tab, ntab);
+            constexpr int M = decltype(mm)::value;
+            if (decltype(gr)::value) kb_grain_sweep<M, double, CELL_RESID><<<ntab, kRedChunk, 0, st>>>(A, tab, ntab, 0);
+            else kb_resid_top<M><<<ntab, kRedChunk, 0, st>>>(A, tab, ntab);
             launched();
         });
     });

@@ -497,6 +497,12 @@ __device__ __forceinline__ void row_scale(const SCoef<R>& K, R D[3][6]) {
 #pragma unroll
         for (int s = 1; s < 6; ++s) D[p][s] = mul_rn(D[p][s], K.sd[s]);
 }
+// the central difference along d that row_interior hands on, from the two neighbours
+template <class R>
+__device__ __forceinline__ R node_diff(const SCoef<R>& K, int d, R p, R m) {
+    if constexpr (sizeof(R) == 8) return sub_rn(p, m);
+    else return (p - m) * K.h[d];
+}
 // (FP64: row_interior's FP32 differences are scaled already)
 template <class R>
 __device__ __forceinline__ void grad_scale(const SCoef<R>& K, R g[3][3]) {
