@@ -45,18 +45,19 @@ __device__ __forceinline__ void reg_ijk(const Reg& r, unsigned t, int& i, int& j
     j = r.lo[1] + (int)jj;
     k = r.lo[2] + (int)kk;
 }
-// A region as the part inside a box, and the slabs around that part.  Per-node sweeps run the inside
-// first and the slabs in further blocks of the same launch: a warp that mixes a boundary row's one-sided
-// gradient and stress with interior rows pays for both, and with rows of 65 nodes nearly every warp did
-// (in FP64 about 70 operations on top of 100).  65^3 isotropic solve, all levels: Jacobi 28.6 -> 21.1 us a
-// sweep, residual 27.8 -> 20.3; 97 x 81 x 113 cubic Jacobi 470 -> 407.  In FP32 the operations
-// do not bound: 129^3 cubic Fapply 97.7 -> 94.9, but the coarse levels' Jacobi 25.7 -> 27.5 and residual 25.9 ->
-// 26.5 us, so those two keep all their nodes in one part there.
+// A region as the part inside a box, and the slabs around that part.  Per-node sweeps run the slabs in a
+// launch's first blocks (they take longer, and last they were its tail) and the inside in the rest: a warp
+// that mixes a boundary row's one-sided gradient and stress with interior rows pays for both, and with rows of
+// 65 nodes nearly every warp did (in FP64 about 70 operations on top of 100).  65^3 isotropic solve, all
+// levels: Jacobi 28.6 -> 21.1 us a sweep, residual 27.8 -> 20.3; 97 x 81 x 113 cubic Jacobi 470 -> 407.  Slabs first:
+// 129^3 cubic stress and energy 503 -> 489, set-up 1381 -> 1340, FP32 Fapply call 104.8 -> 102.0.  In FP32 the
+// operations do not bound: 129^3 cubic Fapply 97.7 -> 94.9, but the coarse levels' Jacobi 25.7 -> 27.5 and
+// residual 25.9 -> 26.5 us, so those two keep all their nodes in one part there.
 struct Parts {
     Reg in;               // n == 0: none
     Reg slab[6];
     unsigned end[6];      // nodes of slabs 0 .. q
-    unsigned in_blocks;
+    unsigned out_blocks;  // blocks of the slabs, before those of the inside
 };
 inline Parts make_parts(const Box3& r, Box3 inside) {
     Parts P;
@@ -86,7 +87,7 @@ inline Parts make_parts(const Box3& r, Box3 inside) {
         n += P.slab[q].n;
         P.end[q] = n;
     }
-    P.in_blocks = (P.in.n + kBlock - 1) / kBlock;
+    P.out_blocks = (P.end[5] + kBlock - 1) / kBlock;
     return P;
 }
 // the inside for the FP64 Jacobi sweep and residual; empty in FP32
@@ -95,16 +96,16 @@ inline Box3 parts_inside(const Geo& g) {
     if (sizeof(R) == 8) return geo_interior(g);
     return Box3{{1, 1, 1}, {0, 0, 0}};
 }
-inline unsigned parts_blocks(const Parts& P) { return P.in_blocks + (P.end[5] + kBlock - 1) / kBlock; }
+inline unsigned parts_blocks(const Parts& P) { return P.out_blocks + (P.in.n + kBlock - 1) / kBlock; }
 // this thread's node; false: none.  The whole block is inside or outside.
 __device__ __forceinline__ bool parts_ijk(const Parts& P, bool inside, int& i, int& j, int& k) {
     if (inside) {
-        const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+        const unsigned t = (blockIdx.x - P.out_blocks) * blockDim.x + threadIdx.x;
         if (t >= P.in.n) return false;
         reg_ijk(P.in, t, i, j, k);
         return true;
     }
-    unsigned t = (blockIdx.x - P.in_blocks) * blockDim.x + threadIdx.x;
+    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= P.end[5]) return false;
     int q = 0;
     unsigned before = 0;
@@ -193,7 +194,7 @@ constexpr int sweep_min_blocks() {
 template <int M, class R, bool GR>
 __global__ void __launch_bounds__(kBlock) k_fapply(OpParams P, SCoef<R> K, Parts parts, View<const R> C, Grains<R> G,
                                                    View<const R> u, View<R> f) {
-    const bool inside = blockIdx.x < parts.in_blocks;
+    const bool inside = blockIdx.x >= parts.out_blocks;
     int i, j, k;
     if (!parts_ijk(parts, inside, i, j, k)) return;
     R v[3];
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_residual(
                                                                                  View<const R> x, View<const R> b,
                                                                                  View<R> r, unsigned long long* norm,
                                                                                  View<float> r32) {
-    const bool inside = sizeof(R) == 8 && blockIdx.x < parts.in_blocks;
+    const bool inside = sizeof(R) == 8 && blockIdx.x >= parts.out_blocks;
     double mx = 0.0;
     int i, j, k;
     if (parts_ijk(parts, inside, i, j, k)) {
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_jacobi(Op
                                                                                View<const R> invD,
                                                                                View<const R> xi, View<const R> b,
                                                                                View<R> xo, R omega) {
-    const bool inside = sizeof(R) == 8 && blockIdx.x < parts.in_blocks;
+    const bool inside = sizeof(R) == 8 && blockIdx.x >= parts.out_blocks;
     int i, j, k;
     if (!parts_ijk(parts, inside, i, j, k)) return;
     if (inside) jacobi_node<M, R, GR, SAME, true>(P, K, C, G, invD, xi, b, xo, omega, i, j, k);
@@ -534,7 +535,7 @@ template <int M, class R>
 __global__ void __launch_bounds__(kBlock) k_diagonal(OpParams P, SCoef<R> K, Parts parts, View<const R> C, View<R> D,
                                                      View<R> invD, int* nan_flag) {
     constexpr int NC = NCoef<M>::value;
-    const bool inside = blockIdx.x < parts.in_blocks;
+    const bool inside = blockIdx.x >= parts.out_blocks;
     int i, j, k;
     if (!parts_ijk(parts, inside, i, j, k)) return;
     const Geo& g = P.g;
@@ -623,7 +624,7 @@ __global__ void __launch_bounds__(kBlock) k_diagonal(OpParams P, SCoef<R> K, Par
 // 30 FP64 operations a value need 0.30).
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_restrict(Geo gc, Parts parts, View<R> crse, View<const R> fine) {
-    const bool inside = blockIdx.x < parts.in_blocks;
+    const bool inside = blockIdx.x >= parts.out_blocks;
     int I, J, Kc;
     if (!parts_ijk(parts, inside, I, J, Kc)) return;
     const bool xe = !inside && (I == gc.dlo[0] || I == gc.dhi[0]);

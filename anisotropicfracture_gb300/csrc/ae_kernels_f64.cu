@@ -247,7 +247,7 @@ inline Parts post_parts(const Geo& g) {
 }
 __global__ void __launch_bounds__(kBlock) k_strain(Geo g, SCoef<double> K, Parts parts, View<const double> u,
                                                    View<double> e, int voigt) {
-    const bool inside = blockIdx.x < parts.in_blocks;
+    const bool inside = blockIdx.x >= parts.out_blocks;
     int i, j, k;
     if (!parts_ijk(parts, inside, i, j, k)) return;
     double gu[3][3];
@@ -272,7 +272,7 @@ template <int M>
 __global__ void __launch_bounds__(kBlock) k_stress(Geo g, SCoef<double> K, Parts parts, View<const double> C,
                                                    View<const double> u, View<double> sg, int voigt, int energy) {
     constexpr int NC = NCoef<M>::value;
-    const bool inside = blockIdx.x < parts.in_blocks;
+    const bool inside = blockIdx.x >= parts.out_blocks;
     int i, j, k;
     if (!parts_ijk(parts, inside, i, j, k)) return;
     double gu[3][3], s[3][3], a[NC];
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(kBlock) k_newton_dw(SCoef<double> K, Reg reg, 
 __global__ void __launch_bounds__(kBlock) k_newton_rhs(Geo g, BCP bc, SCoef<double> K, Parts parts, Box3 bx1,
                                                        View<const double> u, View<const double> b,
                                                        View<const double> dw, View<double> rhs) {
-    const bool inside = blockIdx.x < parts.in_blocks;
+    const bool inside = blockIdx.x >= parts.out_blocks;
     int i, j, k;
     if (!parts_ijk(parts, inside, i, j, k)) return;
     const long long ob = b.at(i, j, k), orr = rhs.at(i, j, k), ow = dw.at(i, j, k);
