@@ -69,13 +69,14 @@ __device__ __forceinline__ void level_apply(const CellLevelDev& L, int uniform, 
 constexpr int kCellThreads = 256;
 // Resident blocks per SM requested for the FP32 cell sweeps (smoother, correction residual);
 // 0: the compiler's choice.  On a 512-cell mixed batch:
-//   finest level on a grain map: 4 blocks (64 registers), 482 solves/s, against 444 with the
-//     compiler's 80 registers;
+//   finest level on a grain map (kb_grain_sweep and the first sweep of a cycle): 4 blocks (64
+//     registers), 482 solves/s, against 444 with the compiler's 80 registers;
 //   per-node levels: 3 blocks (80 registers, about 100 B of spills), 507 solves/s, against 482
 //     with the compiler's 118 registers.
 #ifndef AE_CELL_SMOOTH_BLOCKS
 #define AE_CELL_SMOOTH_BLOCKS 4
 #endif
+// FP64 on a grain map: 2 blocks (128 registers, 34 KB of tables and queue each)
 #ifndef AE_CELL_GRAIN64_BLOCKS
 #define AE_CELL_GRAIN64_BLOCKS 2
 #endif

@@ -55,9 +55,9 @@ FAPPLY32_BYTES_PER_NODE_GRAINS = 12 + 2 + 12
 # split sweep's tiled kernel over the interior box (x 12, b 12, 1/D 12, id + direction mask 4,
 # out 12 = 52 algorithmic bytes), per node of that box; per node: the one-pass kernel.
 JACOBI32_TRAFFIC_PER_NODE = {True: 52.1, False: 131.1}
-# FP64 operations per node (FMA counted as 2) of the FP64 Fapply on a grain map: ncu counts of
-# DFMA / DADD / DMUL thread instructions at 129^3 nodes
-FAPPLY64_FLOPS_PER_NODE_GRAINS = 215.0
+# FP64 operations per node (FMA counted as 2) of the FP64 Fapply on a grain map: the interior row's 99
+# operations, 60 of them FMAs; the 6 % of the nodes with a grad C column add to it
+FAPPLY64_FLOPS_PER_NODE_GRAINS = 159.0
 # FP64 composite iterations the config needs (measured by this benchmark's FP64 solve, which
 # matches the oracle iteration for iteration); used to extrapolate the CPU oracle's per-iteration
 # time to a full solve in the reference arm, which cannot afford a full CPU solve.
