@@ -185,8 +185,11 @@ inline bool same_layout(const View<A>& a, const View<B>& b) {
 #ifndef AE_PERNODE_SWEEP_BLOCKS
 #define AE_PERNODE_SWEEP_BLOCKS 0
 #endif
-template <class R, bool GR>
+template <class R, bool GR, int M = MM>
 constexpr int sweep_min_blocks() {
+    // 45 slots in FP32: two blocks need 128 registers; without the request the compiler took 130 to 140 for
+    // some variants, one block: 97^3 Jacobi sweep 147 us, residual 161, against 89.5 and 92.1
+    if (M == MAJOR && sizeof(R) == 4) return 2;
     return sizeof(R) != 4 ? 0 : GR ? AE_GRAIN_SWEEP_BLOCKS : AE_PERNODE_SWEEP_BLOCKS;
 }
 
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(kBlock) k_fapply(OpParams P, SCoef<R> K, Parts
 
 // ------------------------------------------------------------------ residual (+ norm, + FP32 copy)
 template <int M, class R, bool NORM, bool R32, bool GR, bool SAME>
-__global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_residual(OpParams P, SCoef<R> K, Parts parts,
+__global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR, M>()) k_residual(OpParams P, SCoef<R> K, Parts parts,
                                                                                  View<const R> C, Grains<R> G,
                                                                                  View<const R> x, View<const R> b,
                                                                                  View<R> r, unsigned long long* norm,
@@ -310,7 +313,7 @@ __global__ void __launch_bounds__(kBlock) k_jacobi_zero(Geo g, Reg reg, View<con
 }
 
 template <int M, class R, bool GR, bool SAME>
-__global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR>()) k_jacobi(OpParams P, SCoef<R> K, Parts parts,
+__global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR, M>()) k_jacobi(OpParams P, SCoef<R> K, Parts parts,
                                                                                View<const R> C, Grains<R> G,
                                                                                View<const R> invD,
                                                                                View<const R> xi, View<const R> b,
