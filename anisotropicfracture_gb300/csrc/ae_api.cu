@@ -1240,6 +1240,10 @@ int ae_op_set_model_grains(ae_op* op, int amrlev, const ae_fab* grain_id, int ng
             ids = cview(fab_view<int>(d));
         }
         const int nc = op->ncoef;
+        // the split sweeps' node ids and row numbers are those of the map and table replaced here: until the
+        // next prepare an FP64 product takes the per-node sweep, which reads both as they are
+        split_free(L.split);
+        L.split_built = false;
         if (!L.gid) L.gid = op->alloc<unsigned short>(L.nn);
         if (L.gcap < ngrains) {
             // 4 more: the sweeps copy the tables in whole 16 bytes
