@@ -3,6 +3,7 @@
 #include <type_traits>
 
 #include "ae_bottom_ell.h"
+#include "ae_div.h"
 #include "ae_kernels.cuh"
 #include "ae_krylov.cuh"
 
@@ -16,17 +17,6 @@ std::atomic<long long> g_kernel_launches{0};
 
 AE_INST_COPY(double, double)
 AE_INST_COPY(double, float)
-
-// a / d from inv = 1 / d: the product and one correction by its remainder
-__device__ __forceinline__ double div_by(double a, double d, double inv) {
-    const double q = a * inv;
-    const double c = fma(fma(-d, q, a), inv, q);
-    // outside the range where the remainder is exact, or with infinities, divide
-    const unsigned e = ((unsigned)__double2hiint(c) >> 20) & 0x7ff, ed = ((unsigned)__double2hiint(d) >> 20) & 0x7ff,
-                   ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ff;
-    const bool zero = (__double_as_longlong(a) << 1) == 0;
-    return ed - 64u < 0x780u && (zero || (e - 64u < 0x780u && ea - 64u < 0x780u)) ? c : a / d;
-}
 
 // ------------------------------------------------------------------ BC::Operator::Elastic::Init
 // src/BC/Operator/Elastic.H:106-181: boundary values into the rhs on every domain-boundary node.
