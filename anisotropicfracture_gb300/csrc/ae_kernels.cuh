@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 
 #include "ae_device.cuh"
 #include "ae_launch.h"
@@ -51,8 +52,10 @@ __device__ __forceinline__ void reg_ijk(const Reg& r, unsigned t, int& i, int& j
 // 65 nodes nearly every warp did (in FP64 about 70 operations on top of 100).  65^3 isotropic solve, all
 // levels: Jacobi 28.6 -> 21.1 us a sweep, residual 27.8 -> 20.3; 97 x 81 x 113 cubic Jacobi 470 -> 407.  Slabs first:
 // 129^3 cubic stress and energy 503 -> 489, set-up 1381 -> 1340, FP32 Fapply call 104.8 -> 102.0.  In FP32 the
-// operations do not bound: 129^3 cubic Fapply 97.7 -> 94.9, but the coarse levels' Jacobi 25.7 -> 27.5 and
-// residual 25.9 -> 26.5 us, so those two keep all their nodes in one part there.
+// operations do not bound: 129^3 cubic Fapply 97.7 -> 94.9, but the coarse levels' Jacobi 25.7 -> 27.5 us, so
+// that keeps all its nodes in one part; the residual and the 45-slot Fapply take the plain region (Region below):
+// as Parts, 129^3 cubic residual 112.9 us, now 108.5, isotropic 59.4, now 56.9 (five blocks; of the compiler's
+// own accord four, 68.0); 45 slots at 129^3 211 us and at 33^3 12.3, now 187 and 8.2.
 struct Parts {
     Reg in;               // n == 0: none
     Reg slab[6];
@@ -90,7 +93,7 @@ inline Parts make_parts(const Box3& r, Box3 inside) {
     P.out_blocks = (P.end[5] + kBlock - 1) / kBlock;
     return P;
 }
-// the inside for the FP64 Jacobi sweep and residual; empty in FP32
+// the inside for the FP64 Jacobi sweep; empty in FP32
 template <class R>
 inline Box3 parts_inside(const Geo& g) {
     if (sizeof(R) == 8) return geo_interior(g);
@@ -114,6 +117,29 @@ __device__ __forceinline__ bool parts_ijk(const Parts& P, bool inside, int& i, i
     return true;
 }
 inline unsigned nblocks(unsigned n) { return (n + kBlock - 1) / kBlock; }
+
+// What a sweep runs over: Parts (APART) or, where the interior is not taken apart, the plain region, whose
+// kernels are shorter and take fewer registers.
+template <bool APART>
+using Region = std::conditional_t<APART, Parts, Reg>;
+template <bool APART>
+inline Region<APART> make_region(const Box3& r, const Geo& g) {
+    if constexpr (APART) return make_parts(r, geo_interior(g));
+    else return make_reg(r);
+}
+inline unsigned region_blocks(const Parts& P) { return parts_blocks(P); }
+inline unsigned region_blocks(const Reg& r) { return nblocks(r.n); }
+__device__ __forceinline__ bool region_inside(const Parts& P) { return blockIdx.x >= P.out_blocks; }
+__device__ __forceinline__ bool region_inside(const Reg&) { return false; }
+__device__ __forceinline__ bool region_ijk(const Parts& P, bool inside, int& i, int& j, int& k) {
+    return parts_ijk(P, inside, i, j, k);
+}
+__device__ __forceinline__ bool region_ijk(const Reg& r, bool, int& i, int& j, int& k) {
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= r.n) return false;
+    reg_ijk(r, t, i, j, k);
+    return true;
+}
 
 // after every kernel launch: surface launch errors and count the launch
 inline void launched() {
@@ -194,12 +220,17 @@ constexpr int sweep_min_blocks() {
 }
 
 // ------------------------------------------------------------------ Fapply
+// (45 slots in FP32: one row and two requested blocks; 129^3 nodes 211 us with both rows, 198 with one row and
+// the compiler's 102 registers, 187 with the 128 of two blocks)
+template <int M, class R>
+constexpr bool kFapplyApart = sizeof(R) == 8 || M != MAJOR;
 template <int M, class R, bool GR>
-__global__ void __launch_bounds__(kBlock) k_fapply(OpParams P, SCoef<R> K, Parts parts, View<const R> C, Grains<R> G,
-                                                   View<const R> u, View<R> f) {
-    const bool inside = blockIdx.x >= parts.out_blocks;
+__global__ void __launch_bounds__(kBlock, M == MAJOR && sizeof(R) == 4 ? 2 : 0)
+    k_fapply(OpParams P, SCoef<R> K, Region<kFapplyApart<M, R>> region, View<const R> C, Grains<R> G, View<const R> u,
+             View<R> f) {
+    const bool inside = region_inside(region);
     int i, j, k;
-    if (!parts_ijk(parts, inside, i, j, k)) return;
+    if (!region_ijk(region, inside, i, j, k)) return;
     R v[3];
     const R sc = inside ? apply_any<M, R, GR, true>(P, K, C, G, u, i, j, k, v)
                         : apply_any<M, R, GR, false>(P, K, C, G, u, i, j, k, v);
@@ -209,16 +240,22 @@ __global__ void __launch_bounds__(kBlock) k_fapply(OpParams P, SCoef<R> K, Parts
 }
 
 // ------------------------------------------------------------------ residual (+ norm, + FP32 copy)
+template <class R>
+constexpr bool kResidualApart = sizeof(R) == 8;
+template <int M, class R, bool GR>
+constexpr int residual_min_blocks() {
+    return M == ISO && sizeof(R) == 4 && !GR ? 5 : sweep_min_blocks<R, GR, M>();
+}
 template <int M, class R, bool NORM, bool R32, bool GR, bool SAME>
-__global__ void __launch_bounds__(kBlock, sweep_min_blocks<R, GR, M>()) k_residual(OpParams P, SCoef<R> K, Parts parts,
+__global__ void __launch_bounds__(kBlock, residual_min_blocks<M, R, GR>()) k_residual(OpParams P, SCoef<R> K, Region<kResidualApart<R>> region,
                                                                                  View<const R> C, Grains<R> G,
                                                                                  View<const R> x, View<const R> b,
                                                                                  View<R> r, unsigned long long* norm,
                                                                                  View<float> r32) {
-    const bool inside = sizeof(R) == 8 && blockIdx.x >= parts.out_blocks;
+    const bool inside = region_inside(region);
     double mx = 0.0;
     int i, j, k;
-    if (parts_ijk(parts, inside, i, j, k)) {
+    if (region_ijk(region, inside, i, j, k)) {
         R v[3];
         // SAME: every view has the layout of x (checked by the launcher)
         const long long ox = x.at(i, j, k);
