@@ -33,6 +33,7 @@
 
 #include "ae_kernels.cuh"
 #include "ae_split.h"
+#include "ae_split_rules.h"
 
 namespace ae {
 
@@ -857,20 +858,6 @@ void tile_smem_attr() {
             AE_CUDA_CHECK(cudaFuncSetAttribute(k_sweep_tile64<M, TABS, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                TL<double>::oT + tables));
     });
-}
-
-// Planes per block: the split of nz planes into chunks that takes the fewest plane times, waves of
-// blocks times the planes a block goes through (two more than it computes, and about four plane times
-// to fill its ring).
-int tile_kz(long long tiles, int nz, long long wave) {
-    int best = nz;
-    long long cost = -1;
-    for (int n = 1; n <= (nz + 3) / 4; ++n) {
-        const int kz = (nz + n - 1) / n;
-        const long long c = ((tiles * ((nz + kz - 1) / kz) + wave - 1) / wave) * (kz + 6);
-        if (cost < 0 || c < cost) cost = c, best = kz;
-    }
-    return best;
 }
 
 // the tiled kernel of one operation over I; b: the right-hand side, invD: 1/D (Jacobi only)
