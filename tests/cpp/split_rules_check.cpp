@@ -1,5 +1,5 @@
 // The launch rules of the split sweeps (csrc/ae_split_rules.h): a chunking of planes covers them, is not finer
-// than four planes, and is none of those measured well behind the best.  Exit status 0 when every case holds.
+// than three planes, and is none of those measured well behind the best.  Exit status 0 when every case holds.
 #include <cstdio>
 #include <initializer_list>
 
@@ -9,7 +9,7 @@ int main() {
     for (int nz = 1; nz <= 300; ++nz)
         for (long long tiles : {1ll, 2ll, 9ll, 30ll, 64ll, 85ll, 126ll, 152ll, 153ll, 256ll, 1000ll, 12321ll}) {
             const int kz = ae::tile_kz(tiles, nz, 152);
-            if (kz < 1 || kz > nz || (nz >= 4 && kz < 4)) {
+            if (kz < 1 || kz > nz || (nz >= 3 && kz < 3)) {
                 std::printf("tiles %lld, %d planes: chunks of %d\n", tiles, nz, kz);
                 return 1;
             }
