@@ -33,7 +33,6 @@
 
 #include "ae_kernels.cuh"
 #include "ae_split.h"
-#include "ae_split_rules.h"
 
 namespace ae {
 
@@ -236,10 +235,10 @@ template <int M, bool TABS, int OP>
 __global__ void __launch_bounds__(kTileThreads, 1)
     k_sweep_tile64(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_b,
                  const __grid_constant__ CUtensorMap tm_i, const __grid_constant__ CUtensorMap tm_g, SCoef<double> K, TileGeo T,
-                 int uniform, int sy, int sz, int sc, const unsigned* __restrict__ gidm,
+                 int uniform, int sy, int sz, long long sc, const unsigned* __restrict__ gidm,
                  const double* __restrict__ tab, const double* __restrict__ rows, int rows_bytes, int tab_bytes,
                  const double* __restrict__ x, const double* b, const double* __restrict__ invD, double* out, int osy, int osz,
-                 int osc, double omega, int* err) {
+                 long long osc, double omega, int* err) {
     using R = double;
     using L = TL<R>;
     constexpr int NC = NCoef<M>::value, TS = row_stride<M>();
@@ -902,9 +901,9 @@ void launch_tile(const OpParams& P, const SplitList& sl, const Box3& I, const Bo
                     out.sy, out.sz, out.sc, omega, err);
             } else {
                 k_sweep_tile64<Mv, TABS, OP><<<grid, kTileThreads, TL<double>::oT + (TABS ? rows_bytes + tab_bytes : 0), st>>>(
-                    tx, tb, ti, tg, K, T, P.uniform, (int)x.sy, (int)x.sz, (int)x.sc, sl.gidm, G.tab, sl.rows64,
+                    tx, tb, ti, tg, K, T, P.uniform, (int)x.sy, (int)x.sz, x.sc, sl.gidm, G.tab, sl.rows64,
                     TABS ? (int)rows_bytes : 0, TABS ? (int)tab_bytes : 0, x.p, b, invD, po, (int)out.sy,
-                    (int)out.sz, (int)out.sc, omega, err);
+                    (int)out.sz, out.sc, omega, err);
             }
             launched();
         };
@@ -924,8 +923,7 @@ bool split_supported(const Geo& g) {
     // 0 on level 0 and on refined patches with 2 ghost layers, 1 or 2 where one touches the domain's
     // low face
     const Box3 I = geo_interior(g);
-    // and the tiled kernels' offsets into the three components are 32-bit
-    return ((I.lo[0] - 1 - S.lo[0]) & 3) <= T32B - 34 && 3 * geo_nn(g) < (1ll << 31);
+    return ((I.lo[0] - 1 - S.lo[0]) & 3) <= T32B - 34 && split_range(geo_nn(g) / (S.hi[2] - S.lo[2] + 1), geo_nn(g));
 }
 
 // count and fill the list of region R \ I (and, with gidm, the id/mask array)

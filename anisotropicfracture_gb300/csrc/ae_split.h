@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "ae_launch.h"
+#include "ae_split_rules.h"
 
 namespace ae {
 
@@ -22,10 +23,10 @@ constexpr int kSplitMaxGrains = 1 << 16;
 
 // whether a level's layout allows the split sweep (row pitch a multiple of 4 nodes)
 bool split_supported(const Geo& g);
-// whether the split sweep can write a view: offsets into its three components are 32-bit
+// whether the split sweep can write a view
 template <class R>
 bool split_out(const View<R>& v) {
-    return 3 * v.sc < (1ll << 31);
+    return split_range(v.sz, v.sc);
 }
 // Build the node list and the id/mask array of a grain-map level (gid laid out like the level's
 // storage, at most kSplitMaxGrains grains) and the grains' row numbers; allocates sl's arrays with

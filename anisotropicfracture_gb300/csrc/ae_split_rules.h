@@ -22,4 +22,8 @@ inline int tile_kz(long long tiles, int nz, long long wave) {
     return best;
 }
 
+// Whether the tiled kernels can index an array of planes of sz elements, sc elements a component: offsets
+// inside a component are 32-bit (the components' own are not), and run a few planes past the box.
+inline bool split_range(long long sz, long long sc) { return sc + 8 * sz < (1ll << 31); }
+
 }  // namespace ae

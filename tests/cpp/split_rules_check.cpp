@@ -1,5 +1,6 @@
 // The launch rules of the split sweeps (csrc/ae_split_rules.h): a chunking of planes covers them, is not finer
-// than three planes, and is none of those measured well behind the best.  Exit status 0 when every case holds.
+// than three planes, and is none of those measured well behind the best; the sizes taken keep every offset an
+// int.  Exit status 0 when every case holds.
 #include <cstdio>
 #include <initializer_list>
 
@@ -30,6 +31,15 @@ int main() {
         for (int g : c.good) ok = ok || g == kz;
         if (!ok) {
             std::printf("tiles %d, %d planes: chunks of %d\n", c.tiles, c.nz, kz);
+            return 1;
+        }
+    }
+    // cubes of n nodes an edge, rows padded to 4: taken as long as the last offset a tile can form, two planes
+    // past the box and a tile's columns and rows past the last plane, is an int
+    for (long long n = 17; n < 1400; ++n) {
+        const long long px = (n + 3) / 4 * 4, sz = px * n, sc = sz * n, last = sz * (n + 2) + px * 8 + 32;
+        if (ae::split_range(sz, sc) ? last > 2147483647ll : n <= 1200) {
+            std::printf("%lld nodes an edge\n", n);
             return 1;
         }
     }
