@@ -83,15 +83,18 @@ constexpr int kCellThreads = 256;
 #ifndef AE_CELL_SMOOTH_BLOCKS_PERNODE
 #define AE_CELL_SMOOTH_BLOCKS_PERNODE 3
 #endif
-template <class R, bool GR>
+template <int M, class R, bool GR>
 constexpr int cell_min_blocks() {
+    // FP64, 21 slots per node: two blocks need 128 registers; the compiler took 186 for the smoother, one block:
+    // 19 cells of 64^3, fixed cycles, 58.5 ms, with two 56.3
+    if (M == MM && sizeof(R) == 8 && !GR) return 2;
     return sizeof(R) != 4 ? 0 : GR ? AE_CELL_SMOOTH_BLOCKS : AE_CELL_SMOOTH_BLOCKS_PERNODE;
 }
 
 // one damped-Jacobi sweep of the correction at level m: from2 = 0 reads cor and writes cor2,
 // from2 = 1 the reverse.  ZERO: the input is the zero vector (the first sweep of a V-cycle).
 template <int M, class R, bool ZERO, bool GR>
-__global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, GR>()) kb_smooth(CellArgs A, const Work* __restrict__ tab, int ntab, int m,
+__global__ void __launch_bounds__(kCellThreads, cell_min_blocks<M, R, GR>()) kb_smooth(CellArgs A, const Work* __restrict__ tab, int ntab, int m,
                                                           int from2) {
     for (int e = blockIdx.x; e < ntab; e += gridDim.x) {
         const Work w = tab[e];
@@ -147,7 +150,7 @@ __global__ void __launch_bounds__(kCellThreads) kb_copy2(CellArgs A, const Work*
 
 // rescor = res - A cor at level m (inplace: into res)
 template <int M, class R>
-__global__ void __launch_bounds__(kCellThreads, cell_min_blocks<R, false>()) kb_rescor(CellArgs A, const Work* __restrict__ tab, int ntab, int m,
+__global__ void __launch_bounds__(kCellThreads, cell_min_blocks<M, R, false>()) kb_rescor(CellArgs A, const Work* __restrict__ tab, int ntab, int m,
                                                           int inplace) {
     for (int e = blockIdx.x; e < ntab; e += gridDim.x) {
         const Work w = tab[e];
