@@ -75,6 +75,47 @@ __device__ __forceinline__ void cell_apply(const SCoef<R>& K, bool uniform, cons
     }
 }
 
+// A u = row_factor f at node t of a Voronoi cell stored as a grain id per node and a per-grain coefficient
+// table (tab[g * ncoef + q]), in FP64 with a table of the row's numbers beside it (rows).  The arithmetic is
+// that of cell_apply on the equivalent per-node field; a direction whose two neighbours lie in the same grain has an exactly zero stiffness
+// difference, so its column of the grad C term is zero and its loads are skipped.
+template <int M, class R>
+__device__ __forceinline__ void cell_apply_grains(const SCoef<R>& K, bool uniform,
+                                                  const unsigned short* __restrict__ gid,
+                                                  const R* __restrict__ tab, const double* __restrict__ rows,
+                                                  const R* __restrict__ U, int us, int t, const POff& o, R f[3]) {
+    constexpr int NC = NCoef<M>::value;
+    const int g = __ldg(gid + t);
+    const CellAt<R> at{U + t, us, o};
+    R gu[3][3];
+    if constexpr (sizeof(R) == 8) {
+        R D[3][6];
+        row_diffs<R>(K, at, D, gu);
+        row_scale(K, D);
+        row_sum<M>([&](int n) { return __ldg(rows + g * RowN<M>::value + n); }, D, f);
+    } else {
+        row_interior<M, R>(K, at, [&](int q) { return __ldg(tab + g * NC + q); }, gu, f);
+    }
+    if (!uniform) {
+        const int gp[3] = {__ldg(gid + t + o.xp), __ldg(gid + t + o.yp), __ldg(gid + t + o.zp)};
+        const int gm[3] = {__ldg(gid + t + o.xm), __ldg(gid + t + o.ym), __ldg(gid + t + o.zm)};
+        R col[3][3];
+        grad_scale(K, gu);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (gp[d] == gm[d]) {
+                col[d][0] = col[d][1] = col[d][2] = R(0);
+            } else {
+                const R* cp = tab + gp[d] * NC;
+                const R* cm = tab + gm[d] * NC;
+                gradC_col_f<M, R>([&](int q) { return __ldg(cp + q) - __ldg(cm + q); }, gu, d, col[d]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) f[r] = row_gradc(K, f[r], col[0][r], col[1][r], col[2][r]);
+    }
+}
+
 // interior diagonal (src/Operator/Elastic.cpp:320-341): C_{pjpj} (-2 / dx_j^2)
 template <int M, class R>
 __device__ __forceinline__ void cell_diag(const SCoef<R>& K, const R* __restrict__ C, int cs, int t, R d[3]) {

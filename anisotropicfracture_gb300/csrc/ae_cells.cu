@@ -63,6 +63,7 @@ size_t cell_layout(CellRes& c, char* base) {
         L.K32 = scoef_of<float>(dx);
         L.gid = nullptr;
         L.ngrains = 0;
+        L.march = 0;
         L.tab64 = nullptr;
         L.tab32 = nullptr;
         L.rows64 = nullptr;
@@ -304,11 +305,28 @@ void CellEngine::rebuild() {
     solve_base.assign(ncell, 0);
     maxL = 0;
     reps0 = 0;
+    // the cells that march: rows of up to kMarchX nodes, of up to kMarchXs, or none, by the work there is
+    const auto march_nodes = [&](int rows) {
+        long long n = 0;
+        for (const CellRes* r : live)
+            if (cell_can_march(r->lv[0], rows)) n += (long long)r->lv[0].nn * r->nrhs;
+        return n;
+    };
+    march_rows = 0;
+    if (march_nodes(kMarchXs) >= (model == AE_MODEL_DIAGONAL ? kMarchMinNodesD : kMarchMinNodes)) march_rows = kMarchXs;
+    if (march_nodes(kMarchX) >= kMarchMinNodesX) march_rows = kMarchX;
+    int longest = 0;
+    long long nodes = 0;
     for (int c = 0; c < ncell; ++c) {
         CellRes* r = live[c];
         CellDev& d = hcells[c];
         d.nlev = r->nlev;
         for (int m = 0; m < r->nlev; ++m) d.lv[m] = r->lv[m];
+        d.lv[0].march = cell_can_march(r->lv[0], march_rows);
+        if (d.lv[0].march) {
+            longest = std::max(longest, d.lv[0].n[0]);
+            nodes += (long long)d.lv[0].nn * r->nrhs;
+        }
         solve_base[c] = (int)hsolves.size();
         for (int k = 0; k < r->nrhs; ++k) {
             SolveDev s = r->sol[k];
@@ -318,8 +336,9 @@ void CellEngine::rebuild() {
             hsolves.push_back(s);
         }
         maxL = std::max(maxL, r->nlev);
-        reps0 |= !r->lv[0].gid ? kRepNode : cell_marches(r->lv[0]) ? kRepMarch : kRepGrains;
+        reps0 |= !r->lv[0].gid ? kRepNode : d.lv[0].march ? kRepMarch : kRepGrains;
     }
+    march_rows = longest;
     nsolves = (int)hsolves.size();
     if ((size_t)ncell > cap_cells || !dcells) {
         if (dcells) AEH_CHECK(cudaFree(dcells));
@@ -366,14 +385,11 @@ void CellEngine::rebuild() {
     tred.upload(st);
     // marching runs: as many planes each as leave every resident block two of them, at most 8 (the two
     // planes loaded beside those computed cost a quarter of them then)
-    long long nodes = 0;
-    for (int c = 0; c < ncell; ++c)
-        if (cell_marches(live[c]->lv[0])) nodes += (long long)live[c]->lv[0].nn * live[c]->nrhs;
     march_kz = (int)std::max(2ll, std::min(8ll, nodes / (2ll * kMarchNodes * nsm * kMarchBlocks)));
     tmarch.h.clear();
     for (int c = 0; c < ncell; ++c) {
-        const CellLevelDev& L = live[c]->lv[0];
-        if (!cell_marches(L)) continue;
+        const CellLevelDev& L = hcells[c].lv[0];
+        if (!L.march) continue;
         const int sz = L.n[0] * L.n[1];
         for (int z = 0; z < L.n[2]; z += march_kz)
             for (int c0 = 0; c0 < sz; c0 += kMarchNodes)

@@ -34,6 +34,7 @@ struct CellLevelDev {
     // the finest level read these instead of the per-node arrays (same values, far fewer bytes).
     unsigned short* gid;
     int ngrains;
+    int march;  // in the engine's descriptors: whether the FP32 finest-level sweeps march
     double* tab64;
     float* tab32;
     double* rows64;
@@ -104,17 +105,29 @@ struct Shape {
     int grid;
 };
 
-// Grain-map cells whose FP32 finest-level sweeps march (kb_grain_march): whole rows of a plane and the
-// grains' numbers fit its shared memory.
-constexpr int kMarchX = 64, kMarchGrains = 96;
+// How the finest-level sweeps of cells on a grain map run (CellEngine::rebuild); every way computes the same
+// bits.  "nodes" below are those of all solves together.
+//
+// FP32: marching (kb_grain_march) or one pass (kb_smooth, kb_rescor).  A cell can march when its rows and its
+// grains' numbers fit the kernel's shared memory: rows of up to 128 nodes in the wider of two forms (51 KB a
+// block, still four an SM), up to 64 in the other (38 KB).  Marching wins once its blocks, which take several
+// planes each, fill the chip a few times: for 21 or 2 slots from 1.5 million nodes on, for 9 slots, which leave
+// less to save, from 3 million, with rows over 64 nodes from 5 million.  Time of a fixed number of cycles, ms,
+// one pass / marching:
+//   21 slots   24 cells of 24^3 (0.33 M nodes) 7.2 / 8.0   6 of 64^3 (1.6 M) 14.0 / 13.6   46 (12 M) 89 / 80
+//    9 slots    6 cells of 64^3 8.9 / 9.3                 11 (2.9 M) 15.3 / 15.3           46 60 / 54
+//   rows of 96  3 cells (2.7 M) 21.2 / 22.0                7 (6.2 M) 46.0 / 44.2           14 (12 M) 88 / 84
+constexpr int kMarchX = 128, kMarchXs = 64, kMarchGrains = 96;
+constexpr long long kMarchMinNodes = 1500000, kMarchMinNodesD = 3000000, kMarchMinNodesX = 5000000;
 constexpr int kMarchNodes = 256, kMarchBlocks = 4;  // nodes of a plane a block takes, resident blocks per SM
-__host__ __device__ inline bool cell_marches(const CellLevelDev& L) {
-    return L.gid != nullptr && L.n[0] <= kMarchX && L.ngrains <= kMarchGrains;
+inline bool cell_can_march(const CellLevelDev& L, int rows) {
+    return L.gid != nullptr && L.n[0] <= rows && L.ngrains <= kMarchGrains;
 }
-// their work: entry start = first node of a run of nodes in plane z, kz planes from there on
+// the marching cells' work: entry start = first node of a run of nodes in plane z, kz planes from there on
 struct MarchTab {
     const Work* tab;
     int n, kz, grid;
+    int rows;  // the longest row among the cells
 };
 
 // ---- launchers (ae_cells_kernels.cu); model 0 ISO, 1 MM, 2 DIAG

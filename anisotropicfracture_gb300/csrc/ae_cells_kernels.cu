@@ -59,18 +59,19 @@ __device__ __forceinline__ bool rep_skips(bool GR, int m, const CellLevelDev& L)
     return GR ? (m != 0 || L.gid == nullptr) : (m == 0 && L.gid != nullptr);
 }
 
-// f = A u at node t of level m
-template <int M, class R>
+// A u = row_factor f at node t of level m
+template <int M, class R, bool GR>
 __device__ __forceinline__ void level_apply(const CellLevelDev& L, int uniform, const R* U, int t, const POff& o,
                                             R f[3]) {
-    cell_apply<M, R>(kfield<R>(L), uniform, cfield<R>(L), L.nn, U, L.nn, t, o, f);
+    if constexpr (GR) cell_apply_grains<M, R>(kfield<R>(L), uniform, L.gid, tabfield<R>(L), L.rows64, U, L.nn, t, o, f);
+    else cell_apply<M, R>(kfield<R>(L), uniform, cfield<R>(L), L.nn, U, L.nn, t, o, f);
 }
 
 constexpr int kCellThreads = 256;
 // Resident blocks per SM requested for the FP32 cell sweeps (smoother, correction residual);
 // 0: the compiler's choice.  On a 512-cell mixed batch:
-//   finest level on a grain map (kb_grain_sweep and the first sweep of a cycle): 4 blocks (64
-//     registers), 482 solves/s, against 444 with the compiler's 80 registers;
+//   finest level on a grain map: 4 blocks (64 registers), 482 solves/s, against 444 with the
+//     compiler's 80 registers;
 //   per-node levels: 3 blocks (80 registers, about 100 B of spills), 507 solves/s, against 482
 //     with the compiler's 118 registers.
 #ifndef AE_CELL_SMOOTH_BLOCKS
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<M, R, GR>()) kb_
         if (m >= S.nlev - 1 || !S.st->active) continue;
         const CellLevelDev& L = A.cells[S.cell].lv[m];
         if (rep_skips(GR, m, L)) continue;
+        if (GR && !ZERO && sizeof(R) == 4 && L.march) continue;  // kb_grain_march's
         const int t = w.start + threadIdx.x;
         const int nn = L.nn;
         if (t >= nn) continue;
@@ -124,7 +126,7 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<M, R, GR>()) kb_
         cell_ijk(L.n, t, i, j, k);
         const POff o = cell_offsets(L.n, i, j, k);
         R f[3];
-        level_apply<M, R>(L, A.uniform, xin, t, o, f);
+        level_apply<M, R, GR>(L, A.uniform, xin, t, o, f);
         const R sc = row_factor(kfield<R>(L));
 #pragma unroll
         for (int p = 0; p < 3; ++p)
@@ -149,8 +151,8 @@ __global__ void __launch_bounds__(kCellThreads) kb_copy2(CellArgs A, const Work*
 }
 
 // rescor = res - A cor at level m (inplace: into res)
-template <int M, class R>
-__global__ void __launch_bounds__(kCellThreads, cell_min_blocks<M, R, false>()) kb_rescor(CellArgs A, const Work* __restrict__ tab, int ntab, int m,
+template <int M, class R, bool GR>
+__global__ void __launch_bounds__(kCellThreads, cell_min_blocks<M, R, GR>()) kb_rescor(CellArgs A, const Work* __restrict__ tab, int ntab, int m,
                                                           int inplace) {
     for (int e = blockIdx.x; e < ntab; e += gridDim.x) {
         const Work w = tab[e];
@@ -159,7 +161,8 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<M, R, false>()) 
         // (top level) also runs on single-level cells
         if ((!inplace && m >= S.nlev - 1) || !S.st->active) continue;
         const CellLevelDev& L = A.cells[S.cell].lv[m];
-        if (rep_skips(false, m, L)) continue;
+        if (rep_skips(GR, m, L)) continue;
+        if (GR && sizeof(R) == 4 && L.march) continue;  // kb_grain_march's
         const int t = w.start + threadIdx.x;
         const int nn = L.nn;
         if (t >= nn) continue;
@@ -168,7 +171,7 @@ __global__ void __launch_bounds__(kCellThreads, cell_min_blocks<M, R, false>()) 
         cell_ijk(L.n, t, i, j, k);
         const POff o = cell_offsets(L.n, i, j, k);
         R f[3];
-        level_apply<M, R>(L, A.uniform, V.cor, t, o, f);
+        level_apply<M, R, GR>(L, A.uniform, V.cor, t, o, f);
         R* out = inplace ? V.res : V.rescor;
         const R sc = row_factor(kfield<R>(L));
 #pragma unroll
@@ -377,7 +380,7 @@ __global__ void __launch_bounds__(kCellThreads) kb_resid_top(CellArgs A, const W
             cell_ijk(L.n, t, i, j, k);
             const POff o = cell_offsets(L.n, i, j, k);
             double f[3];
-            level_apply<M, double>(L, A.uniform, S.x, t, o, f);
+            level_apply<M, double, false>(L, A.uniform, S.x, t, o, f);
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
                 v[p] = row_residual(S.b[p * nn + t], L.K64.i2[0], f[p]);
@@ -389,32 +392,31 @@ __global__ void __launch_bounds__(kCellThreads) kb_resid_top(CellArgs A, const W
 }
 
 // ------------------------------------------------------------------ finest level on a grain map
-// The smoother, the correction residual and the top residual of Voronoi cells.  A block takes its run of
-// nodes in two passes: every node's row without the grad C term, then, packed into as few warps as hold
+// The smoother, the correction residual and the top residual of Voronoi cells in FP64.  A block takes its run
+// of nodes in two passes: every node's row without the grad C term, then, packed into as few warps as hold
 // them, the nodes whose neighbours lie in different grains, which get that term added.  In one pass nearly
-// every warp holds such a node and pays three columns of gathers (FP32) or operations (FP64) for all its
-// lanes.  The grains' numbers are in shared memory (up to kGrainTabs<R>; loaded when a block comes to
-// another cell): rows of an odd number of words, so that lanes in different grains hit different banks.
-// FP64 takes the row's 36 numbers from a table instead of forming them from the 21 slots (60 operations).
-// The arithmetic is that of cell_apply on the equivalent per-node field; a direction whose two neighbours
-// lie in the same grain has an exactly zero stiffness difference, so its column is zero.
+// every warp holds such a node and pays three columns of operations for all its lanes.  The grains' numbers
+// are in shared memory (up to kGrainTabs; loaded when a block comes to another cell): rows of an odd number
+// of words, so that lanes in different grains hit different banks.  The row's 36 numbers come from a table
+// instead of being formed from the 21 slots (60 operations).  The arithmetic is that of cell_apply on the
+// equivalent per-node field; a direction whose two neighbours lie in the same grain has an exactly zero
+// stiffness difference, so its column is zero.
 //
-// 128 cells of 16 to 64 nodes an edge: FP64 residual 5.14 -> 3.71 ms a call.  The FP32 sweeps gain nothing
-// by this alone (0.415 against 0.444 ms: 690 instructions a node, mostly wrapped addresses); they march below,
-// and this form serves the cells that do not fit there.
-template <class R>
-constexpr int kGrainTabs = sizeof(R) == 8 ? 56 : kMarchGrains;
+// 128 cells of 16 to 64 nodes an edge: residual 5.14 -> 3.71 ms a call.  In FP32 two passes are slower than
+// one (0.444 against 0.415 ms): those sweeps march (kb_grain_march) or take one pass (kb_smooth, kb_rescor).
+constexpr int kGrainTabs = 56;
 template <int M, class R>
-constexpr int grain_words() {  // slots, 1 / D, row numbers
+constexpr int grain_words() {  // slots, 1 / D, row numbers (FP64)
     const int n = NCoef<M>::value + 3 + (sizeof(R) == 8 ? RowN<M>::value : 0);
     return n | 1;
 }
 enum CellOp { CELL_SMOOTH, CELL_RESCOR, CELL_RESID };
-template <int M, class R, int OP>
-__global__ void __launch_bounds__(kCellThreads, sizeof(R) == 4 ? AE_CELL_SMOOTH_BLOCKS : AE_CELL_GRAIN64_BLOCKS)
+template <int M, int OP>
+__global__ void __launch_bounds__(kCellThreads, AE_CELL_GRAIN64_BLOCKS)
     kb_grain_sweep(CellArgs A, const Work* __restrict__ tab, int ntab, int flag) {
+    using R = double;
     constexpr int NC = NCoef<M>::value, TS = grain_words<M, R>();
-    __shared__ R ts[kGrainTabs<R> * TS];
+    __shared__ R ts[kGrainTabs * TS];
     __shared__ R qf[3][kCellThreads];
     __shared__ unsigned char qt[kCellThreads];
     __shared__ int qn;
@@ -426,9 +428,8 @@ __global__ void __launch_bounds__(kCellThreads, sizeof(R) == 4 ? AE_CELL_SMOOTH_
         if (!S.st->active) continue;
         const CellLevelDev& L = A.cells[S.cell].lv[0];
         if (rep_skips(true, 0, L)) continue;
-        if (sizeof(R) == 4 && cell_marches(L)) continue;
         const int nn = L.nn;
-        const bool in_smem = L.ngrains <= kGrainTabs<R>;
+        const bool in_smem = L.ngrains <= kGrainTabs;
         __syncthreads();  // the block is done with the queue and the numbers
         if (threadIdx.x == 0) qn = 0;
         if (in_smem && have != S.cell) {
@@ -436,8 +437,7 @@ __global__ void __launch_bounds__(kCellThreads, sizeof(R) == 4 ? AE_CELL_SMOOTH_
                 const int g = q / TS, c = q - g * TS;
                 if (c < NC) ts[q] = tabfield<R>(L)[g * NC + c];
                 else if (c < NC + 3) ts[q] = itabfield<R>(L)[3 * g + c - NC];
-                else if constexpr (sizeof(R) == 8)
-                    if (c < NC + 3 + RowN<M>::value) ts[q] = L.rows64[g * RowN<M>::value + c - NC - 3];
+                else if (c < NC + 3 + RowN<M>::value) ts[q] = L.rows64[g * RowN<M>::value + c - NC - 3];
             }
             have = S.cell;
         }
@@ -486,14 +486,10 @@ __global__ void __launch_bounds__(kCellThreads, sizeof(R) == 4 ? AE_CELL_SMOOTH_
                            __ldg(gid + o.zp) != __ldg(gid + o.zm);
                 R gu[3][3];
                 const CellAt<R> at{u + t, nn, o};
-                if constexpr (sizeof(R) == 8) {
-                    R D[3][6];
-                    row_diffs<R>(K, at, D, gu);
-                    row_scale(K, D);
-                    row_sum<M>([&](int n) { return SM ? ts[g * TS + NC + 3 + n] : __ldg(L.rows64 + g * RowN<M>::value + n); }, D, f);
-                } else {
-                    row_interior<M, R>(K, at, [&](int q) { return slot(g, q); }, gu, f);
-                }
+                R D[3][6];
+                row_diffs<R>(K, at, D, gu);
+                row_scale(K, D);
+                row_sum<M>([&](int n) { return SM ? ts[g * TS + NC + 3 + n] : __ldg(L.rows64 + g * RowN<M>::value + n); }, D, f);
                 if (!wide) finish(t, g, f);
             }
             const unsigned ball = __ballot_sync(0xffffffffu, wide);
@@ -553,7 +549,7 @@ __global__ void __launch_bounds__(kCellThreads, sizeof(R) == 4 ? AE_CELL_SMOOTH_
     }
 }
 
-// The FP32 sweeps of those cells (cell_marches): a block takes kMarchNodes consecutive nodes of a plane
+// The FP32 sweeps of cells on a grain map that march (CellLevelDev::march): a block takes kMarchNodes consecutive nodes of a plane
 // and marches up to kz planes in k.  A ring of four planes in shared memory holds the whole rows the
 // block's nodes touch, wrapped in y and z as they are loaded (cp.async, one plane ahead), so that a
 // displacement is read from global memory once a block and no address in the row is wrapped but along x;
@@ -565,22 +561,23 @@ __global__ void __launch_bounds__(kCellThreads, sizeof(R) == 4 ? AE_CELL_SMOOTH_
 // smoother sweep 0.415 -> 0.314 ms, residual of the correction 0.417 -> 0.300.  A queue per warp over several
 // planes, its neighbours read from global memory, took 0.333; two planes a thread, 96 registers and five
 // blocks of 128 threads, 0.356; five blocks of this form (spills) 0.367.
-constexpr int kMarchW = kMarchNodes - 1 + 4 * kMarchX;  // words a component's rows take at most
-constexpr int kMarchRing = 4;                            // planes k - 1, k, k + 1 and the next
-template <int M>
+constexpr int kMarchRing = 4;  // planes k - 1, k, k + 1 and the next
+template <int X>
+constexpr int kMarchW = kMarchNodes - 1 + 4 * X;  // words a component's rows of up to X nodes take at most
+template <int M, int X>
 constexpr size_t march_smem() {
-    return sizeof(float) * (kMarchRing * 3 * kMarchW + kGrainTabs<float> * grain_words<M, float>() + 4 * kMarchNodes + 2);
+    return sizeof(float) * (kMarchRing * 3 * kMarchW<X> + kMarchGrains * grain_words<M, float>() + 4 * kMarchNodes + 2);
 }
-template <int M, int OP>
+template <int M, int OP, int X>
 __global__ void __launch_bounds__(kMarchNodes, kMarchBlocks)
     kb_grain_march(CellArgs A, const Work* __restrict__ tab, int ntab, int kz, int flag) {
     using R = float;
-    constexpr int NC = NCoef<M>::value, TS = grain_words<M, R>();
+    constexpr int NC = NCoef<M>::value, TS = grain_words<M, R>(), W = kMarchW<X>;
     extern __shared__ __align__(16) unsigned char march_mem[];
-    R* const ring = reinterpret_cast<R*>(march_mem);  // [kMarchRing][3][kMarchW]
-    R* const ts = ring + kMarchRing * 3 * kMarchW;
+    R* const ring = reinterpret_cast<R*>(march_mem);  // [kMarchRing][3][W]
+    R* const ts = ring + kMarchRing * 3 * W;
     const int lane = threadIdx.x & 31;
-    R* const qf = ts + kGrainTabs<R> * TS;  // [3][kMarchNodes]: a queued node's row so far
+    R* const qf = ts + kMarchGrains * TS;  // [3][kMarchNodes]: a queued node's row so far
     int* const qt = reinterpret_cast<int*>(qf + 3 * kMarchNodes);  // its thread
     int* const qn = qt + kMarchNodes;                                // entries, of even and odd planes
     int have = -1;  // the cell whose numbers are in ts
@@ -607,7 +604,7 @@ __global__ void __launch_bounds__(kMarchNodes, kMarchBlocks)
         const int words = (j1 - j0 + 3) * n0;
         const int at = (j - j0 + 1) * n0 + i, xp = i == n0 - 1 ? 1 - n0 : 1, xm = i == 0 ? n0 - 1 : -1;
         __syncthreads();  // the block is done with the ring and the numbers
-        constexpr int kLoads = (kMarchW + kMarchNodes - 1) / kMarchNodes;
+        constexpr int kLoads = (W + kMarchNodes - 1) / kMarchNodes;
         int from[kLoads];  // the thread's words of a plane: their place in the cell's plane, or none
 #pragma unroll
         for (int l = 0; l < kLoads; ++l) {
@@ -618,12 +615,12 @@ __global__ void __launch_bounds__(kMarchNodes, kMarchBlocks)
         }
         const auto load = [&](int k) {  // plane k, z0 - 1 <= k <= z1
             const R* src = u + (k < 0 ? k + n2 : k >= n2 ? k - n2 : k) * sz;
-            R* dst = ring + (k & (kMarchRing - 1)) * (3 * kMarchW) + threadIdx.x;
+            R* dst = ring + (k & (kMarchRing - 1)) * (3 * W) + threadIdx.x;
 #pragma unroll
             for (int l = 0; l < kLoads; ++l)
                 if (from[l] >= 0)
 #pragma unroll
-                    for (int p = 0; p < 3; ++p) cp_async<4>(dst + p * kMarchW + l * kMarchNodes, src + from[l] + p * nn);
+                    for (int p = 0; p < 3; ++p) cp_async<4>(dst + p * W + l * kMarchNodes, src + from[l] + p * nn);
             cp_async_commit();
         };
         load(z0 - 1);
@@ -653,7 +650,7 @@ __global__ void __launch_bounds__(kMarchNodes, kMarchBlocks)
             cp_async_wait<0>();
             __syncthreads();
             if (k + 1 < z1) load(k + 2);
-            const auto slot = [&](int kk) { return ring + (kk & (kMarchRing - 1)) * (3 * kMarchW); };
+            const auto slot = [&](int kk) { return ring + (kk & (kMarchRing - 1)) * (3 * W); };
             const R* pl[3] = {slot(k - 1) + at, slot(k) + at, slot(k + 1) + at};
             const int t = cm + k * sz;
             const int up = k == n2 - 1 ? (1 - n2) * sz : sz, down = k == 0 ? (n2 - 1) * sz : -sz;
@@ -667,11 +664,11 @@ __global__ void __launch_bounds__(kMarchNodes, kMarchBlocks)
             row_interior<M, R>(
                 K,
                 [&](int p, int a, int bb, int c) {
-                    return pl[c + 1][p * kMarchW + (a > 0 ? xp : a < 0 ? xm : 0) + (bb > 0 ? n0 : bb < 0 ? -n0 : 0)];
+                    return pl[c + 1][p * W + (a > 0 ? xp : a < 0 ? xm : 0) + (bb > 0 ? n0 : bb < 0 ? -n0 : 0)];
                 },
                 [&](int q) { return ts[g * TS + q]; }, gu, f);
             if (act && !wide) {
-                const R xc[3] = {pl[1][0], pl[1][kMarchW], pl[1][2 * kMarchW]};
+                const R xc[3] = {pl[1][0], pl[1][W], pl[1][2 * W]};
                 finish(t, g, xc, f);
             }
             int* const n = qn + (k & 1);
@@ -700,9 +697,9 @@ __global__ void __launch_bounds__(kMarchNodes, kMarchBlocks)
 #pragma unroll
                 for (int p = 0; p < 3; ++p) {
                     fq[p] = qf[p * kMarchNodes + threadIdx.x];
-                    gv[p][0] = node_diff(K, 0, qc[p * kMarchW + qxp], qc[p * kMarchW + qxm]);
-                    gv[p][1] = node_diff(K, 1, qc[p * kMarchW + n0], qc[p * kMarchW - n0]);
-                    gv[p][2] = node_diff(K, 2, qp[p * kMarchW], qm[p * kMarchW]);
+                    gv[p][0] = node_diff(K, 0, qc[p * W + qxp], qc[p * W + qxm]);
+                    gv[p][1] = node_diff(K, 1, qc[p * W + n0], qc[p * W - n0]);
+                    gv[p][2] = node_diff(K, 2, qp[p * W], qm[p * W]);
                 }
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
@@ -716,7 +713,7 @@ __global__ void __launch_bounds__(kMarchNodes, kMarchBlocks)
                 }
 #pragma unroll
                 for (int r = 0; r < 3; ++r) fq[r] = row_gradc(K, fq[r], col[0][r], col[1][r], col[2][r]);
-                const R xc[3] = {qc[0], qc[kMarchW], qc[2 * kMarchW]};
+                const R xc[3] = {qc[0], qc[W], qc[2 * W]};
                 finish(tq, __ldg(gids + tq), xc, fq);
             }
         }
@@ -1067,23 +1064,37 @@ void by_rep(int reps, F&& f) {
     if (reps & kRepNode) f(std::false_type());
     if (reps & (kRepGrains | kRepMarch)) f(std::true_type());
 }
-// grain maps, smoother and correction residual: marching cells in FP32 apart from the others
+// grain maps, smoother and correction residual: two passes in FP64; in FP32 marching cells apart from the
+// others, which take one pass
 template <int M, class R, int OP>
 void launch_grain_sweep(const CellArgs& A, const Work* tab, int ntab, Shape sh, int flag, int reps, const MarchTab& mt,
                         cudaStream_t st) {
-    if (reps & (sizeof(R) == 4 ? kRepGrains : kRepGrains | kRepMarch)) {
-        kb_grain_sweep<M, R, OP><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, flag);
-        launched();
-    }
-    if constexpr (sizeof(R) == 4) {
-        if (reps & kRepMarch) {
-            constexpr size_t smem = march_smem<M>();
-            static std::once_flag once;
-            std::call_once(once, [] {
-                AE_CUDA_CHECK(cudaFuncSetAttribute(kb_grain_march<M, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            });
-            kb_grain_march<M, OP><<<std::min(mt.n, mt.grid), kMarchNodes, smem, st>>>(A, mt.tab, mt.n, mt.kz, flag);
+    if constexpr (sizeof(R) == 8) {
+        if (reps & (kRepGrains | kRepMarch)) {
+            kb_grain_sweep<M, OP><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, flag);
             launched();
+        }
+    } else {
+        if (reps & kRepGrains) {
+            if constexpr (OP == CELL_SMOOTH)
+                kb_smooth<M, R, false, true><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, 0, flag);
+            else
+                kb_rescor<M, R, true><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, 0, flag);
+            launched();
+        }
+        if (reps & kRepMarch) {
+            const auto go = [&](auto x) {
+                constexpr int X = decltype(x)::value;
+                constexpr size_t smem = march_smem<M, X>();
+                static std::once_flag once;
+                std::call_once(once, [] {
+                    AE_CUDA_CHECK(cudaFuncSetAttribute(kb_grain_march<M, OP, X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                });
+                kb_grain_march<M, OP, X><<<std::min(mt.n, mt.grid), kMarchNodes, smem, st>>>(A, mt.tab, mt.n, mt.kz, flag);
+                launched();
+            };
+            if (mt.rows <= kMarchXs) go(std::integral_constant<int, kMarchXs>());
+            else go(std::integral_constant<int, kMarchX>());
         }
     }
 }
@@ -1128,7 +1139,7 @@ void cells_launch_rescor(int model, int prec, const CellArgs& A, const Work* tab
         by_prec(prec, [&](auto r) {
             using R = decltype(r);
             if (reps & kRepNode) {
-                kb_rescor<M, R><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, m, inplace);
+                kb_rescor<M, R, false><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, m, inplace);
                 launched();
             }
             launch_grain_sweep<M, R, CELL_RESCOR>(A, tab, ntab, sh, inplace, reps, mt, st);
@@ -1161,7 +1172,7 @@ void cells_launch_resid_top(int model, const CellArgs& A, const Work* tab, int n
     dispatch_model<double>(model, [&](auto mm) {
         by_rep(reps, [&](auto gr) {
             constexpr int M = decltype(mm)::value;
-            if (decltype(gr)::value) kb_grain_sweep<M, double, CELL_RESID><<<ntab, kRedChunk, 0, st>>>(A, tab, ntab, 0);
+            if (decltype(gr)::value) kb_grain_sweep<M, CELL_RESID><<<ntab, kRedChunk, 0, st>>>(A, tab, ntab, 0);
             else kb_resid_top<M><<<ntab, kRedChunk, 0, st>>>(A, tab, ntab);
             launched();
         });
