@@ -316,12 +316,16 @@ void CellEngine::rebuild() {
     if (march_nodes(kMarchXs) >= (model == AE_MODEL_DIAGONAL ? kMarchMinNodesD : kMarchMinNodes)) march_rows = kMarchXs;
     if (march_nodes(kMarchX) >= kMarchMinNodesX) march_rows = kMarchX;
     int longest = 0;
-    long long nodes = 0;
+    long long nodes = 0, grain_nodes = 0, grains = 0;
     for (int c = 0; c < ncell; ++c) {
         CellRes* r = live[c];
         CellDev& d = hcells[c];
         d.nlev = r->nlev;
         for (int m = 0; m < r->nlev; ++m) d.lv[m] = r->lv[m];
+        if (r->lv[0].gid) {
+            grain_nodes += (long long)r->lv[0].nn * r->nrhs;
+            grains += (long long)r->lv[0].ngrains * r->nrhs;
+        }
         d.lv[0].march = cell_can_march(r->lv[0], march_rows);
         if (d.lv[0].march) {
             longest = std::max(longest, d.lv[0].n[0]);
@@ -339,6 +343,7 @@ void CellEngine::rebuild() {
         reps0 |= !r->lv[0].gid ? kRepNode : d.lv[0].march ? kRepMarch : kRepGrains;
     }
     march_rows = longest;
+    two_pass = grain_nodes >= (grain_nodes >= kTwoPassGrainNodes * grains ? kTwoPassMinNodesWide : kTwoPassMinNodes);
     nsolves = (int)hsolves.size();
     if ((size_t)ncell > cap_cells || !dcells) {
         if (dcells) AEH_CHECK(cudaFree(dcells));
@@ -473,7 +478,7 @@ void CellEngine::begin(const std::vector<int>& cell_slots, const ae_solver_opts&
     cells_launch_rhs(model, A, tsub.d, tsub.n, st);
     cells_launch_mean(A, dslots, ns, 0, 1, st);
     cells_launch_project(prec, 1, A, tsub.d, tsub.n, st);
-    cells_launch_resid_top(model, A, tsub.d, tsub.n, reps0, st);
+    cells_launch_resid_top(model, A, tsub.d, tsub.n, reps0, two_pass, st);
     cells_launch_mean(A, dslots, ns, 0, 0, st);
     cells_launch_project(prec, 0, A, tsub.d, tsub.n, st);
     cells_launch_status(A, dslots, ns, 1, tol_rel, tol_abs, o.max_iter, dcount, nullptr, st);
@@ -521,7 +526,7 @@ void CellEngine::iteration_body(int prec, const ae_solver_opts& o, double tol_re
         cells_launch_update(prec, A, tred.d, tred.n, st);
         if (c + 1 < inner) cells_launch_rescor(model, prec, A, table(0).d, table(0).n, shape(0), 0, 1, reps0, march(), st);
     }
-    cells_launch_resid_top(model, A, tred.d, tred.n, reps0, st);
+    cells_launch_resid_top(model, A, tred.d, tred.n, reps0, two_pass, st);
     cells_launch_mean(A, nullptr, nsolves, 0, 0, st);
     cells_launch_project(prec, 0, A, tred.d, tred.n, st);
     cells_launch_status(A, nullptr, nsolves, 0, tol_rel, tol_abs, o.max_iter, dcount, dactive, st);

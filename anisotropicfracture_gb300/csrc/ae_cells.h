@@ -123,11 +123,19 @@ constexpr int kMarchNodes = 256, kMarchBlocks = 4;  // nodes of a plane a block 
 inline bool cell_can_march(const CellLevelDev& L, int rows) {
     return L.gid != nullptr && L.n[0] <= rows && L.ngrains <= kMarchGrains;
 }
+// FP64: two passes (kb_grain_sweep) or one.  Two passes pack the nodes at grain boundaries, but run one after
+// the other and start by loading the grains' numbers: one pass wins on little work, the more so the more of
+// the nodes lie at a boundary.  FP64 cycles, ms, two passes / one: one cell of 16^3 in 32 grains 1.80 / 1.59,
+// 48 of them (0.2 M nodes) 5.22 / 5.04, one of 48^3 3.16 / 3.27, 24 of 16^3 in 8 grains 2.29 / 2.37, 24 of
+// 24^3 in 32 (0.33 M) 6.69 / 6.95, 24 of 32^3 (0.8 M) 12.9 / 14.2.
+constexpr long long kTwoPassMinNodes = 300000, kTwoPassMinNodesWide = 90000;
+constexpr int kTwoPassGrainNodes = 512;  // nodes per grain from which the lower of the two limits holds
 // the marching cells' work: entry start = first node of a run of nodes in plane z, kz planes from there on
 struct MarchTab {
     const Work* tab;
     int n, kz, grid;
-    int rows;  // the longest row among the cells
+    int rows;       // the longest row among the cells
+    bool two_pass;  // the FP64 sweeps of all cells on a grain map: kb_grain_sweep, or one pass
 };
 
 // ---- launchers (ae_cells_kernels.cu); model 0 ISO, 1 MM, 2 DIAG
@@ -148,7 +156,8 @@ void cells_launch_interp(int prec, const CellArgs& A, const Work* tab, int ntab,
 void cells_launch_bottom(int model, int prec, const CellArgs& A, int nsolves, const KrylovParams& kp,
                          cudaStream_t st);
 // FP64 top level (tab: level-0 runs of kRedChunk nodes, one block each)
-void cells_launch_resid_top(int model, const CellArgs& A, const Work* tab, int ntab, int reps, cudaStream_t st);
+void cells_launch_resid_top(int model, const CellArgs& A, const Work* tab, int ntab, int reps, bool two_pass,
+                            cudaStream_t st);
 void cells_launch_rhs(int model, const CellArgs& A, const Work* tab, int ntab, cudaStream_t st);
 // per-solve mean of the partials: which 0 residual/rhs -> mean, 1 w -> wmean, 2 stress -> sig
 // (slots: the solve slots to visit, nullptr = 0 .. nsolves-1)

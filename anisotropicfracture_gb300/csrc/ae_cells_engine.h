@@ -67,7 +67,8 @@ struct CellEngine {
     Table tred;
     Table tmarch;
     int march_kz = 1, march_rows = 0;
-    MarchTab march() const { return MarchTab{tmarch.d, tmarch.n, march_kz, nsm * kMarchBlocks, march_rows}; }
+    bool two_pass = false;
+    MarchTab march() const { return MarchTab{tmarch.d, tmarch.n, march_kz, nsm * kMarchBlocks, march_rows, two_pass}; }
     Table tcell[kMaxCellLevels];
     // launch shapes per level (chunk option index and grid); forced[m] set by the caller
     int chunk_idx[kMaxCellLevels];

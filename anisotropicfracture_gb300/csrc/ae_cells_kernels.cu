@@ -364,14 +364,14 @@ __device__ __forceinline__ void block_partials(double (&v)[NQ], double* dst) {
 }
 
 // r = b - A x at level 0 with per-chunk sums of r (tab: one kRedChunk run per entry)
-template <int M>
-__global__ void __launch_bounds__(kCellThreads) kb_resid_top(CellArgs A, const Work* __restrict__ tab, int ntab) {
+template <int M, bool GR>
+__global__ void __launch_bounds__(kCellThreads, cell_min_blocks<M, double, GR>()) kb_resid_top(CellArgs A, const Work* __restrict__ tab, int ntab) {
     for (int e = blockIdx.x; e < ntab; e += gridDim.x) {
         const Work w = tab[e];
         const SolveDev& S = A.solves[w.id];
         if (!S.st->active) continue;
         const CellLevelDev& L = A.cells[S.cell].lv[0];
-        if (rep_skips(false, 0, L)) continue;
+        if (rep_skips(GR, 0, L)) continue;
         const int t = w.start + threadIdx.x;
         const int nn = L.nn;
         double v[3] = {0.0, 0.0, 0.0};
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(kCellThreads) kb_resid_top(CellArgs A, const W
             cell_ijk(L.n, t, i, j, k);
             const POff o = cell_offsets(L.n, i, j, k);
             double f[3];
-            level_apply<M, double, false>(L, A.uniform, S.x, t, o, f);
+            level_apply<M, double, GR>(L, A.uniform, S.x, t, o, f);
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
                 v[p] = row_residual(S.b[p * nn + t], L.K64.i2[0], f[p]);
@@ -1069,19 +1069,21 @@ void by_rep(int reps, F&& f) {
 template <int M, class R, int OP>
 void launch_grain_sweep(const CellArgs& A, const Work* tab, int ntab, Shape sh, int flag, int reps, const MarchTab& mt,
                         cudaStream_t st) {
-    if constexpr (sizeof(R) == 8) {
+    if (sizeof(R) == 8 && mt.two_pass) {
         if (reps & (kRepGrains | kRepMarch)) {
             kb_grain_sweep<M, OP><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, flag);
             launched();
         }
-    } else {
-        if (reps & kRepGrains) {
-            if constexpr (OP == CELL_SMOOTH)
-                kb_smooth<M, R, false, true><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, 0, flag);
-            else
-                kb_rescor<M, R, true><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, 0, flag);
-            launched();
-        }
+        return;
+    }
+    if (reps & (sizeof(R) == 8 ? kRepGrains | kRepMarch : kRepGrains)) {
+        if constexpr (OP == CELL_SMOOTH)
+            kb_smooth<M, R, false, true><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, 0, flag);
+        else
+            kb_rescor<M, R, true><<<grid_of(ntab, sh), sh.chunk, 0, st>>>(A, tab, ntab, 0, flag);
+        launched();
+    }
+    if constexpr (sizeof(R) == 4) {
         if (reps & kRepMarch) {
             const auto go = [&](auto x) {
                 constexpr int X = decltype(x)::value;
@@ -1167,13 +1169,15 @@ void cells_launch_bottom(int model, int prec, const CellArgs& A, int nsolves, co
     });
     launched();
 }
-void cells_launch_resid_top(int model, const CellArgs& A, const Work* tab, int ntab, int reps, cudaStream_t st) {
+void cells_launch_resid_top(int model, const CellArgs& A, const Work* tab, int ntab, int reps, bool two_pass,
+                            cudaStream_t st) {
     if (ntab == 0) return;
     dispatch_model<double>(model, [&](auto mm) {
         by_rep(reps, [&](auto gr) {
             constexpr int M = decltype(mm)::value;
-            if (decltype(gr)::value) kb_grain_sweep<M, CELL_RESID><<<ntab, kRedChunk, 0, st>>>(A, tab, ntab, 0);
-            else kb_resid_top<M><<<ntab, kRedChunk, 0, st>>>(A, tab, ntab);
+            constexpr bool GR = decltype(gr)::value;
+            if (GR && two_pass) kb_grain_sweep<M, CELL_RESID><<<ntab, kRedChunk, 0, st>>>(A, tab, ntab, 0);
+            else kb_resid_top<M, GR><<<ntab, kRedChunk, 0, st>>>(A, tab, ntab);
             launched();
         });
     });

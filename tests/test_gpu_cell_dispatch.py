@@ -1,6 +1,7 @@
 """Finest-level sweeps of cells on a grain map over the rules that choose them.  FP32: cells of at most 96
 grains march, with rows of up to 64 nodes once such cells hold 1.5 million nodes of solves (9 slots: 3
-million), with rows of up to 128 from 5 million on; the others take one pass.  A filler cell beside
+million), with rows of up to 128 from 5 million on; the others take one pass.  FP64: two passes from 300
+thousand nodes of solves on, from 90 thousand if a grain holds 512 of them, else one.  A filler cell beside
 the one under test sets the totals.  Every way runs the arithmetic of the per-node sweeps on the equivalent
 field, so solutions agree bit for bit with a cell given as that field."""
 import numpy as np
@@ -75,3 +76,11 @@ def test_fp32_sweeps_equal_the_field_bit_for_bit(n, ngr, filler):
 @pytest.mark.parametrize("filler", [NONE, ROWS64, ROWS64D, ROWS128])
 def test_fp32_sweeps_of_the_other_kinds(model, n, ngr, filler):
     _check(n, ngr, 1, filler, model)
+
+
+# 56 grains fill the FP64 tables, 57 do not
+@pytest.mark.parametrize("model", [models.MAJORMINOR, models.ISOTROPIC, models.DIAGONAL])
+@pytest.mark.parametrize("n,ngr", [(4, 2), (20, 57), ((12, 34, 6), 56), (48, 30)])
+@pytest.mark.parametrize("filler", [NONE, ROWS64])
+def test_fp64_sweeps_equal_the_field_bit_for_bit(model, n, ngr, filler):
+    _check(n, ngr, 0, filler, model)
