@@ -495,11 +495,10 @@ def parity_at_size(op, levels, bc, device):
         u = rng.standard_normal(shape)
         b = rng.standard_normal(shape)
         ud, bd = torch.from_numpy(u).to(device), torch.from_numpy(b).to(device)
-        f = torch.zeros_like(ud)
+        f, r, xd = torch.zeros_like(ud), torch.zeros_like(ud), ud.clone()
+        torch.cuda.synchronize()  # the operator runs on a stream of the caller's, not on the default one
         op.Fapply(a, 0, Field(f, lo), Field(ud, lo))
-        r = torch.zeros_like(ud)
         op.Residual(a, 0, Field(r, lo), Field(ud, lo), Field(bd, lo))
-        xd = ud.clone()
         op.Fsmooth(a, 0, Field(xd, lo), Field(bd, lo), 2, 2.0 / 3.0)
         torch.cuda.synchronize()
         got = {"fapply": f.cpu().numpy(), "residual": r.cpu().numpy(), "fsmooth": xd.cpu().numpy()}
@@ -1033,6 +1032,7 @@ def main():
     op.set_stream(stream.cuda_stream)
     dev = torch.device("cuda", local)
     rhs_d = [torch.zeros((3,) + level_shape(L), dtype=torch.float64, device=dev) for L in levels]
+    torch.cuda.synchronize()  # the operator runs on `stream`, the fill above on the default one
     for a, L in enumerate(levels):  # BC::Operator::Elastic::Init through the library
         op.BCInit(a, Field(rhs_d[a], tuple(L["store_lo"])))
     torch.cuda.synchronize()
