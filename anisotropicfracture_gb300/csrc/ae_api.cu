@@ -154,7 +154,7 @@ struct ae_op_s {
     bool have32 = false;
     bool prepared32 = false;
     bool tiled32 = false, tiled64 = false;  // z-marching tiled sweeps per precision (opt-in)
-    bool split32 = true;                    // split FP32 sweeps on grain-map levels (AE_SPLIT=0: off)
+    bool split32 = true;                    // split sweeps on grain-map levels (AE_SPLIT=0: off)
     bool zero_sweep = true;                 // stencil-free first sweep from a zero correction (AE_ZERO_SWEEP=0: off)
     long long bytes = 0;
     std::vector<void*> allocs;
@@ -505,7 +505,7 @@ void check_tma_flag(ae_op* op) {
     AE_CHECK(cudaStreamSynchronize(op->st));
     if (*f) {
         AE_CHECK(cudaMemsetAsync(op->dflag + 2, 0, sizeof(int), op->st));
-        throw ApiErr(AE_ERR_CUDA, "a shared-memory tile load of the split FP32 sweep did not complete");
+        throw ApiErr(AE_ERR_CUDA, "a shared-memory tile load of a split sweep did not complete");
     }
 }
 

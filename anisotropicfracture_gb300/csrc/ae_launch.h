@@ -113,8 +113,8 @@ void launch_fapply(const OpParams& P, View<const R> C, View<const R> u, View<R> 
 template <class R>
 void launch_residual(const OpParams& P, View<const R> C, View<const R> x, View<const R> b, View<R> r,
                      unsigned long long* norm, View<float>* r32, cudaStream_t st, Grains<R> G = Grains<R>{});
-// One damped-Jacobi sweep: xo = (1-w) xi + w (b - (A xi - D xi)) / D on grow(valid,1)∩dom,
-// zero on the ring grow(valid,2) \ grow(valid,1), copy elsewhere.
+// One damped-Jacobi sweep: xo = xi + w (b - A xi) / D on grow(valid,1)∩dom (Operator.cpp:154 without the
+// terms in D that cancel), zero on the ring grow(valid,2) \ grow(valid,1), copy elsewhere.
 template <class R>
 void launch_jacobi(const OpParams& P, View<const R> C, View<const R> invD, View<const R> xi,
                    View<const R> b, View<R> xo, R omega, cudaStream_t st, Grains<R> G = Grains<R>{});

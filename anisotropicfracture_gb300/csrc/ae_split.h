@@ -1,4 +1,4 @@
-// Split FP32 sweeps on Voronoi (grain-map) levels: a tiled kernel over the interior box plus
+// Split sweeps on Voronoi (grain-map) levels, FP32 and FP64: a tiled kernel over the interior box plus
 // the per-node code over a list of the nodes that need it (see ae_split.cu).
 #pragma once
 #include <cuda_runtime.h>
