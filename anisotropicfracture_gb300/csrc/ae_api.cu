@@ -353,8 +353,15 @@ void alloc_level_fp32(ae_op* op) {
 }
 
 // The four-warp form of the assembled matrix, when the level is small enough for it.
-void upload_bottom_ell(ae_op* op, MGLevel& L, const std::vector<int>& rp, const std::vector<int>& cl,
-                       const std::vector<double>& vl) {
+void upload_bottom_ell(ae_op* op, MGLevel& L, const std::vector<int>& rp) {
+    if ((int)rp.size() - 1 > kBottomQuadLayers * kEllThreads) return;
+    std::vector<int> cl((size_t)L.csr_nnz);
+    std::vector<double> vl((size_t)L.csr_nnz);
+    if (L.csr_nnz) {
+        AE_CHECK(cudaMemcpyAsync(cl.data(), L.csr_col, sizeof(int) * L.csr_nnz, cudaMemcpyDeviceToHost, op->st));
+        AE_CHECK(cudaMemcpyAsync(vl.data(), L.csr_val, sizeof(double) * L.csr_nnz, cudaMemcpyDeviceToHost, op->st));
+        AE_CHECK(cudaStreamSynchronize(op->st));
+    }
     const BottomEllHost h = bottom_ell(rp, cl, vl, kBottomQuadLayers);
     if (!h.ok) return;
     BottomEll& m = L.ell;
@@ -395,7 +402,7 @@ void upload_bottom_ell(ae_op* op, MGLevel& L, const std::vector<int>& rp, const 
 }
 
 // The coarsest level of AMR level 0 as an FP64 CSR matrix (levels of up to kBottomCsrMaxN
-// unknowns): dense columns A e_j on the device, compressed here, uploaded once per preparation.
+// unknowns): dense columns A e_j and their packing on the device, once per preparation.
 void assemble_bottom(ae_op* op) {
     MGLevel& L = op->amr[0].mg.back();
     if (L.csr_built && L.csr_uniform == op->uniform) return;
@@ -422,34 +429,21 @@ void assemble_bottom(ae_op* op) {
         cudaGetLastError();
         return;
     }
-    std::vector<double> h((size_t)(N * N));
     launch_bottom_assemble(a, A.p, E.p, st);
-    AE_CHECK(cudaMemcpyAsync(h.data(), A.p, sizeof(double) * N * N, cudaMemcpyDeviceToHost, st));
-    AE_CHECK(cudaStreamSynchronize(st));
-    std::vector<int> rp((size_t)N + 1, 0), cl;
-    std::vector<double> vl;
-    for (long long r = 0; r < N; ++r) {
-        for (long long c = 0; c < N; ++c) {
-            const double v = h[(size_t)(r * N + c)];
-            if (v != 0.0) {
-                cl.push_back((int)c);
-                vl.push_back(v);
-            }
-        }
-        rp[(size_t)r + 1] = (int)cl.size();
-    }
-    const int nnz = (int)cl.size();
     if (!L.csr_rowptr) L.csr_rowptr = op->alloc<int>(N + 1);
+    std::vector<int> rp((size_t)N + 1, 0);
+    launch_csr_count(A.p, (int)N, L.csr_rowptr, st);
+    AE_CHECK(cudaMemcpyAsync(rp.data() + 1, L.csr_rowptr, sizeof(int) * N, cudaMemcpyDeviceToHost, st));
+    AE_CHECK(cudaStreamSynchronize(st));
+    for (long long r = 0; r < N; ++r) rp[(size_t)r + 1] += rp[(size_t)r];
+    const int nnz = rp[(size_t)N];
     if (nnz > L.csr_cap) {
         L.csr_col = op->alloc<int>(nnz);
         L.csr_val = op->alloc<double>(nnz);
         L.csr_cap = nnz;
     }
     AE_CHECK(cudaMemcpyAsync(L.csr_rowptr, rp.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice, st));
-    if (nnz) {
-        AE_CHECK(cudaMemcpyAsync(L.csr_col, cl.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice, st));
-        AE_CHECK(cudaMemcpyAsync(L.csr_val, vl.data(), sizeof(double) * nnz, cudaMemcpyHostToDevice, st));
-    }
+    launch_csr_fill(A.p, (int)N, L.csr_rowptr, L.csr_col, L.csr_val, st);
     // chunks of at most kCsrChunk nonzeros, row by row
     std::vector<int> cp, rc;
     csr_chunks(rp, kCsrChunk, cp, rc);
@@ -465,7 +459,7 @@ void assemble_bottom(ae_op* op) {
     L.csr_nnz = nnz;
     L.csr_nchunk = nchunk;
     L.csr_ok = true;
-    upload_bottom_ell(op, L, rp, cl, vl);
+    upload_bottom_ell(op, L, rp);
 }
 
 // FP32 copies of the stiffness and 1 / diagonal on every level (mixed-precision cycle)

@@ -26,15 +26,21 @@ struct BottomEllHost {
 
 // warp-wide FP64 instructions of one product on the busiest warp, for chunks of c nonzeros
 inline int bottom_ell_cost(const std::vector<int>& lens, int c) {
-    std::vector<int> chunks;
+    std::vector<int> count(c + 1, 0);  // chunks of each length
     int most = 1;
     for (int n : lens) {
         most = std::max(most, (n + c - 1) / c);
-        for (int q = 0; q < n; q += c) chunks.push_back(std::min(c, n - q));
+        count[c] += n / c;
+        count[n % c] += 1;
     }
-    std::sort(chunks.rbegin(), chunks.rend());
+    // groups of 32 chunks, longest first: each as long as its first
     int load[kEllWarps] = {};
-    for (size_t g = 0; g < chunks.size(); g += 32) *std::min_element(load, load + kEllWarps) += chunks[g];
+    int len = c, before = 0;  // chunks longer than len
+    for (int g = 0;; g += 32) {
+        while (len > 0 && g >= before + count[len]) before += count[len--];
+        if (len == 0) break;
+        *std::min_element(load, load + kEllWarps) += len;
+    }
     return *std::max_element(load, load + kEllWarps) + (most > kEllLongRow ? 3 + (most - 1) / 8 : most - 1);
 }
 
@@ -42,7 +48,7 @@ inline BottomEllHost bottom_ell(const std::vector<int>& rowptr, const std::vecto
                                 const std::vector<double>& val, int max_layers) {
     BottomEllHost h;
     const int N = (int)rowptr.size() - 1;
-    if (N < 1) return h;
+    if (N < 1 || N > max_layers * kEllThreads) return h;
     std::vector<int> lens(N), byrow(N);
     for (int r = 0; r < N; ++r) lens[r] = rowptr[r + 1] - rowptr[r];
     int best = 0;

@@ -765,7 +765,7 @@ void launch_ring_interp_fix(const Geo& gf, View<double> x, View<const float> ecr
 // FP64 at a small fraction of its FP32 rate, and the stencil form of the level operator costs a few
 // hundred FP64 instructions per node on one SM; the assembled rows cost one FMA per nonzero.  Column
 // j is the operator applied to the unit vector e_j (so every entry is the stencil's own coefficient
-// sum for that pair of unknowns); the host compresses the columns to CSR.
+// sum for that pair of unknowns); its nonzeros are packed on the device, a warp per row.
 
 // block j: column j of the dense N x N matrix A (row-major); E holds one unit vector per block
 template <int M>
@@ -793,6 +793,44 @@ void launch_bottom_assemble(const BottomArgs& a, double* A, double* E, cudaStrea
     dispatch_model4<double>(a.P.model, [&](auto m) {
         k_bottom_assemble<decltype(m)::value><<<(unsigned)(3 * a.nn), 128, 0, st>>>(a, A, E);
     });
+    launched();
+}
+
+// Packing the nonzeros here instead of copying the dense matrix (19 MB for 1536 unknowns) to the host and packing
+// there: the first FP64 solve of a preparation is charged with all of the assembly.  8^3 nodes, 21 slots, first
+// solve over a repeated one: 3.3 ms with the packing on the host, 0.9 here.
+constexpr int kPackThreads = 128;
+__global__ void __launch_bounds__(kPackThreads) k_csr_count(const double* __restrict__ A, int N, int* __restrict__ count) {
+    const int r = (int)((blockIdx.x * kPackThreads + threadIdx.x) / 32), lane = threadIdx.x & 31;
+    if (r >= N) return;
+    int n = 0;
+    for (int c = lane; c < N; c += 32) n += A[(long long)r * N + c] != 0.0;
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0) count[r] = n;
+}
+__global__ void __launch_bounds__(kPackThreads) k_csr_fill(const double* __restrict__ A, int N, const int* __restrict__ rowptr,
+                                                           int* __restrict__ col, double* __restrict__ val) {
+    const int r = (int)((blockIdx.x * kPackThreads + threadIdx.x) / 32), lane = threadIdx.x & 31;
+    if (r >= N) return;
+    int at = rowptr[r];
+    for (int c0 = 0; c0 < N; c0 += 32) {
+        const int c = c0 + lane;
+        const double v = c < N ? A[(long long)r * N + c] : 0.0;
+        const unsigned ball = __ballot_sync(0xffffffffu, v != 0.0);
+        if (v != 0.0) {
+            const int q = at + __popc(ball & ((1u << lane) - 1u));
+            col[q] = c;
+            val[q] = v;
+        }
+        at += __popc(ball);
+    }
+}
+void launch_csr_count(const double* A, int N, int* count, cudaStream_t st) {
+    k_csr_count<<<(unsigned)((N * 32 + kPackThreads - 1) / kPackThreads), kPackThreads, 0, st>>>(A, N, count);
+    launched();
+}
+void launch_csr_fill(const double* A, int N, const int* rowptr, int* col, double* val, cudaStream_t st) {
+    k_csr_fill<<<(unsigned)((N * 32 + kPackThreads - 1) / kPackThreads), kPackThreads, 0, st>>>(A, N, rowptr, col, val);
     launched();
 }
 

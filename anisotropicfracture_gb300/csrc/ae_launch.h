@@ -231,6 +231,9 @@ struct BottomCsr {
 // its chunks' sums, so a long row's dependent FP64 chain is a few chunks long, not the whole row
 constexpr int kCsrChunk = 8;
 void launch_bottom_assemble(const BottomArgs& a, double* A, double* E, cudaStream_t st);
+// its nonzeros: count[r] of row r, then, with the rows' starts known, columns and values in column order
+void launch_csr_count(const double* A, int N, int* count, cudaStream_t st);
+void launch_csr_fill(const double* A, int N, const int* rowptr, int* col, double* val, cudaStream_t st);
 void launch_bottom_csr(const BottomArgs& a, const BottomCsr& m, cudaStream_t st);
 // The same matrix laid out for the four-warp bottom solve (ae_bottom_ell.h): unknowns in slots of
 // 128 threads, rows cut into chunks, chunks in groups of 32.
